@@ -82,7 +82,8 @@ std::string tune_key(const Product& p, bool c_read) {
   return p.signature + ";" + scheme_tag(p.scheme) + ";c=" + (c_read ? "1" : "0");
 }
 
-std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms) {
+std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms,
+                                          const dev::LaunchHints& hints) {
   std::vector<PlainChoice> out;
   // The model's choice first (ties go to it).
   {
@@ -90,7 +91,7 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
     if (dev::use_tiny_batched(M, N, K, H)) {
       m.tiny = true;
     } else {
-      dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, &m.kernel, &m.splits, &m.chunk);
+      dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, hints, &m.kernel, &m.splits, &m.chunk);
     }
     out.push_back(m);
   }
@@ -138,7 +139,7 @@ PlainChoice model_choice(const Product& p, int num_sms) {
     return c;
   }
   if (p.split_pin > 0) {
-    c.kernel = p.kernel_pin ? p.kernel_pin : dev::choose_plain_kernel(dt, v.M, v.N, v.K, v.H, num_sms);
+    c.kernel = p.kernel_pin ? p.kernel_pin : dev::choose_plain_kernel(dt, v.M, v.N, v.K, v.H, num_sms, p.hints);
     if (p.split_pin > 1 && v.K > 1) {
       const int64_t chunk = std::max<int64_t>(64, ((v.K + p.split_pin - 1) / p.split_pin + 63) / 64 * 64);
       const int64_t parts = (v.K + chunk - 1) / chunk;
@@ -149,7 +150,7 @@ PlainChoice model_choice(const Product& p, int num_sms) {
     }
     return c;
   }
-  dev::choose_plain_launch(dt, p.kernel_pin, v.M, v.N, v.K, v.H, num_sms, &c.kernel, &c.splits, &c.chunk);
+  dev::choose_plain_launch(dt, p.kernel_pin, v.M, v.N, v.K, v.H, num_sms, p.hints, &c.kernel, &c.splits, &c.chunk);
   return c;
 }
 
@@ -167,6 +168,7 @@ bool choice_fits(const PlainChoice& c, const Product& p) {
   if (c.tiny) return dev::use_tiny_batched(M, N, K, H) && c.splits == 1;
   bool fam_ok = false;
   for (int f : kFamilies[(int)p.problem.dtype & 3]) fam_ok = fam_ok || (f != 0 && f == c.kernel);
+  fam_ok = fam_ok || (dev::is_stream_kernel(c.kernel) && dev::stream_dtype(c.kernel) == (int)p.problem.dtype && K > 0);
   if (!fam_ok || c.splits < 1) return false;
   if (dev::is_packed_kernel(c.kernel) && !dev::packed_fits(c.kernel, M, N, K, H)) return false;
   if (c.splits == 1) return c.chunk == 0 || c.chunk >= K;
@@ -240,7 +242,9 @@ TuningFile parse_tuning_text(const std::string& text) {
     if (ok && kind == "single") {
       ok = static_cast<bool>(f >> e.choice.kernel >> e.choice.splits >> e.choice.chunk >> tiny >> tuned >> e.ms >>
                              e.tried);
-      ok = ok && (tiny != 0 || (e.choice.kernel >= 1 && e.choice.kernel <= dev::PLAIN_LAST)) &&
+      ok = ok &&
+           (tiny != 0 || (e.choice.kernel >= 1 && e.choice.kernel <= dev::PLAIN_LAST) ||
+            dev::is_stream_kernel(e.choice.kernel)) &&
            e.choice.splits >= 1 && e.choice.splits <= 64 && e.choice.chunk >= 0 &&
            (e.choice.splits == 1 || e.choice.chunk > 0);
     } else if (ok && kind == "list") {

@@ -1253,6 +1253,7 @@ dim3 grid_for(const GemmArgs& g) {
 }  // namespace
 
 const char* plain_kernel_name(int k) {
+  if (is_stream_kernel(k)) return stream_kernel_name(k);
   switch (k) {
     case PLAIN_F32_SIMT_128x128: return "sm100.f32.simt.128x128x16";
     case PLAIN_F32_SIMT_64x64: return "sm100.f32.simt.64x64x16";
@@ -1287,8 +1288,27 @@ bool packed_fits(int kernel, int64_t M, int64_t N, int64_t K, int64_t H) {
          H * L.k_pad < ((int64_t)1 << 31) && K > 0;
 }
 
-int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms) {
+int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
   auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * H; };
+  // Stream tiles (gathers coalesced on both sides, at least a wave of tiles)
+  // against the packed family, f64 on B200: 177147 x 243 x 50 0.207 ms against
+  // 0.290 (direct tile 0.295); 64 x 256^3 0.089 against 0.120; 2048^2 x 512 0.162
+  // against 0.183; 2048^3 0.622 against 0.604. Above K = 512 they are chosen where
+  // their tile pads less (136856 x 22 x 240: 0.092 against 0.273).
+  if (hints.a_gather && hints.b_gather && K > 0) {
+    double waste = 0;
+    const int sk = choose_stream_kernel(dtype, M, N, hints, &waste);
+    if (sk) {
+      int bm = 0, bn = 0, pm = 0, pn = 0;
+      plain_tile_shape(sk, &bm, &bn);
+      plain_tile_shape(PLAIN_F64_PACKED_64x64, &pm, &pn);
+      const bool swap = !hints.d_mfast;
+      const int64_t t = swap ? ((N + bm - 1) / bm) * ((M + bn - 1) / bn) * H : tiles(bm, bn);
+      const double pwaste = (double)((M + pm - 1) / pm * pm) * (double)((N + pn - 1) / pn * pn) / ((double)M * (double)N);
+      const int64_t deep = hints.a_vec && hints.b_vec ? 512 : 256;
+      if (t >= num_sms && (K <= deep || waste * 1.25 < pwaste)) return sk;
+    }
+  }
   // At least a full wave of packed tiles and some depth: the pack pass (one
   // read and one write of each operand) is then small beside the tiles' work.
   static const int packed[4] = {PLAIN_F32_PACKED_128x128, PLAIN_F64_PACKED_64x64, PLAIN_C32_PACKED_1M_64x64,
@@ -1297,6 +1317,12 @@ int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, i
     const int pk = packed[dtype & 3];
     int bm = 0, bn = 0;
     plain_tile_shape(pk, &bm, &bn);
+    // Operands whose gather is not coalesced are packed from K = 8 on when
+    // they are small beside the output (3600 x 5600 x 20 f64, six-index output:
+    // 0.097 ms against 0.124 on the direct tile).
+    if (dtype == 1 && K >= 8 && !(hints.a_gather && hints.b_gather) && (M + N) * K * 8 <= M * N &&
+        tiles(bm, bn) >= 2 * num_sms && packed_fits(pk, M, N, K, H))
+      return pk;
     if (K >= 64 && tiles(bm, bn) >= num_sms && packed_fits(pk, M, N, K, H)) return pk;
   }
   switch (dtype) {
@@ -1338,8 +1364,8 @@ int choose_grouped_kernel(int dtype, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
-void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, int* kernel,
-                         int* splits, int64_t* k_chunk) {
+void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms,
+                         const LaunchHints& hints, int* kernel, int* splits, int64_t* k_chunk) {
   auto tiles = [&](int k) {
     int bm = 0, bn = 0;
     plain_tile_shape(k, &bm, &bn);
@@ -1352,6 +1378,21 @@ void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K,
   *splits = 1;
   *k_chunk = 0;
   const int64_t min_chunk = 512;  // K per split
+  // Small f64 products (at most 64 large tiles, K up to 1024): the small direct
+  // tile, K split until about two CTAs run per SM, without a pack pass (399 x 108
+  // x 357: 19.5 us against 29.8; 160 x 198 x 702: 19.8 against 29.2).
+  if (dtype == 1 && !pinned && K <= 1024 && tiles(PLAIN_F64_DMMA_64x64) <= 64) {
+    const int64_t t = tiles(PLAIN_F64_DMMA_32x32);
+    int64_t s = (2 * num_sms + t - 1) / t;
+    s = s < K / 128 ? s : K / 128;
+    *kernel = PLAIN_F64_DMMA_32x32;
+    if (t < num_sms && s > 1) {
+      const int64_t chunk = ((K + s - 1) / s + 63) / 64 * 64;
+      *splits = (int)((K + chunk - 1) / chunk);
+      *k_chunk = *splits > 1 ? chunk : 0;
+    }
+    return;
+  }
   // Deep contractions split along K take the packed family when it fits.
   const int big = packed_fits(packed[dtype & 3], M, N, K, H) ? packed[dtype & 3] : large[dtype & 3];
   const int k = pinned ? pinned : big;
@@ -1372,7 +1413,7 @@ void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K,
       return;
     }
   }
-  *kernel = pinned ? pinned : choose_plain_kernel(dtype, M, N, K, H, num_sms);
+  *kernel = pinned ? pinned : choose_plain_kernel(dtype, M, N, K, H, num_sms, hints);
 }
 
 namespace {
@@ -1447,6 +1488,7 @@ cudaError_t launch_simt_ring(const GemmArgs& g, cudaStream_t st) {
 
 cudaError_t launch_plain_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.H <= 0) return cudaSuccess;
+  if (is_stream_kernel(kernel)) return launch_stream_gemm(dtype, kernel, g, st);
   switch (kernel) {
     case PLAIN_F32_SIMT_128x128:
       if (dtype != 0) return cudaErrorInvalidValue;
@@ -1484,6 +1526,7 @@ cudaError_t launch_plain_gemm(int dtype, int kernel, const GemmArgs& g, cudaStre
 }
 
 void plain_tile_shape(int kernel, int* bm, int* bn) {
+  if (is_stream_kernel(kernel)) return stream_tile_shape(kernel, bm, bn);
   switch (kernel) {
     case PLAIN_F32_SIMT_128x128: *bm = 128; *bn = 128; return;
     case PLAIN_F32_SIMT_64x64: *bm = 64; *bn = 64; return;

@@ -49,7 +49,7 @@ enum : unsigned {
   STATUS_BAD_ARGUMENT = 2u,
 };
 
-struct GemmArgs {
+struct __align__(16) GemmArgs {
   Scatters s;
   const void* A;
   const void* B;
@@ -58,6 +58,9 @@ struct GemmArgs {
   int64_t M, N, K, H;
   int conj_a, conj_b;
   int a_kfast, b_kfast, d_mfast;
+  // Every 16-byte group of the operand's fast index is contiguous and aligned
+  // (16-byte gathers).
+  int a_vec, b_vec;
   Epilogue e;
   unsigned* status;
   // Split-K: each K chunk of k_chunk (a multiple of the tile depth; 0 = all
@@ -96,11 +99,28 @@ enum PlainKernel : int {
   PLAIN_F64_SKINNY_128x16 = 18,
   PLAIN_F64_SKINNY_128x16_K32 = 19,  // K <= 32: half the A stage, three CTAs per SM
   PLAIN_F64_SKINNY_128x32_K32 = 20,
+  // Gather-fed stream tiles (k_stream.cu): chosen by the model, never pinned.
+  PLAIN_STREAM_FIRST = 21,
+  PLAIN_F64_STREAM_64x64 = 21,
+  PLAIN_F64_STREAM_128x32 = 22,
+  PLAIN_F64_STREAM_64x48 = 23,
+  PLAIN_F64_STREAM_32x128 = 24,
+  PLAIN_STREAM_LAST = 24,
 };
 
 // dtype: 0 f32, 1 f64, 2 c32, 3 c64 (TAPP numbering).
 cudaError_t launch_output_pass(int dtype, const GemmArgs& g, cudaStream_t st);
 cudaError_t launch_plain_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
+// Gather-fed stream tiles (k_stream.cu): persistent, one producer warp per CTA.
+bool is_stream_kernel(int kernel);
+int stream_dtype(int kernel);
+void stream_tile_shape(int kernel, int* bm, int* bn);
+const char* stream_kernel_name(int kernel);
+// The stream family of least padded work for a shape (0: none of the dtype),
+// and its padded outputs per output.
+struct LaunchHints;
+int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste);
+cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
 static_assert(sizeof(GemmArgs) % 16 == 0, "grouped kernels copy GemmArgs in 16-byte words");
 
 // One item of a grouped launch: its arguments and its tile grid.
@@ -126,8 +146,15 @@ cudaError_t launch_wait_selftest(const unsigned* flag, unsigned* status, uint64_
 cudaError_t launch_fill_zero(size_t elem, void* origin, int rank, const int64_t* dims, const int64_t* strides,
                              cudaStream_t st);
 const char* plain_kernel_name(int kernel);
+// What the layout says about a launch beyond its extents: whether gathering an
+// operand along its fast index is coalesced, whether it splits into aligned
+// 16-byte groups, and which index D is unit-stride in. The default says nothing
+// (the stream tiles are then not chosen).
+struct LaunchHints {
+  bool a_gather = false, b_gather = false, a_vec = false, b_vec = false, d_mfast = true;
+};
 // The family the autotuner would pick for a shape (no launch).
-int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms);
+int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
 // Batches of tiny products: per-operand batch strides when the batch scatter
 // vector is an arithmetic sequence from 0, else INT64_MIN (the vector is read).
 struct TinyStrides {
@@ -145,8 +172,8 @@ int choose_grouped_kernel(int dtype, int64_t M, int64_t N, int64_t K);
 // One-launch choice with split-K: the family (or `pinned`) and the number of
 // K chunks (1 = no split). Deep contractions with fewer large tiles than SMs
 // take the large tile and split K so that about two CTAs run per SM.
-void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, int* kernel,
-                         int* splits, int64_t* k_chunk);
+void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms,
+                         const LaunchHints& hints, int* kernel, int* splits, int64_t* k_chunk);
 // Sum of the split-K partials (fixed order) and the epilogue into D.
 cudaError_t launch_splitk_reduce(int dtype, const GemmArgs& g, int splits, cudaStream_t st);
 

@@ -146,6 +146,28 @@ int64_t sequence_stride(const std::vector<int64_t>& v) {
     if (v[i] != (int64_t)i * s) return INT64_MIN;
   return s;
 }
+
+// Whether a gather along a fast index is coalesced: three steps in four are 1
+// or -1.
+bool mostly_unit(const std::vector<int64_t>& fast) {
+  size_t unit = 0;
+  for (size_t i = 1; i < fast.size(); ++i) unit += std::llabs(fast[i] - fast[i - 1]) == 1;
+  return fast.size() < 2 || 4 * unit >= 3 * (fast.size() - 1);
+}
+
+// Whether an operand's elements split into aligned 16-byte groups along its
+// fast index: groups of `v` entries of `fast` are consecutive and start at a
+// multiple of `v`, and every other offset is a multiple of `v`.
+bool vector_groups(const std::vector<int64_t>& fast, const std::vector<int64_t>& slow, const std::vector<int64_t>& h,
+                   int64_t v) {
+  for (size_t i = 0; i < fast.size(); ++i)
+    if (i % v == 0 ? fast[i] % v != 0 : fast[i] != fast[i - 1] + 1) return false;
+  for (int64_t x : slow)
+    if (x % v != 0) return false;
+  for (int64_t x : h)
+    if (x % v != 0) return false;
+  return true;
+}
 }  // namespace
 
 Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1)) {
@@ -154,6 +176,14 @@ Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1))
   view = orient(packed, swap);
   tiny_h = dev::TinyStrides{sequence_stride(view.h_a), sequence_stride(view.h_b), sequence_stride(view.h_c),
                             sequence_stride(view.h_d)};
+  const int64_t v = 16 / (int64_t)dtype_size(problem.dtype);
+  const std::vector<int64_t>&af = view.a_kfast ? view.a_k : view.a_m, &as = view.a_kfast ? view.a_m : view.a_k;
+  const std::vector<int64_t>&bf = view.b_kfast ? view.b_k : view.b_n, &bs = view.b_kfast ? view.b_n : view.b_k;
+  hints.a_vec = vector_groups(af, as, view.h_a, v);
+  hints.b_vec = vector_groups(bf, bs, view.h_b, v);
+  hints.a_gather = mostly_unit(af);
+  hints.b_gather = mostly_unit(bf);
+  hints.d_mfast = view.d_mfast;
   signature = problem_signature(*this);
 }
 
@@ -298,7 +328,7 @@ std::string Product::report() const {
   }
   o << ",\"autotune_candidates\":[";
   if (scheme == Scheme::Plain) {
-    const auto cands = plain_candidates((int)problem.dtype, view.M, view.N, view.K, view.H, 148);
+    const auto cands = plain_candidates((int)problem.dtype, view.M, view.N, view.K, view.H, 148, hints);
     for (size_t i = 0; i < cands.size(); ++i)
       o << (i ? "," : "") << "\"" << choice_name(cands[i], (int)problem.dtype) << "\"";
   }
@@ -747,6 +777,8 @@ dev::GemmArgs build_args(Product& pr, Executor& ex, Scalar alpha, Scalar beta, b
   g.a_kfast = pr.view.a_kfast;
   g.b_kfast = pr.view.b_kfast;
   g.d_mfast = pr.view.d_mfast;
+  g.a_vec = pr.hints.a_vec && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0;
+  g.b_vec = pr.hints.b_vec && (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
   g.e = make_epilogue(pr, alpha, beta, c_read);
   g.status = ex.status;
   return g;
@@ -810,7 +842,8 @@ TuneEntry autotune_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, char
                "autotune snapshot of D");
   EventPair ev;
   const std::vector<PlainChoice> cands =
-      plain_candidates((int)pr.problem.dtype, pr.view.M, pr.view.N, pr.view.K, pr.view.H, ex.num_sms);
+      plain_candidates((int)pr.problem.dtype, pr.view.M, pr.view.N, pr.view.K, pr.view.H, ex.num_sms,
+                       pr.hints);
   TuneEntry best;
   best.ms = 0;
   for (size_t i = 0; i < cands.size(); ++i) {
@@ -1017,8 +1050,8 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
       const int64_t mc = cm(c), ncols = cn(c);
       PlainChoice& pc = pcs[c];
       if (dev::use_tiny_batched(mc, ncols, v.K, v.H)) return false;
-      dev::choose_plain_launch((int)p.dtype, pr.kernel_pin, mc, ncols, v.K, v.H, ex.num_sms, &pc.kernel, &pc.splits,
-                               &pc.chunk);
+      dev::choose_plain_launch((int)p.dtype, pr.kernel_pin, mc, ncols, v.K, v.H, ex.num_sms, pr.hints, &pc.kernel,
+                               &pc.splits, &pc.chunk);
       if (pc.splits > 1) return false;
       if (dev::is_packed_kernel(pc.kernel))
         scratch = std::max(scratch,
@@ -1107,6 +1140,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
     check_cuda(cudaStreamWaitEvent(ex.stream, ev[1 + c], 0), "cudaStreamWaitEvent");
     dev::GemmArgs gc = g;
     const int64_t x0 = lo[c] * inner;
+    if (x0 % 4 != 0) gc.a_vec = gc.b_vec = 0;  // the groups no longer start at the chunk's first row
     if (rows) {
       gc.M = chunk_m(c);
       gc.s.a_m += x0;
@@ -1226,7 +1260,7 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
   if (tune) {
     // Room for the largest candidate, and for a copy of D when the call reads it.
     size_t tune_scratch = scratch;
-    for (const auto& c : plain_candidates(dt_code(pr), pr.view.M, pr.view.N, pr.view.K, pr.view.H, ex.num_sms))
+    for (const auto& c : plain_candidates(dt_code(pr), pr.view.M, pr.view.N, pr.view.K, pr.view.H, ex.num_sms, pr.hints))
       tune_scratch = std::max(tune_scratch, plain_scratch(c, pr));
     if (in_place) {
       span_bytes(p, SD, &d_lo, &d_bytes);

@@ -147,6 +147,9 @@ struct Product {
   bool executed = false;
   // Batch strides of the oriented view for the tiny batched kernel.
   dev::TinyStrides tiny_h{};
+  // Layout facts of the oriented view for the launch choice (a_vec, b_vec: whole
+  // aligned 16-byte groups relative to the operand's origin).
+  dev::LaunchHints hints;
   // Unique over the process lifetime (never reused, unlike the address), so a
   // cached grouped graph can never be replayed for a newer plan.
   const uint64_t uid;
@@ -244,7 +247,8 @@ std::string tune_key(const Product& p, bool c_read);
 // Plain-path candidates for a shape: every tile family of the dtype, each with
 // the split-K factors that keep at most four CTAs per SM in flight, and the
 // tiny batched kernel where it applies. The model's choice comes first.
-std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms);
+std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms,
+                                          const dev::LaunchHints& hints);
 // The model's choice (heuristics), honouring the tile and split pins.
 PlainChoice model_choice(const Product& p, int num_sms);
 // Scratch bytes a plain choice needs (split-K partials).
