@@ -88,7 +88,9 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
   // The model's choice first (ties go to it).
   {
     PlainChoice m;
-    if (dev::use_tiny_batched(M, N, K, H)) {
+    if (dev::use_small_batched(M, N, K, H, hints)) {
+      m.kernel = dev::PLAIN_SMALL_BATCHED;
+    } else if (dev::use_tiny_batched(M, N, K, H)) {
       m.tiny = true;
     } else {
       dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, hints, &m.kernel, &m.splits, &m.chunk);
@@ -134,6 +136,10 @@ PlainChoice model_choice(const Product& p, int num_sms) {
   const OrientedView& v = p.view;
   const int dt = (int)p.problem.dtype;
   PlainChoice c;
+  if (!p.kernel_pin && !p.split_pin && dev::use_small_batched(v.M, v.N, v.K, v.H, p.hints)) {
+    c.kernel = dev::PLAIN_SMALL_BATCHED;
+    return c;
+  }
   if (!p.kernel_pin && !p.split_pin && dev::use_tiny_batched(v.M, v.N, v.K, v.H)) {
     c.tiny = true;
     return c;
@@ -169,6 +175,7 @@ bool choice_fits(const PlainChoice& c, const Product& p) {
   bool fam_ok = false;
   for (int f : kFamilies[(int)p.problem.dtype & 3]) fam_ok = fam_ok || (f != 0 && f == c.kernel);
   fam_ok = fam_ok || (dev::is_stream_kernel(c.kernel) && dev::stream_dtype(c.kernel) == (int)p.problem.dtype && K > 0);
+  if (c.kernel == dev::PLAIN_SMALL_BATCHED) return dev::small_batched_fits(M, N, K, H) && c.splits == 1;
   if (!fam_ok || c.splits < 1) return false;
   if (dev::is_packed_kernel(c.kernel) && !dev::packed_fits(c.kernel, M, N, K, H)) return false;
   if (c.splits == 1) return c.chunk == 0 || c.chunk >= K;
@@ -244,7 +251,7 @@ TuningFile parse_tuning_text(const std::string& text) {
                              e.tried);
       ok = ok &&
            (tiny != 0 || (e.choice.kernel >= 1 && e.choice.kernel <= dev::PLAIN_LAST) ||
-            dev::is_stream_kernel(e.choice.kernel)) &&
+            dev::is_stream_kernel(e.choice.kernel) || e.choice.kernel == dev::PLAIN_SMALL_BATCHED) &&
            e.choice.splits >= 1 && e.choice.splits <= 64 && e.choice.chunk >= 0 &&
            (e.choice.splits == 1 || e.choice.chunk > 0);
     } else if (ok && kind == "list") {

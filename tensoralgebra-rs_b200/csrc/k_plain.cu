@@ -1254,6 +1254,7 @@ dim3 grid_for(const GemmArgs& g) {
 
 const char* plain_kernel_name(int k) {
   if (is_stream_kernel(k)) return stream_kernel_name(k);
+  if (k == PLAIN_SMALL_BATCHED) return "sm100.small-batched";
   switch (k) {
     case PLAIN_F32_SIMT_128x128: return "sm100.f32.simt.128x128x16";
     case PLAIN_F32_SIMT_64x64: return "sm100.f32.simt.64x64x16";

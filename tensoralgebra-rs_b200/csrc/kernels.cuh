@@ -106,6 +106,8 @@ enum PlainKernel : int {
   PLAIN_F64_STREAM_64x48 = 23,
   PLAIN_F64_STREAM_32x128 = 24,
   PLAIN_STREAM_LAST = 24,
+  // Batches of small products (k_small.cu): chosen by the model, never pinned.
+  PLAIN_SMALL_BATCHED = 40,
 };
 
 // dtype: 0 f32, 1 f64, 2 c32, 3 c64 (TAPP numbering).
@@ -152,6 +154,7 @@ const char* plain_kernel_name(int kernel);
 // (the stream tiles are then not chosen).
 struct LaunchHints {
   bool a_gather = false, b_gather = false, a_vec = false, b_vec = false, d_mfast = true;
+  bool h_inner = false;  // the batch index has the smallest stride of A', B' and D
 };
 // The family the autotuner would pick for a shape (no launch).
 int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
@@ -166,6 +169,35 @@ inline bool use_tiny_batched(int64_t M, int64_t N, int64_t K, int64_t H) {
   return M * N * K <= 256 && H >= 64;
 }
 cudaError_t launch_tiny_batched(int dtype, const GemmArgs& g, const TinyStrides& hs, int num_sms, cudaStream_t st);
+
+// Batches of small products with whole products in shared memory (k_small.cu).
+struct SmallIndex {
+  int64_t n = 0;         // extent (the batch's is not used)
+  int64_t lead = 0;      // first step
+  int64_t stride = 0;    // step of a regular vector from 0
+  const int64_t* vec = nullptr;
+};
+struct SmallLayout {
+  SmallIndex h_a, a_m, a_k, h_b, b_n, b_k, h_d, d_m, d_n, h_c, c_m, c_n;
+  bool regular = false;  // every vector is an arithmetic sequence from 0
+};
+inline bool small_batched_fits(int64_t M, int64_t N, int64_t K, int64_t H) {
+  return M >= 1 && N >= 1 && K >= 1 && M <= 32 && N <= 32 && K <= 32 && H < ((int64_t)1 << 31);
+}
+// Whether the model takes them. They read each element once where the tiny
+// kernel reads it once per output it enters, and where a tile kernel pads every
+// product to its tile. B200, us per call: f64 65536 products of 4^3 14.6 against
+// 43.8 (tiny), c64 131072 of 3^3 18.7 against 47.6 (tiny), f64 8192 of 32 x 4 x 32
+// 21.9 against 74.8 (tiles), f32 100000 of 5 x 7 x 13 24 against 4312 (tiles). The
+// tiny kernel stays the faster one for products with next to no reuse (f32 200000
+// of 12 x 1 x 1 21 against 36, of 1 x 1 x 30 25 against 31) and where the batch is
+// innermost in all operands, as its lanes then read consecutive elements (f64 65536
+// of 4^3 14.4 against 15.0). Few products do not fill the groups.
+inline bool use_small_batched(int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints) {
+  return small_batched_fits(M, N, K, H) && H >= 256 && M * N * K >= 48 &&
+         !(hints.h_inner && use_tiny_batched(M, N, K, H));
+}
+cudaError_t launch_small_batched(int dtype, const GemmArgs& g, const SmallLayout& L, cudaStream_t st);
 
 // Family of an item inside a grouped launch (the list fills the GPU).
 int choose_grouped_kernel(int dtype, int64_t M, int64_t N, int64_t K);

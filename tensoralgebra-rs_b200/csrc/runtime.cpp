@@ -179,11 +179,40 @@ Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1))
   const int64_t v = 16 / (int64_t)dtype_size(problem.dtype);
   const std::vector<int64_t>&af = view.a_kfast ? view.a_k : view.a_m, &as = view.a_kfast ? view.a_m : view.a_k;
   const std::vector<int64_t>&bf = view.b_kfast ? view.b_k : view.b_n, &bs = view.b_kfast ? view.b_n : view.b_k;
+  small.regular = true;
+  const auto small_index = [&](const std::vector<int64_t>& x) {
+    dev::SmallIndex i;
+    i.n = (int64_t)x.size();
+    i.lead = x.size() > 1 ? x[1] - x[0] : 0;
+    i.stride = sequence_stride(x);
+    small.regular = small.regular && i.stride != INT64_MIN;
+    return i;
+  };
+  if (dev::small_batched_fits(view.M, view.N, view.K, view.H)) {
+    small.h_a = small_index(view.h_a);
+    small.a_m = small_index(view.a_m);
+    small.a_k = small_index(view.a_k);
+    small.h_b = small_index(view.h_b);
+    small.b_n = small_index(view.b_n);
+    small.b_k = small_index(view.b_k);
+    small.h_d = small_index(view.h_d);
+    small.d_m = small_index(view.d_m);
+    small.d_n = small_index(view.d_n);
+    small.h_c = small_index(view.h_c);
+    small.c_m = small_index(view.c_m);
+    small.c_n = small_index(view.c_n);
+  }
   hints.a_vec = vector_groups(af, as, view.h_a, v);
   hints.b_vec = vector_groups(bf, bs, view.h_b, v);
   hints.a_gather = mostly_unit(af);
   hints.b_gather = mostly_unit(bf);
   hints.d_mfast = view.d_mfast;
+  const auto step = [](const std::vector<int64_t>& x) {
+    return x.size() > 1 ? (uint64_t)std::llabs(x[1] - x[0]) : UINT64_MAX;
+  };
+  hints.h_inner = step(view.h_a) < std::min(step(view.a_m), step(view.a_k)) &&
+                  step(view.h_b) < std::min(step(view.b_n), step(view.b_k)) &&
+                  step(view.h_d) < std::min(step(view.d_m), step(view.d_n));
   signature = problem_signature(*this);
 }
 
@@ -512,6 +541,18 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, const Plain
   if (c.tiny) {
     Timed t(ex, "tiny_batched");
     check_cuda(dev::launch_tiny_batched(dt, g, pr.tiny_h, ex.num_sms, ex.stream), "tiny batched launch");
+    return;
+  }
+  if (c.kernel == dev::PLAIN_SMALL_BATCHED) {
+    dev::SmallLayout L = pr.small;
+    const struct {
+      dev::SmallIndex& i;
+      const int64_t* v;
+    } vec[] = {{L.h_a, g.s.h_a}, {L.a_m, g.s.a_m}, {L.a_k, g.s.a_k}, {L.h_b, g.s.h_b}, {L.b_n, g.s.b_n}, {L.b_k, g.s.b_k},
+               {L.h_d, g.s.h_d}, {L.d_m, g.s.d_m}, {L.d_n, g.s.d_n}, {L.h_c, g.s.h_c}, {L.c_m, g.s.c_m}, {L.c_n, g.s.c_n}};
+    for (auto& x : vec) x.i.vec = x.v;
+    Timed t(ex, dev::plain_kernel_name(c.kernel));
+    check_cuda(dev::launch_small_batched(dt, g, L, ex.stream), "small batched launch");
     return;
   }
   if (dev::is_packed_kernel(c.kernel)) {

@@ -147,6 +147,7 @@ struct Product {
   bool executed = false;
   // Batch strides of the oriented view for the tiny batched kernel.
   dev::TinyStrides tiny_h{};
+  dev::SmallLayout small;  // device vectors filled in per launch
   // Layout facts of the oriented view for the launch choice (a_vec, b_vec: whole
   // aligned 16-byte groups relative to the operand's origin).
   dev::LaunchHints hints;
