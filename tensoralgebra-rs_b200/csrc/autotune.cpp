@@ -132,11 +132,12 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
   return out;
 }
 
-PlainChoice model_choice(const Product& p, int num_sms) {
+PlainChoice model_choice(const Product& p, int num_sms, bool general) {
   const OrientedView& v = p.view;
+  const dev::LaunchHints hints = general ? dev::LaunchHints{} : p.hints;
   const int dt = (int)p.problem.dtype;
   PlainChoice c;
-  if (!p.kernel_pin && !p.split_pin && dev::use_small_batched(v.M, v.N, v.K, v.H, p.hints)) {
+  if (!p.kernel_pin && !p.split_pin && dev::use_small_batched(v.M, v.N, v.K, v.H, hints)) {
     c.kernel = dev::PLAIN_SMALL_BATCHED;
     return c;
   }
@@ -145,7 +146,7 @@ PlainChoice model_choice(const Product& p, int num_sms) {
     return c;
   }
   if (p.split_pin > 0) {
-    c.kernel = p.kernel_pin ? p.kernel_pin : dev::choose_plain_kernel(dt, v.M, v.N, v.K, v.H, num_sms, p.hints);
+    c.kernel = p.kernel_pin ? p.kernel_pin : dev::choose_plain_kernel(dt, v.M, v.N, v.K, v.H, num_sms, hints);
     if (p.split_pin > 1 && v.K > 1) {
       const int64_t chunk = std::max<int64_t>(64, ((v.K + p.split_pin - 1) / p.split_pin + 63) / 64 * 64);
       const int64_t parts = (v.K + chunk - 1) / chunk;
@@ -156,8 +157,14 @@ PlainChoice model_choice(const Product& p, int num_sms) {
     }
     return c;
   }
-  dev::choose_plain_launch(dt, p.kernel_pin, v.M, v.N, v.K, v.H, num_sms, p.hints, &c.kernel, &c.splits, &c.chunk);
+  dev::choose_plain_launch(dt, p.kernel_pin, v.M, v.N, v.K, v.H, num_sms, hints, &c.kernel, &c.splits, &c.chunk);
   return c;
+}
+
+size_t stream_scratch(const Product& p, int64_t M, int64_t N) {
+  const int dt = (int)p.problem.dtype;
+  return (p.hints.a_gather ? 0 : dev::stream_panel_bytes(dt, M, p.view.K, p.view.H) + 256) +
+         (p.hints.b_gather ? 0 : dev::stream_panel_bytes(dt, N, p.view.K, p.view.H) + 256);
 }
 
 size_t plain_scratch(const PlainChoice& c, const Product& p) {
@@ -165,6 +172,7 @@ size_t plain_scratch(const PlainChoice& c, const Product& p) {
   size_t s = 0;
   if (dev::is_packed_kernel(c.kernel))
     s += dev::packed_workspace_bytes(dev::packed_layout(c.kernel, p.view.M, p.view.N, p.view.K, p.view.H)) + 512;
+  if (dev::is_stream_kernel(c.kernel)) s += stream_scratch(p, p.view.M, p.view.N);
   if (c.splits > 1) s += (size_t)c.splits * p.view.H * p.view.M * p.view.N * dtype_size(p.problem.dtype) + 256;
   return s;
 }

@@ -61,6 +61,9 @@ struct __align__(16) GemmArgs {
   // Every 16-byte group of the operand's fast index is contiguous and aligned
   // (16-byte gathers).
   int a_vec, b_vec;
+  // Non-zero: the operand is a dense panel [H][K][ld], rows fastest, and its
+  // scatter vectors are not read (stream tiles after a pack pass).
+  int64_t a_ld, b_ld;
   Epilogue e;
   unsigned* status;
   // Split-K: each K chunk of k_chunk (a multiple of the tile depth; 0 = all
@@ -105,7 +108,13 @@ enum PlainKernel : int {
   PLAIN_F64_STREAM_128x32 = 22,
   PLAIN_F64_STREAM_64x48 = 23,
   PLAIN_F64_STREAM_32x128 = 24,
-  PLAIN_STREAM_LAST = 24,
+  PLAIN_F32_STREAM_128x64 = 25,
+  PLAIN_F32_STREAM_128x48 = 26,
+  PLAIN_F32_STREAM_128x32 = 27,
+  PLAIN_C32_STREAM_64x64 = 28,
+  PLAIN_C32_STREAM_64x32 = 29,
+  PLAIN_C32_STREAM_64x24 = 30,
+  PLAIN_STREAM_LAST = 30,
   // Batches of small products (k_small.cu): chosen by the model, never pinned.
   PLAIN_SMALL_BATCHED = 40,
 };
@@ -123,6 +132,10 @@ const char* stream_kernel_name(int kernel);
 struct LaunchHints;
 int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste);
 cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
+// Dense panel of one operand (0 = A', 1 = B') for the stream tiles: its bytes, and
+// the pass that writes it and points `g` at it.
+size_t stream_panel_bytes(int dtype, int64_t rows, int64_t K, int64_t H);
+cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, void* panel, cudaStream_t st);
 static_assert(sizeof(GemmArgs) % 16 == 0, "grouped kernels copy GemmArgs in 16-byte words");
 
 // One item of a grouped launch: its arguments and its tile grid.
@@ -148,11 +161,13 @@ cudaError_t launch_wait_selftest(const unsigned* flag, unsigned* status, uint64_
 cudaError_t launch_fill_zero(size_t elem, void* origin, int rank, const int64_t* dims, const int64_t* strides,
                              cudaStream_t st);
 const char* plain_kernel_name(int kernel);
-// What the layout says about a launch beyond its extents: whether gathering an
+// What the layout says about a launch beyond its extents (`known` unset: nothing,
+// and only the families that need no such knowledge are chosen): whether gathering an
 // operand along its fast index is coalesced, whether it splits into aligned
 // 16-byte groups, and which index D is unit-stride in. The default says nothing
 // (the stream tiles are then not chosen).
 struct LaunchHints {
+  bool known = false;
   bool a_gather = false, b_gather = false, a_vec = false, b_vec = false, d_mfast = true;
   bool h_inner = false;  // the batch index has the smallest stride of A', B' and D
 };
@@ -194,7 +209,7 @@ inline bool small_batched_fits(int64_t M, int64_t N, int64_t K, int64_t H) {
 // innermost in all operands, as its lanes then read consecutive elements (f64 65536
 // of 4^3 14.4 against 15.0). Few products do not fill the groups.
 inline bool use_small_batched(int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints) {
-  return small_batched_fits(M, N, K, H) && H >= 256 && M * N * K >= 48 &&
+  return hints.known && small_batched_fits(M, N, K, H) && H >= 256 && M * N * K >= 48 &&
          !(hints.h_inner && use_tiny_batched(M, N, K, H));
 }
 cudaError_t launch_small_batched(int dtype, const GemmArgs& g, const SmallLayout& L, cudaStream_t st);

@@ -202,6 +202,7 @@ Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1))
     small.c_m = small_index(view.c_m);
     small.c_n = small_index(view.c_n);
   }
+  hints.known = true;
   hints.a_vec = vector_groups(af, as, view.h_a, v);
   hints.b_vec = vector_groups(bf, bs, view.h_b, v);
   hints.a_gather = mostly_unit(af);
@@ -535,9 +536,11 @@ void join_side(Executor& ex) {
 }
 
 // One plain execution in the configuration `c` (scratch: the split-K partials).
-void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, const PlainChoice& c, char* scratch,
+void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const PlainChoice& c, char* scratch,
                   size_t scratch_bytes) {
   const int dt = (int)pr.problem.dtype;
+  dev::GemmArgs g = g0;
+  char* const scratch_end = scratch + scratch_bytes;
   if (c.tiny) {
     Timed t(ex, "tiny_batched");
     check_cuda(dev::launch_tiny_batched(dt, g, pr.tiny_h, ex.num_sms, ex.stream), "tiny batched launch");
@@ -598,6 +601,25 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, const Plain
       check_cuda(dev::launch_splitk_reduce(dt, gs, c.splits, ex.stream), "split-K reduce launch");
     }
     return;
+  }
+  if (dev::is_stream_kernel(c.kernel)) {
+    // Complex elements are gathered whole: operands off their natural alignment
+    // take the direct tile.
+    if (dt == 2 && ((reinterpret_cast<uintptr_t>(g0.A) | reinterpret_cast<uintptr_t>(g0.B)) & 7) != 0) {
+      PlainChoice d = c;
+      d.kernel = dev::PLAIN_C32_SIMT_64x64;
+      return launch_plain(pr, ex, g0, d, scratch, scratch_bytes);
+    }
+    for (int which = 0; which < 2; ++which) {
+      if (which == 0 ? pr.hints.a_gather : pr.hints.b_gather) continue;
+      const size_t bytes = dev::stream_panel_bytes(dt, which == 0 ? g.M : g.N, g.K, g.H);
+      char* panel = reinterpret_cast<char*>(align_up((uintptr_t)scratch, 256));
+      if (panel + bytes > scratch_end) throw Error(ERR_INTERNAL, "stream panel workspace too small");
+      Timed t(ex, "stream_pack");
+      check_cuda(dev::launch_stream_pack(dt, g, which, panel, ex.stream), "stream pack launch");
+      scratch = panel + bytes;
+    }
+    scratch_bytes = (size_t)(scratch_end - scratch);
   }
   if (c.splits > 1) {
     // Split-K: partial tiles into the scratch, then the reduce + epilogue.
@@ -1097,6 +1119,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
       if (dev::is_packed_kernel(pc.kernel))
         scratch = std::max(scratch,
                            dev::packed_workspace_bytes(dev::packed_layout(pc.kernel, mc, ncols, v.K, v.H)) + 512);
+      if (dev::is_stream_kernel(pc.kernel)) scratch = std::max(scratch, stream_scratch(pr, mc, ncols));
     }
     return true;
   };
@@ -1296,6 +1319,12 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
     }
   }
   size_t scratch = output_only ? 0 : scheme_scratch(pr, pc, ex.num_sms);
+  if (pr.scheme == Scheme::Plain && !output_only && !pr.kernel_pin &&
+      align_up(total, 256) + align_up(scratch, 256) + 1024 > ex.ws_limit) {
+    // Beyond the workspace cap: the choice that needs no layout hints.
+    pc = model_choice(pr, ex.num_sms, true);
+    scratch = scheme_scratch(pr, pc, ex.num_sms);
+  }
   int64_t d_lo = 0;
   size_t d_bytes = 0, snap = 0;
   if (tune) {

@@ -251,7 +251,10 @@ std::string tune_key(const Product& p, bool c_read);
 std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms,
                                           const dev::LaunchHints& hints);
 // The model's choice (heuristics), honouring the tile and split pins.
-PlainChoice model_choice(const Product& p, int num_sms);
+// `general`: without the layout's hints (the families that take any layout).
+PlainChoice model_choice(const Product& p, int num_sms, bool general = false);
+// Dense panels of the operands whose gather is not coalesced (stream tiles).
+size_t stream_scratch(const Product& p, int64_t M, int64_t N);
 // Scratch bytes a plain choice needs (split-K partials).
 size_t plain_scratch(const PlainChoice& c, const Product& p);
 // Whether a choice (from a tuning-cache file, say) is valid for a product: a
