@@ -93,7 +93,11 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
     } else if (dev::use_tiny_batched(M, N, K, H)) {
       m.tiny = true;
     } else {
-      dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, hints, &m.kernel, &m.splits, &m.chunk);
+      // The families a caller can name; the tensor-core stream tiles, where the
+      // model takes them, are timed beside these (autotune_plain).
+      dev::LaunchHints named = hints;
+      named.off32 = false;
+      dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, named, &m.kernel, &m.splits, &m.chunk);
     }
     out.push_back(m);
   }
@@ -172,7 +176,7 @@ size_t plain_scratch(const PlainChoice& c, const Product& p) {
   size_t s = 0;
   if (dev::is_packed_kernel(c.kernel))
     s += dev::packed_workspace_bytes(dev::packed_layout(c.kernel, p.view.M, p.view.N, p.view.K, p.view.H)) + 512;
-  if (dev::is_stream_kernel(c.kernel)) s += stream_scratch(p, p.view.M, p.view.N);
+  if (dev::is_tc_stream(c.kernel)) s += stream_scratch(p, p.view.M, p.view.N);
   if (c.splits > 1) s += (size_t)c.splits * p.view.H * p.view.M * p.view.N * dtype_size(p.problem.dtype) + 256;
   return s;
 }
@@ -182,7 +186,9 @@ bool choice_fits(const PlainChoice& c, const Product& p) {
   if (c.tiny) return dev::use_tiny_batched(M, N, K, H) && c.splits == 1;
   bool fam_ok = false;
   for (int f : kFamilies[(int)p.problem.dtype & 3]) fam_ok = fam_ok || (f != 0 && f == c.kernel);
-  fam_ok = fam_ok || (dev::is_stream_kernel(c.kernel) && dev::stream_dtype(c.kernel) == (int)p.problem.dtype && K > 0);
+  fam_ok = fam_ok || (dev::is_stream_kernel(c.kernel) && dev::stream_dtype(c.kernel) == (int)p.problem.dtype && K > 0 &&
+                       (!dev::is_tc_stream(c.kernel) ||
+                        (c.splits == 1 && dev::tc_stream_fits((int)p.problem.dtype, M, N, K, H, p.hints))));
   if (c.kernel == dev::PLAIN_SMALL_BATCHED) return dev::small_batched_fits(M, N, K, H) && c.splits == 1;
   if (!fam_ok || c.splits < 1) return false;
   if (dev::is_packed_kernel(c.kernel) && !dev::packed_fits(c.kernel, M, N, K, H)) return false;

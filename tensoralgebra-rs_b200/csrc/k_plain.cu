@@ -1291,31 +1291,23 @@ bool packed_fits(int kernel, int64_t M, int64_t N, int64_t K, int64_t H) {
 
 int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
   auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * H; };
-  // Stream tiles (at least a wave of tiles) against the packed family, f64 on
-  // B200: 177147 x 243 x 50 0.207 ms against 0.290 (direct tile 0.295); 64 x 256^3
-  // 0.089 against 0.120; 2048^2 x 512 0.162 against 0.183; 2048^3 0.622 against
-  // 0.604. Above K = 512 they are chosen where their tile pads less (136856 x 22 x
-  // 240: 0.092 against 0.273). An operand whose gather is not coalesced is copied
-  // to a dense panel first (f32, c32), where the panels are small beside the output.
+  // Stream tiles (gathers coalesced on both sides, at least a wave of tiles)
+  // against the packed family, f64 on B200: 177147 x 243 x 50 0.207 ms against
+  // 0.290 (direct tile 0.295); 64 x 256^3 0.089 against 0.120; 2048^2 x 512 0.162
+  // against 0.183; 2048^3 0.622 against 0.604. Above K = 512 they are chosen where
+  // their tile pads less (136856 x 22 x 240: 0.092 against 0.273).
   const bool gather = hints.a_gather && hints.b_gather;
-  const bool panels = (dtype == 0 || dtype == 2) && K >= 8 &&
-                      ((hints.a_gather ? 0 : M) + (hints.b_gather ? 0 : N)) * K * 8 <= M * N;
-  if (hints.known && (gather || panels) && K > 0) {
+  if (hints.known && dtype == 1 && gather && K > 0) {
     double waste = 0;
     const int sk = choose_stream_kernel(dtype, M, N, hints, &waste);
     if (sk) {
-      static const int other[4] = {PLAIN_F32_PACKED_128x128, PLAIN_F64_PACKED_64x64, PLAIN_C32_PACKED_1M_64x64,
-                                   PLAIN_C64_PACKED_3M_64x32};
       int bm = 0, bn = 0, pm = 0, pn = 0;
       plain_tile_shape(sk, &bm, &bn);
-      plain_tile_shape(other[dtype & 3], &pm, &pn);
+      plain_tile_shape(PLAIN_F64_PACKED_64x64, &pm, &pn);
       const bool swap = !hints.d_mfast;
       const int64_t t = swap ? ((N + bm - 1) / bm) * ((M + bn - 1) / bn) * H : tiles(bm, bn);
       const double pwaste = (double)((M + pm - 1) / pm * pm) * (double)((N + pn - 1) / pn * pn) / ((double)M * (double)N);
-      // FFMA (f32, c32; the producer warp's element copies of a k-fast operand
-      // bound a deep K): 2048^2 x 64 f32 30 us against 32 packed, x 256 87 against
-      // 68; c32 66 against 74, 220 against 215.
-      const int64_t deep = dtype != 1 ? 96 : hints.a_vec && hints.b_vec ? 512 : 256;
+      const int64_t deep = hints.a_vec && hints.b_vec ? 512 : 256;
       if (t >= num_sms && (K <= deep || waste * 1.25 < pwaste)) return sk;
     }
   }
@@ -1387,6 +1379,10 @@ void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K,
                                 PLAIN_C64_PACKED_3M_64x32};
   *splits = 1;
   *k_chunk = 0;
+  if (!pinned && use_tc_stream(dtype, M, N, K, H, num_sms, hints)) {
+    *kernel = dtype == 0 ? PLAIN_F32_TC_STREAM : PLAIN_C32_TC_STREAM;
+    return;
+  }
   const int64_t min_chunk = 512;  // K per split
   // Small f64 products (at most 64 large tiles, K up to 1024): the small direct
   // tile, K split until about two CTAs run per SM, without a pack pass (399 x 108

@@ -78,12 +78,12 @@ struct StageGather {
   static constexpr int RREG = (ROWS + 31) / 32, V = 16 / ES;
   int64_t off[RREG];  // row lane + 32 j
 
-  __device__ __forceinline__ void init(const int64_t* rows, int64_t r0, int64_t nrows, int64_t ld, int lane) {
+  __device__ __forceinline__ void init(const int64_t* rows, int64_t r0, int64_t nrows, int lane) {
     const int64_t last = nrows - 1 - r0;
 #pragma unroll
     for (int j = 0; j < RREG; ++j) {
-      const int64_t r = r0 + min((int64_t)(lane + 32 * j), last);
-      off[j] = (ld ? r : __ldg(rows + r)) * ES;
+      const int64_t r = lane + 32 * j;
+      off[j] = __ldg(rows + r0 + (r < last ? r : last)) * ES;
     }
   }
   __device__ __forceinline__ int64_t row_off(int r) const {  // r / 32 uniform and known at compile time
@@ -334,193 +334,6 @@ struct StreamF64 {
   }
 };
 
-// FP32 pairs (sm_100 f32x2 arithmetic; each half rounds as its own operation).
-__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpair2(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-// f32 and c32 on the FFMA pipe: WGM x WGN warps. A lane holds two groups of
-// consecutive rows (16 bytes each: four real, two complex) and TN consecutive
-// columns, lanes 8 along the rows by 4 along the columns, so a k costs a warp two
-// shared-memory wavefronts for A and one or two for B against 2 TN (real) or 4 TN
-// (complex) FFMA cycles per SM sub-core and group. Pairs of FMAs are
-// (row, row + 1) for f32 and, for c32, (re, im) of a row times B's real part in one
-// accumulator and times its imaginary part in a second; their halves are combined
-// (with the conjugations as signs) when the stage's sums are added to the totals.
-// The sums restart every stage (16 k), as in the direct tiles.
-template <bool CPLX, int WGM, int WGN, int TN, int STG, int MINB_>
-struct StreamFma {
-  static constexpr bool SWZ = false;
-  static constexpr int ES = CPLX ? 8 : 4, WARPS = WGM * WGN, V = CPLX ? 2 : 4;  // rows of a group
-  static constexpr int BM = WGM * 16 * V, BN = WGN * 4 * TN, BK = 16;
-  static constexpr int SA = BM + V, SB = (BN + V - 1) / V * V + V;
-  static constexpr int STAGES = STG, MINB = MINB_;
-  static constexpr int A_BYTES = BK * SA * ES, B_BYTES = BK * SB * ES;
-  static constexpr int NA = CPLX ? 2 : 1;  // accumulators per pair
-  using u64 = unsigned long long;
-
-  u64 tot[4][TN];
-  int m0, n0;  // the lane's first row and column of the tile
-  float s1, s2, s3;
-
-  __device__ __forceinline__ StreamFma(int warp, int lane)
-      : m0((warp % WGM) * 16 * V + (lane & 7) * V), n0((warp / WGM) * 4 * TN + (lane >> 3) * TN) {}
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) tot[i][j] = 0ull;
-  }
-  __device__ __forceinline__ void tile_begin(const GemmArgs& g) {
-    s2 = g.conj_a ? -1.f : 1.f;
-    s3 = g.conj_b ? -1.f : 1.f;
-    s1 = -s2 * s3;
-  }
-  __device__ __forceinline__ void k1(u64 (&acc)[NA][4][TN], const char* A, const char* B) const {
-    u64 a[4];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(A + 8 * V * q * ES);
-      a[2 * q] = v.x;
-      a[2 * q + 1] = v.y;
-    }
-    float b[NA * TN];
-    if constexpr (NA * TN % 4 == 0) {
-#pragma unroll
-      for (int j = 0; j < NA * TN / 4; ++j) {
-        const float4 v = *reinterpret_cast<const float4*>(B + 16 * j);
-        b[4 * j] = v.x;
-        b[4 * j + 1] = v.y;
-        b[4 * j + 2] = v.z;
-        b[4 * j + 3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < NA * TN / 2; ++j) {
-        const float2 v = *reinterpret_cast<const float2*>(B + 8 * j);
-        b[2 * j] = v.x;
-        b[2 * j + 1] = v.y;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < TN; ++j)
-#pragma unroll
-      for (int p = 0; p < NA; ++p) {
-        const u64 d = pair2(b[NA * j + p], b[NA * j + p]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) fma2(acc[p][i][j], a[i], d);
-      }
-  }
-  __device__ __forceinline__ void stage(const char* sA, const char* sB, int kv) {
-    const char* A = sA + m0 * ES;
-    const char* B = sB + n0 * ES;
-    u64 acc[NA][4][TN];
-#pragma unroll
-    for (int p = 0; p < NA; ++p)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[p][i][j] = 0ull;
-    if (kv == BK) {
-#pragma unroll
-      for (int kk = 0; kk < BK; ++kk) k1(acc, A + kk * SA * ES, B + kk * SB * ES);
-    } else {
-#pragma unroll 2
-      for (int kk = 0; kk < kv; ++kk) k1(acc, A + kk * SA * ES, B + kk * SB * ES);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        if constexpr (CPLX) {
-          const float2 p = unpair2(acc[0][i][j]), q = unpair2(acc[NA - 1][i][j]);
-          tot[i][j] = add2(tot[i][j], pair2(fmaf(s1, q.y, p.x), fmaf(s2, p.y, s3 * q.x)));
-        } else {
-          tot[i][j] = add2(tot[i][j], acc[0][i][j]);
-        }
-      }
-  }
-  // Row r of the lane's (0 .. 2 V - 1) in the tile.
-  __device__ __forceinline__ int row(int r) const { return m0 + (r / V) * 8 * V + r % V; }
-  __device__ __forceinline__ void value(int r, int j, float& re, float& im) const {
-    const float2 v = unpair2(tot[CPLX ? r : r / 2][j]);
-    re = CPLX ? v.x : (r & 1) ? v.y : v.x;
-    im = CPLX ? v.y : 0.f;
-  }
-  __device__ __forceinline__ void store(const GemmArgs& g, const TileSlot<BM, BN>& s) {
-    using T = typename Elem<float, CPLX>::type;
-    const int mrem = (int)min((int64_t)BM, g.M - s.m0), nrem = (int)min((int64_t)BN, g.N - s.n0);
-    if (g.partial) {
-      T* P = static_cast<T*>(g.partial) + ((s.split * g.H + s.h) * g.N + s.n0) * g.M + s.m0;
-#pragma unroll
-      for (int r = 0; r < 2 * V; ++r)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          float re, im;
-          value(r, j, re, im);
-          if (row(r) < mrem && n0 + j < nrem) Elem<float, CPLX>::store(P + (n0 + j) * g.M + row(r), re, im);
-        }
-      return;
-    }
-    const Epilogue e = g.e;
-    T* Db = static_cast<T*>(g.D) + g.s.h_d[s.h];
-    const T* Cb = static_cast<const T*>(g.C) + (e.beta_zero ? 0 : g.s.h_c[s.h]);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int rr = row(q * V);
-      const int64_t dm = s.dm[rr];
-      // A whole group consecutive in D (the rows past the end repeat the last
-      // offset, so their groups are not).
-      bool run = e.beta_zero != 0 && rr + V <= mrem;
-#pragma unroll
-      for (int i = 1; i < V; ++i) run = run && s.dm[rr + i] == dm + i;
-      if (CPLX) run = run && e.plain != 0;
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const int cc = n0 + j;
-        if (cc >= nrem) continue;
-        T* d = Db + dm + s.dn[cc];
-        if (run && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
-          ulonglong2 v = make_ulonglong2(tot[2 * q][j], tot[2 * q + 1][j]);
-          if (!CPLX && !e.plain) {
-            const float al = (float)e.alpha_re;
-            const float2 x = unpair2(v.x), y = unpair2(v.y);
-            v = make_ulonglong2(pair2(x.x * al, x.y * al), pair2(y.x * al, y.y * al));
-          }
-          *reinterpret_cast<ulonglong2*>(d) = v;
-          continue;
-        }
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          if (rr + i >= mrem) continue;
-          float re, im;
-          value(q * V + i, j, re, im);
-          T* di = Db + s.dm[rr + i] + s.dn[cc];
-          if (e.plain && CPLX && (reinterpret_cast<uintptr_t>(di) & 7) == 0)
-            *reinterpret_cast<float2*>(di) = make_float2(re, im);
-          else
-            epilogue_store<float, CPLX>(e, re, im, Cb + s.cm[rr + i] + s.cn[cc], di);
-        }
-      }
-    }
-  }
-};
-
 template <class Op>
 struct StreamSmem {
   static constexpr int STAGE = Op::A_BYTES + Op::B_BYTES;
@@ -658,13 +471,13 @@ stream_kernel(const __grid_constant__ GemmArgs gp, const GroupItem* __restrict__
         n0 = nt * BN;
         kb = g.k_chunk ? split * g.k_chunk : 0;
         kspan = (g.k_chunk ? min(g.K, kb + g.k_chunk) : g.K) - kb;
-        ga.init(g.s.a_m, m0, g.M, g.a_ld, lane);
-        gb.init(g.s.b_n, n0, g.N, g.b_ld, lane);
+        ga.init(g.s.a_m, m0, g.M, lane);
+        gb.init(g.s.b_n, n0, g.N, lane);
         const int64_t k0 = kb + (klane < kspan ? klane : 0);
-        ka = (g.a_ld ? k0 * g.a_ld : __ldg(g.s.a_k + k0)) * ES;
-        kbr = (g.b_ld ? k0 * g.b_ld : __ldg(g.s.b_k + k0)) * ES;
-        ha = (g.a_ld ? h * g.K * g.a_ld : __ldg(g.s.h_a + h)) * ES;
-        hb = (g.b_ld ? h * g.K * g.b_ld : __ldg(g.s.h_b + h)) * ES;
+        ka = __ldg(g.s.a_k + k0) * ES;
+        kbr = __ldg(g.s.b_k + k0) * ES;
+        ha = __ldg(g.s.h_a + h) * ES;
+        hb = __ldg(g.s.h_b + h) * ES;
       }
       const int nk = end ? 0 : (int)((kspan + BK - 1) / BK), kvl = (int)(kspan - (int64_t)(nk - 1) * BK);
       // The slot's previous tile has been written back.
@@ -714,14 +527,13 @@ stream_kernel(const __grid_constant__ GemmArgs gp, const GroupItem* __restrict__
       const char* Bb = static_cast<const char*>(g.B) + hb;
       const int64_t* ak = g.s.a_k + kb + klane;
       const int64_t* bk = g.s.b_k + kb + klane;
-      const int64_t a_ld = g.a_ld, b_ld = g.b_ld;
       bool alive = true;
       for (int i = 0; i < nk; ++i) {
         const int64_t kac = ka, kbc = kbr;
         const int64_t kn = (int64_t)(i + 1) * BK;
         if (kn + klane < kspan) {
-          ka = a_ld ? ka + BK * a_ld * ES : __ldg(ak + kn) * ES;
-          kbr = b_ld ? kbr + BK * b_ld * ES : __ldg(bk + kn) * ES;
+          ka = __ldg(ak + kn) * ES;
+          kbr = __ldg(bk + kn) * ES;
         }
         if (!mbar_wait(&empty[stage], (sround & 1u) ^ 1u)) {
           alive = false;
@@ -806,13 +618,6 @@ using SF64_128x32 = StreamF64<4, 1, 2, 4, 3, 3>;
 using SF64_64x48 = StreamF64<4, 1, 1, 6, 4, 3>;
 using SF64_32x128 = StreamF64<1, 4, 2, 4, 3, 3>;
 
-using SF32_128x64 = StreamFma<false, 2, 4, 4, 4, 2>;
-using SF32_128x48 = StreamFma<false, 2, 3, 4, 4, 2>;
-using SF32_128x32 = StreamFma<false, 2, 2, 4, 4, 4>;
-using SC32_64x64 = StreamFma<true, 2, 4, 4, 4, 1>;
-using SC32_64x32 = StreamFma<true, 2, 2, 4, 4, 2>;
-using SC32_64x24 = StreamFma<true, 2, 2, 3, 4, 3>;
-
 // The roles of A' and B' (and of the output's rows and columns) exchanged.
 GemmArgs swapped(const GemmArgs& g) {
   GemmArgs t = g;
@@ -853,39 +658,8 @@ struct StreamFamily {
 const StreamFamily kStream[] = {
     {1, 64, 64, "sm100.f64.dmma884.stream.64x64x16"},   {1, 128, 32, "sm100.f64.dmma884.stream.128x32x16"},
     {1, 64, 48, "sm100.f64.dmma884.stream.64x48x16"},   {1, 32, 128, "sm100.f64.dmma884.stream.32x128x16"},
-    {0, 128, 64, "sm100.f32.simt.stream.128x64x16"},    {0, 128, 48, "sm100.f32.simt.stream.128x48x16"},
-    {0, 128, 32, "sm100.f32.simt.stream.128x32x16"},    {2, 64, 64, "sm100.c32.simt.stream.64x64x16"},
-    {2, 64, 32, "sm100.c32.simt.stream.64x32x16"},      {2, 64, 24, "sm100.c32.simt.stream.64x24x16"},
+    {0, 128, 128, "sm100.f32.tcgen05.stream.128x128x32"}, {2, 64, 128, "sm100.c32.tcgen05.stream.64x128x32"},
 };
-
-// Copy of an operand into a dense panel [H][K][ld], rows fastest: one 32-row x
-// 32-k tile per CTA, read along whichever index is the faster one in memory.
-template <class T>
-__global__ void __launch_bounds__(256) stream_pack_kernel(const T* __restrict__ X, const int64_t* __restrict__ rows,
-                                                          const int64_t* __restrict__ ks, const int64_t* __restrict__ hs,
-                                                          int64_t nrows, int64_t K, int64_t H, int64_t ld, int kfast,
-                                                          T* __restrict__ out) {
-  __shared__ T tile[32][33];
-  const int64_t tr = (nrows + 31) / 32, tk = (K + 31) / 32;
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
-  for (int64_t t = blockIdx.x; t < tr * tk * H; t += gridDim.x) {
-    const int64_t r0 = t % tr * 32, k0 = t / tr % tk * 32, h = t / tr / tk;
-    const T* base = X + hs[h];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int rr = kfast ? y + 8 * j : x, kk = kfast ? x : y + 8 * j;
-      if (r0 + rr < nrows && k0 + kk < K) tile[kk][rr] = base[rows[r0 + rr] + ks[k0 + kk]];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int kk = y + 8 * j;
-      if (r0 + x < nrows && k0 + kk < K) out[(h * K + k0 + kk) * ld + r0 + x] = tile[kk][x];
-    }
-    __syncthreads();
-  }
-}
-int64_t panel_ld(int64_t rows) { return (rows + 15) / 16 * 16; }
 
 }  // namespace
 
@@ -897,52 +671,15 @@ void stream_tile_shape(int kernel, int* bm, int* bn) {
 int stream_dtype(int kernel) { return kStream[kernel - PLAIN_STREAM_FIRST].dtype; }
 const char* stream_kernel_name(int kernel) { return kStream[kernel - PLAIN_STREAM_FIRST].name; }
 
-size_t stream_panel_bytes(int dtype, int64_t rows, int64_t K, int64_t H) {
-  const int es = dtype == 0 ? 4 : dtype == 3 ? 16 : 8;
-  return (size_t)H * K * panel_ld(rows) * es + 256;
-}
-
-cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, void* panel, cudaStream_t st) {
-  const bool a = which == 0;
-  const int64_t rows = a ? g.M : g.N, ld = panel_ld(rows);
-  const int64_t tiles = ((rows + 31) / 32) * ((g.K + 31) / 32) * g.H;
-  const unsigned grid = (unsigned)(tiles < 4096 ? tiles : 4096);
-  const int64_t *rs = a ? g.s.a_m : g.s.b_n, *ks = a ? g.s.a_k : g.s.b_k, *hs = a ? g.s.h_a : g.s.h_b;
-  const void* X = a ? g.A : g.B;
-  const int kfast = a ? g.a_kfast : g.b_kfast;
-  if (dtype == 0)
-    stream_pack_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(X), rs, ks, hs, rows, g.K, g.H, ld, kfast,
-                                                    static_cast<float*>(panel));
-  else if (dtype == 3)
-    return cudaErrorInvalidValue;
-  else
-    stream_pack_kernel<double><<<grid, 256, 0, st>>>(static_cast<const double*>(X), rs, ks, hs, rows, g.K, g.H, ld,
-                                                     kfast, static_cast<double*>(panel));
-  if (a) {
-    g.A = panel;
-    g.a_ld = ld;
-    g.a_kfast = 0;
-    g.a_vec = 1;
-  } else {
-    g.B = panel;
-    g.b_ld = ld;
-    g.b_kfast = 0;
-    g.b_vec = 1;
-  }
-  return cudaGetLastError();
-}
-
 // Each family's padded outputs, weighted by its measured time per padded
-// output relative to the dtype's first (B200, 177147 x 243 x 50 f64: 64 x 64 0.207
+// output relative to 64 x 64 (B200, 177147 x 243 x 50 f64: 64 x 64 0.207
 // ms, 128 x 32 0.238, 64 x 48 0.262 on 1.13 times the padded area, 32 x 128 0.211).
 int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste) {
   static const struct {
     int kernel;
     double weight;
   } table[] = {{PLAIN_F64_STREAM_64x64, 1.0},   {PLAIN_F64_STREAM_128x32, 1.15}, {PLAIN_F64_STREAM_64x48, 1.15},
-               {PLAIN_F64_STREAM_32x128, 1.03}, {PLAIN_F32_STREAM_128x64, 1.0},  {PLAIN_F32_STREAM_128x48, 1.05},
-               {PLAIN_F32_STREAM_128x32, 1.1},  {PLAIN_C32_STREAM_64x64, 1.0},   {PLAIN_C32_STREAM_64x32, 1.05},
-               {PLAIN_C32_STREAM_64x24, 1.1}};
+               {PLAIN_F64_STREAM_32x128, 1.03}};
   const int64_t m = hints.d_mfast ? M : N, n = hints.d_mfast ? N : M;  // the launch's roles
   int best = 0;
   for (const auto& f : table) {
@@ -964,16 +701,12 @@ cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g0, cudaSt
   // Rows of the tile run along D's unit-stride index (the lanes' stores).
   const GemmArgs g = !g0.d_mfast && !g0.partial ? swapped(g0) : g0;
   switch (kernel) {
+    case PLAIN_F32_TC_STREAM:
+    case PLAIN_C32_TC_STREAM: return launch_tc_stream(dtype, g, st);
     case PLAIN_F64_STREAM_64x64: return run_stream<SF64_64x64>(g, st);
     case PLAIN_F64_STREAM_128x32: return run_stream<SF64_128x32>(g, st);
     case PLAIN_F64_STREAM_64x48: return run_stream<SF64_64x48>(g, st);
     case PLAIN_F64_STREAM_32x128: return run_stream<SF64_32x128>(g, st);
-    case PLAIN_F32_STREAM_128x64: return run_stream<SF32_128x64>(g, st);
-    case PLAIN_F32_STREAM_128x48: return run_stream<SF32_128x48>(g, st);
-    case PLAIN_F32_STREAM_128x32: return run_stream<SF32_128x32>(g, st);
-    case PLAIN_C32_STREAM_64x64: return run_stream<SC32_64x64>(g, st);
-    case PLAIN_C32_STREAM_64x32: return run_stream<SC32_64x32>(g, st);
-    case PLAIN_C32_STREAM_64x24: return run_stream<SC32_64x24>(g, st);
   }
   return cudaErrorInvalidValue;
 }

@@ -1,0 +1,745 @@
+// f32 and c32 contractions on the tensor cores without a pack pass.
+//
+// The FFMA pipe (72 TFLOP/s) bounds plain f32 tiles; BF16 products run 20 times
+// faster, and an f32 value is exactly the sum of three BF16 values (8 significant
+// bits each), so six BF16 products with FP32 accumulation carry a product to the
+// rounding of f32 (the terms left out are below 2^-26 of it; error against 64 bits
+// at K = 4096: 1.7e-7 against 2.1e-7 of the FFMA tiles, see k_split.cu). Packing the
+// planes through HBM costs 1.5 times the operand's bytes twice, which a short or
+// moderate K does not win back, so here the split happens on the way into shared
+// memory. One persistent CTA per SM, 128 x 128 tiles, 32-deep stages:
+//
+//   warps 0-7   epilogue: drain the TMEM accumulators to registers, write back
+//               (two warps per 32 rows, each half of the columns).
+//   warps 8-23  producers, two sets of eight that take every other block; a warp
+//               owns 32 rows of A' (or B'), loads its elements through the scatter
+//               vectors to registers while the other set splits, splits them and
+//               stores the planes in the tensor core's order (K-major core
+//               matrices, no swizzle; the 16-byte step between depth groups keeps
+//               the stores free of bank conflicts).
+//   warp 24     issues tcgen05.mma: x0 y0 into a main accumulator, restarted every
+//               128 k and added up in FP32 registers, the five cross products into
+//               a correction accumulator (the accumulate of the tensor core
+//               truncates; see k_split.cu).
+//
+// c32 runs as the real product of 2M x N x 2K (rows 2m, 2m + 1 of A' hold [re, -im]
+// and [im, re], depths 2k, 2k + 1 of B' re and im): the embedding is a sign flip and
+// a swap of the split planes, so a complex element is split once.
+//
+// Values that BF16 planes cannot carry: the producers track the largest and the
+// smallest non-zero magnitude of a tile's operands. A tile with an infinity, a NaN
+// or products near overflow is computed again by FFMA straight from the operands,
+// and so is an output small enough to have lost bits to underflow.
+//
+// Every wait is bounded (a status bit, then the role ends). No cluster, no multicast.
+#include "tc_common.cuh"
+
+namespace tprims {
+namespace dev {
+
+namespace {
+
+using namespace tc;
+
+constexpr int TS_BM = 128, TS_BN = 128, TS_BK = 32, TS_STAGES = 4, TS_CK = 4;
+constexpr int TS_LBO = TS_BM * 16 + 16;     // bytes between 8-deep groups of a plane
+constexpr int TS_PLANE = 4 * TS_LBO;        // 128 rows x 32 k
+constexpr int TS_STAGE = 6 * TS_PLANE;      // three planes of A', three of B'
+constexpr int TS_THREADS = 896;
+constexpr int TS_CPT = TS_BN / 2;           // columns of an epilogue warp
+constexpr int TS_STATS = 4;                 // tiles whose value ranges are kept
+
+struct TsSmem {
+  static constexpr int RING = TS_STAGES * TS_STAGE;
+  static constexpr int COLS = 8 * 4 * TS_CPT * 8;  // per epilogue warp: d_n, c_n of two tiles
+  static constexpr int STAT = TS_STATS * 16 * 8;
+  static constexpr int BARS = (2 * TS_STAGES + 2 * 2 + 2 + 2 * TS_STATS + 1) * 8 + 16;
+  static constexpr int BYTES = 128 + RING + COLS + STAT + BARS;
+};
+
+// K-major operand without swizzle: 8-row x 16-byte core matrices, the ones along
+// the rows 128 bytes apart, the ones along K TS_LBO.
+__device__ __forceinline__ uint64_t ts_desc(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(TS_LBO >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+// kind::f16, BF16 K-major operands, FP32 accumulate, 128 x n.
+__device__ __forceinline__ uint32_t ts_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TS_BM >> 4) << 24);
+}
+
+// The next 8 significant bits of two values (lo half: x), and what is left of them.
+__device__ __forceinline__ uint32_t ts_split(float& x, float& y) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(y), "f"(x));
+  x -= __uint_as_float(w << 16);
+  y -= __uint_as_float(w & 0xffff0000u);
+  return w;
+}
+
+// mbar_wait with the clock read only every 64 polls.
+__device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
+  }
+}
+__device__ __forceinline__ void ts_tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void ts_tmem_st(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
+struct TsTile {
+  int h, m0, n0;  // m0 in rows of A'
+};
+template <bool CPLX>
+__device__ __forceinline__ TsTile ts_tile(const GemmArgs& g, int t, int tm, int tn) {
+  constexpr int EM = CPLX ? TS_BM / 2 : TS_BM;
+  const uint32_t r = (uint32_t)t / (uint32_t)tn, nt = (uint32_t)t - r * (uint32_t)tn;
+  const uint32_t h = r / (uint32_t)tm, mt = r - h * (uint32_t)tm;
+  return {(int)h, (int)mt * EM, (int)nt * TS_BN};
+}
+
+template <int BYTES>
+__device__ __forceinline__ void ts_copy(uint32_t dst, const char* src, bool ok) {
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(ok ? BYTES : 0)
+                 : "memory");
+}
+// Producer of 32 plane rows of one operand: R operand rows x KQ depths per lane
+// (lane / 4 along the rows, lane % 4 along the depth), so a lane's 8 plane depths
+// of a row are one 16-byte store per plane.
+template <bool CPLX, bool IS_A>
+struct TsProducer {
+  static constexpr int E = CPLX ? 2 : 1, ES = 4 * E, KQ = 8 / E, EK = TS_BK / E;
+  static constexpr int R = CPLX && IS_A ? 2 : 4;
+  static constexpr int V = 16 / ES;  // elements of a 16-byte load
+  const GemmArgs& g;
+  const int lane, c, row0;
+  const bool by_rows;
+  int ro[R];  // element offsets of the lane's rows (offsets fit 32 bits, launch_tc_stream)
+  const char* base;
+  bool rows_full;
+  int koff;  // lane's: offset of depth k0 + lane of the next block to load
+
+  __device__ __forceinline__ int64_t ld() const { return IS_A ? g.a_ld : g.b_ld; }
+  __device__ __forceinline__ TsProducer(const GemmArgs& g_, int warp, int lane_)
+      : g(g_), lane(lane_), c(lane_ & 3), row0((warp & 3) * 8 * R + (lane_ >> 2) * R),
+        by_rows(IS_A ? g_.a_vec && !g_.a_kfast : g_.b_vec && !g_.b_kfast) {}
+
+  __device__ __forceinline__ void tile(const TsTile& t) {
+    const int nrows = (int)(IS_A ? g.M : g.N);
+    const int64_t* rows = IS_A ? g.s.a_m : g.s.b_n;
+    const int r0 = (IS_A ? t.m0 : t.n0) + row0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = min(r0 + i, nrows - 1);
+      ro[i] = ld() ? r : __ldg(reinterpret_cast<const int*>(rows + r));
+    }
+    rows_full = __all_sync(0xffffffffu, r0 + R <= nrows);
+    base = static_cast<const char*>(IS_A ? g.A : g.B) +
+           (ld() ? (int64_t)t.h * g.K * ld() : __ldg((IS_A ? g.s.h_a : g.s.h_b) + t.h)) * ES;
+  }
+  __device__ __forceinline__ void fetch_k(int k0) {
+    const int k = min(k0 + (lane < EK ? lane : 0), (int)g.K - 1);
+    koff = ld() ? k * (int)ld() : __ldg(reinterpret_cast<const int*>((IS_A ? g.s.a_k : g.s.b_k) + k));
+  }
+  // The lane's elements of the block at k0 (koff fetched, the last depth's past K),
+  // zero past K.
+  __device__ __forceinline__ void load(float (&v)[R][8], int k0) const {
+    const int kv = min(EK, (int)g.K - k0);
+    const int kq = c * KQ;
+    if (by_rows && rows_full) {
+#pragma unroll
+      for (int q = 0; q < KQ; ++q) {
+        const int o = __shfl_sync(0xffffffffu, koff, kq + q);
+#pragma unroll
+        for (int i = 0; i < R; i += V) {
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (kq + q < kv) x = __ldg(reinterpret_cast<const float4*>(base + (int64_t)(o + ro[i]) * ES));
+          if constexpr (CPLX) {
+            v[i][2 * q] = x.x;
+            v[i][2 * q + 1] = x.y;
+            v[i + 1][2 * q] = x.z;
+            v[i + 1][2 * q + 1] = x.w;
+          } else {
+            v[i][q] = x.x;
+            v[i + 1][q] = x.y;
+            v[i + 2][q] = x.z;
+            v[i + 3][q] = x.w;
+          }
+        }
+      }
+    } else if (!by_rows && (IS_A ? g.a_vec : g.b_vec) && kv == EK) {
+      // by_rows is off, so the 16-byte groups run along the depth.
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int o = __shfl_sync(0xffffffffu, koff, kq + j * V);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(base + (int64_t)(o + ro[i]) * ES));
+          v[i][4 * j] = x.x;
+          v[i][4 * j + 1] = x.y;
+          v[i][4 * j + 2] = x.z;
+          v[i][4 * j + 3] = x.w;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < KQ; ++q) {
+        const int o = __shfl_sync(0xffffffffu, koff, kq + q);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const char* p = base + (int64_t)(o + ro[i]) * ES;
+          if constexpr (CPLX) {
+            float2 x = make_float2(0.f, 0.f);
+            if (kq + q < kv) x = __ldg(reinterpret_cast<const float2*>(p));
+            v[i][2 * q] = x.x;
+            v[i][2 * q + 1] = x.y;
+          } else {
+            v[i][q] = kq + q < kv ? __ldg(reinterpret_cast<const float*>(p)) : 0.f;
+          }
+        }
+      }
+    }
+  }
+
+  // Splits one row's eight values into the planes; mx, mn: the largest and smallest
+  // non-zero leading halves (mn less one, zero as 0x7fff).
+  __device__ __forceinline__ void row(const float (&v)[8], char* d, uint32_t flip, uint32_t& mx, uint32_t& mn) const {
+    uint32_t w[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float x = v[2 * j], y = v[2 * j + 1];
+      w[0][j] = ts_split(x, y);
+      w[1][j] = ts_split(x, y);
+      w[2][j] = ts_split(x, y);
+      const uint32_t a = w[0][j] & 0x7fff7fffu;
+      asm("max.u16x2 %0, %0, %1;" : "+r"(mx) : "r"(a));
+      asm("min.s16x2 %0, %0, %1;" : "+r"(mn) : "r"(a + 0x7fff7fffu));
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      if constexpr (CPLX && IS_A) {
+        // Rows 2r: (re, -im); 2r + 1: (im, re).
+        uint32_t e[4], o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t x = w[p][j] ^ flip;
+          e[j] = x ^ 0x80000000u;
+          o[j] = __byte_perm(x, x, 0x1032);
+        }
+        *reinterpret_cast<uint4*>(d + p * TS_PLANE) = make_uint4(e[0], e[1], e[2], e[3]);
+        *reinterpret_cast<uint4*>(d + p * TS_PLANE + 16) = make_uint4(o[0], o[1], o[2], o[3]);
+      } else {
+        *reinterpret_cast<uint4*>(d + p * TS_PLANE) = make_uint4(w[p][0] ^ flip, w[p][1] ^ flip, w[p][2] ^ flip, w[p][3] ^ flip);
+      }
+    }
+  }
+  // Splits the lane's values into the operand's planes of a stage.
+  __device__ __forceinline__ void split(const float (&v)[R][8], char* planes, uint32_t& mx, uint32_t& mn) const {
+    constexpr int PR = CPLX && IS_A ? 2 : 1;  // plane rows per operand row
+    // Core matrices of consecutive rows follow one another.
+    char* d = planes + c * TS_LBO + PR * row0 * 16;
+    const uint32_t flip = CPLX && (IS_A ? g.conj_a : g.conj_b) ? 0x80000000u : 0u;
+#pragma unroll
+    for (int i = 0; i < R; ++i) row(v[i], d + PR * i * 16, flip, mx, mn);
+  }
+};
+
+template <bool CPLX, bool IS_A>
+__device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64_t* full, uint64_t* empty, int2* stats,
+                                           uint64_t* stat_full, uint64_t* stat_empty, int tiles, int tm, int tn,
+                                           int warp, int lane) {
+  using P = TsProducer<CPLX, IS_A>;
+  P p(g, warp, lane);
+  const int nk = (int)((g.K + P::EK - 1) / P::EK);
+  // Whether this warp's rows of the tile exist (columns of B' past the product's width are not multiplied).
+  const int first = (warp & 3) * 8 * P::R;
+  uint32_t block = (uint32_t)warp >> 3;  // the set's blocks: every other one of the CTA's sequence
+  int t = blockIdx.x, reported = t;  // the block's tile; the first tile whose range is not reported
+  int kb = 0, it = 0;
+  uint32_t mx = 0, mn = 0x7fff7fffu;
+  bool act = false, ok = true;
+  const auto advance = [&](int n) {
+    kb += n;
+    while (kb >= nk) {
+      kb -= nk;
+      t += gridDim.x;
+    }
+  };
+  float v[P::R][8];
+  const auto load = [&](bool new_tile) {
+    if (t >= tiles) return;
+    if (new_tile) {
+      const TsTile x = ts_tile<CPLX>(g, t, tm, tn);
+      p.tile(x);
+      act = IS_A || x.n0 + first < g.N;
+    }
+    if (act) p.load(v, kb * P::EK);
+    // The depth offsets of the set's block after this one.
+    int k = kb + 2;
+    while (k >= nk) k -= nk;
+    p.fetch_k(k * P::EK);
+  };
+  // The value ranges of the tiles before `end`.
+  const auto report = [&](int end) {
+    for (; ok && reported < end; reported += gridDim.x, ++it) {
+      const int s = it % TS_STATS;
+      ok = __all_sync(0xffffffffu, ts_wait(&stat_empty[s], ((uint32_t)(it / TS_STATS) & 1u) ^ 1u));
+      const int hi = (int)__reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
+      const int lo = __reduce_min_sync(0xffffffffu, min((int)(int16_t)(mn & 0xffffu), (int)(int16_t)(mn >> 16)));
+      if (lane == 0 && ok) {
+        stats[s * 16 + warp] = make_int2(hi, lo == 0x7fff ? 0x7fff : (lo - 0x7fff) & 0xffff);
+        mbar_arrive(&stat_full[s]);
+      }
+      __syncwarp();
+      mx = 0;
+      mn = 0x7fff7fffu;
+    }
+  };
+  advance((int)block);
+  p.fetch_k(kb * P::EK);
+  load(true);
+  while (t < tiles) {
+    report(t);
+    const uint32_t stage = block % TS_STAGES, round = block / TS_STAGES;
+    ok = ok && ts_wait(&empty[stage], (round & 1u) ^ 1u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    if (act) p.split(v, ring + stage * TS_STAGE + (IS_A ? 0 : 3 * TS_PLANE), mx, mn);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&full[stage]);
+    // The next block's elements are on their way while the other set splits.
+    const int told = t;
+    advance(2);
+    load(t != told);
+    block += 2;
+  }
+  report(tiles);
+  if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_constant__ GemmArgs g, int tiles, int tm,
+                                                                  int tn) {
+  using T = typename Elem<float, CPLX>::type;
+  constexpr int EK = CPLX ? TS_BK / 2 : TS_BK;
+  extern __shared__ unsigned char ts_smem[];
+  char* ring = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ts_smem) + 127) & ~uintptr_t(127));
+  int64_t* cols = reinterpret_cast<int64_t*>(ring + TsSmem::RING);
+  int2* stats = reinterpret_cast<int2*>(ring + TsSmem::RING + TsSmem::COLS);
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + TsSmem::RING + TsSmem::COLS + TsSmem::STAT);
+  uint64_t* empty = full + TS_STAGES;
+  uint64_t* main_full = empty + TS_STAGES;
+  uint64_t* main_empty = main_full + 2;
+  uint64_t* corr_empty = main_empty + 2;
+  uint64_t* stat_full = corr_empty + 2;
+  uint64_t* stat_empty = stat_full + TS_STATS;
+  uint64_t* done = stat_empty + TS_STATS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nk = (int)((g.K + EK - 1) / EK);
+  if (tid == 0) {
+    for (int s = 0; s < TS_STAGES; ++s) {
+      mbar_init(&full[s], 8);
+      mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&main_full[s], 1);
+      mbar_init(&main_empty[s], 8);
+      mbar_init(&corr_empty[s], 8);
+    }
+    for (int s = 0; s < TS_STATS; ++s) {
+      mbar_init(&stat_full[s], 16);
+      mbar_init(&stat_empty[s], 8);
+    }
+    mbar_init(done, 1);
+    fence_barrier_init();
+  }
+  if (warp == 24) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // Tensor memory, 128 columns each: main 0, main 1, then the corrections of two
+  // tiles, or (K of several chunks) one and the running sums.
+  const uint32_t tmem = *tmem_slot;
+  const bool multi = nk > TS_CK;
+
+  // Registers a thread: 56 x 256 + 88 x 512 + 40 x 128 = the 72 x 896 of the launch.
+  if (warp >= 8 && warp < 24) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    if ((warp & 7) < 4)
+      ts_produce<CPLX, true>(g, ring, full, empty, stats, stat_full, stat_empty, tiles, tm, tn, warp - 8, lane);
+    else
+      ts_produce<CPLX, false>(g, ring, full, empty, stats, stat_full, stat_empty, tiles, tm, tn, warp - 8, lane);
+  } else if (warp >= 24) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 24 && lane == 0) {
+      int stage = 0;
+      uint32_t round = 0, chunk = 0;
+      bool ok = true;
+      int it = 0;
+      for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++it) {
+        const TsTile x = ts_tile<CPLX>(g, t, tm, tn);
+        const int n = min(TS_BN, ((int)g.N - x.n0 + 15) / 16 * 16);
+        const uint32_t idesc = ts_idesc(n);
+        const int cb = multi ? 0 : it & 1;
+        const uint32_t corr = tmem + 256 + 128 * cb;
+        if (!ts_wait(&corr_empty[cb], ((uint32_t)(multi ? it : it >> 1) & 1u) ^ 1u)) ok = false;
+        for (int kb = 0; ok && kb < nk; ++kb) {
+          const int in_chunk = kb % TS_CK;
+          if (!ts_wait(&full[stage], round & 1u) ||
+              (in_chunk == 0 && !ts_wait(&main_empty[chunk & 1], ((chunk >> 1) & 1u) ^ 1u))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(ring + stage * TS_STAGE), sb = sa + 3 * TS_PLANE;
+          const int left = ((int)g.K - kb * EK) * (CPLX ? 2 : 1);
+          const int steps = left > 16 ? 2 : 1;
+          const uint32_t mainacc = tmem + 128 * (chunk & 1);
+          for (int kk = 0; kk < steps; ++kk) {
+            uint64_t a[3], b[3];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+              a[p] = ts_desc(sa + p * TS_PLANE + 2 * kk * TS_LBO);
+              b[p] = ts_desc(sb + p * TS_PLANE + 2 * kk * TS_LBO);
+            }
+            umma_bf16(corr, a[0], b[2], idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_bf16(corr, a[1], b[1], idesc, 1u);
+            umma_bf16(corr, a[2], b[0], idesc, 1u);
+            umma_bf16(corr, a[0], b[1], idesc, 1u);
+            umma_bf16(corr, a[1], b[0], idesc, 1u);
+            umma_bf16(mainacc, a[0], b[0], idesc, (in_chunk | kk) != 0 ? 1u : 0u);
+          }
+          umma_commit(&empty[stage]);
+          if (in_chunk == TS_CK - 1 || kb == nk - 1) {
+            umma_commit(&main_full[chunk & 1]);
+            ++chunk;
+          }
+          if (++stage == TS_STAGES) {
+            stage = 0;
+            ++round;
+          }
+        }
+      }
+      if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+      // Nothing of this CTA's tensor work is in flight when it ends.
+      umma_commit(done);
+      if (!ts_wait(done, 0)) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+    }
+    __syncwarp();
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const int col0 = (warp >> 2) * TS_CPT;
+    int64_t* cols_w = cols + warp * 4 * TS_CPT;
+    const uint32_t lane_addr = ((uint32_t)(32 * (warp & 3)) << 16) + col0;
+    const int prow = 32 * (warp & 3) + lane, comp = CPLX ? prow & 1 : 0;
+    const Epilogue e = g.e;
+    uint32_t chunk = 0;
+    int it = 0;
+    bool ok = true;
+    // Output offsets of a tile, fetched while the one before it is written back.
+    int64_t nd = 0, nc = 0;
+    const auto fetch = [&](const TsTile& x, int buf) {
+      const int m = min(x.m0 + (CPLX ? prow >> 1 : prow), (int)g.M - 1);
+      nd = __ldg(g.s.d_m + m) + __ldg(g.s.h_d + x.h);
+      if (!e.beta_zero) nc = __ldg(g.s.c_m + m) + __ldg(g.s.h_c + x.h);
+#pragma unroll
+      for (int j = 0; j < TS_CPT / 32; ++j) {
+        const int n = min(x.n0 + col0 + lane + 32 * j, (int)g.N - 1);
+        const uint32_t d = smem_u32(cols_w + buf * 2 * TS_CPT + lane + 32 * j);
+        ts_copy<8>(d, reinterpret_cast<const char*>(g.s.d_n + n), true);
+        if (!e.beta_zero) ts_copy<8>(d + TS_CPT * 8, reinterpret_cast<const char*>(g.s.c_n + n), true);
+      }
+    };
+    fetch(ts_tile<CPLX>(g, blockIdx.x, tm, tn), 0);
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++it) {
+      const TsTile x = ts_tile<CPLX>(g, t, tm, tn);
+      const int m = x.m0 + (CPLX ? prow >> 1 : prow), n0 = x.n0 + col0;
+      const bool mok = m < (int)g.M;
+      const int nrem = max(0, min(TS_CPT, (int)g.N - n0));
+      T* Db = static_cast<T*>(g.D) + nd;
+      const T* Cb = static_cast<const T*>(g.C) + nc;
+      const int64_t *dn_s = cols_w + (it & 1) * 2 * TS_CPT, *cn_s = dn_s + TS_CPT;
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      if (t + (int)gridDim.x < tiles) fetch(ts_tile<CPLX>(g, t + gridDim.x, tm, tn), (it + 1) & 1);
+      const int cb = multi ? 0 : it & 1;
+      const uint32_t corr = tmem + 256 + 128 * cb + lane_addr, total = tmem + 384 + lane_addr;
+      for (int kb = 0; kb + TS_CK < nk; kb += TS_CK, ++chunk) {
+        if (!ts_wait(&main_full[chunk & 1], (chunk >> 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t acc = tmem + 128 * (chunk & 1) + lane_addr;
+#pragma unroll 1
+        for (int q = 0; 8 * q < nrem; ++q) {
+          uint32_t r[8];
+          ts_tmem_ld(acc + 8 * q, r);
+          if (kb) {
+            uint32_t u[8];
+            ts_tmem_ld(total + 8 * q, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(r[j]));
+          } else {
+            tmem_ld_wait();
+          }
+          ts_tmem_st(total + 8 * q, r);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&main_empty[chunk & 1]);
+      }
+      // The last chunk's commit covers the cross products; then the value ranges
+      // of the tile's operands.
+      const int s = it % TS_STATS;
+      if (ok) ok = ts_wait(&main_full[chunk & 1], (chunk >> 1) & 1u);
+      if (ok) ok = ts_wait(&stat_full[s], (uint32_t)(it / TS_STATS) & 1u);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      int amax = 0, bmax = 0, amin = 0x7fff, bmin = 0x7fff;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const int2 a = stats[s * 16 + w / 4 * 8 + w % 4], b = stats[s * 16 + w / 4 * 8 + 4 + w % 4];
+        amax = max(amax, a.x);
+        amin = min(amin, a.y);
+        bmax = max(bmax, b.x);
+        bmin = min(bmin, b.y);
+      }
+      const float thr = split_guard((amax >> 7) - 127, amin == 0x7fff ? 999 : (amin >> 7) - 127, (bmax >> 7) - 127,
+                                    bmin == 0x7fff ? 999 : (bmin >> 7) - 127);
+      const bool guard = thr != 0.f;
+      uint64_t again = 0;
+      const uint32_t acc = tmem + 128 * (chunk & 1) + lane_addr;
+#pragma unroll 1
+      for (int q = 0; 8 * q < nrem; ++q) {
+        {
+          uint32_t r[8], c[8];
+          ts_tmem_ld(acc + 8 * q, r);
+          ts_tmem_ld(corr + 8 * q, c);
+          tmem_ld_wait();
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+          if (multi) {
+            ts_tmem_ld(total + 8 * q, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]) + v[j];
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(c[j]);
+          if (!guard && e.plain && 8 * q + 8 <= nrem) {
+            float* Df = reinterpret_cast<float*>(Db) + comp;
+            if (mok) {
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) {
+                const longlong2 o = *reinterpret_cast<const longlong2*>(dn_s + 8 * q + j);
+                Df[o.x * (CPLX ? 2 : 1)] = v[j];
+                Df[o.y * (CPLX ? 2 : 1)] = v[j + 1];
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+              // v[j] without a dynamic register index.
+              float y = v[0];
+#pragma unroll
+              for (int i = 1; i < 8; ++i) y = j == i ? v[i] : y;
+              const int jj = 8 * q + j;
+              const float o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
+              bool low = split_lost(thr, y);
+              if (CPLX) low = low || split_lost(thr, o);
+              if (jj >= nrem || !mok || comp) continue;
+              if (low)
+                again |= (uint64_t)1 << jj;
+              else
+                epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
+            }
+          }
+          __syncwarp();
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&main_empty[chunk & 1]);
+        mbar_arrive(&corr_empty[cb]);
+        mbar_arrive(&stat_empty[s]);
+      }
+      ++chunk;
+      for (; again; again &= again - 1) {
+        const int j = __ffsll((long long)again) - 1;
+        const float2 r = ffma_dot<CPLX>(g, x.h, m, n0 + j);
+        epilogue_store<float, CPLX>(e, r.x, r.y, Cb + (e.beta_zero ? 0 : cn_s[j]), Db + dn_s[j]);
+      }
+      __syncwarp();
+    }
+    if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 24) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// Copy of an operand into a dense panel [H][K][ld], rows fastest: 32 rows by 32 of
+// the index that is fastest in memory (depth or batch; FAST 0: rows, with 32
+// depths) per CTA, through shared memory.
+template <class T, int FAST>
+__global__ void __launch_bounds__(256) stream_pack_kernel(const T* __restrict__ X, const int64_t* __restrict__ rows,
+                                                          const int64_t* __restrict__ ks, const int64_t* __restrict__ hs,
+                                                          int64_t nrows, int64_t K, int64_t H, int64_t ld,
+                                                          T* __restrict__ out) {
+  __shared__ T tile[32][33];
+  // The second index of a tile: the batch (FAST 2) or the depth; `o` the other.
+  const int64_t n2 = FAST == 2 ? H : K, no = FAST == 2 ? K : H;
+  const int64_t* s2 = FAST == 2 ? hs : ks;
+  const int64_t* so = FAST == 2 ? ks : hs;
+  const int64_t tr = (nrows + 31) / 32, t2 = (n2 + 31) / 32;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int64_t t = blockIdx.x; t < tr * t2 * no; t += gridDim.x) {
+    const int64_t r0 = t % tr * 32, q0 = t / tr % t2 * 32, o = t / tr / t2;
+    const T* base = X + so[o];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int rr = FAST ? y + 8 * j : x, q = FAST ? x : y + 8 * j;
+      if (r0 + rr < nrows && q0 + q < n2) tile[q][rr] = base[rows[r0 + rr] + s2[q0 + q]];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int q = y + 8 * j;
+      if (r0 + x < nrows && q0 + q < n2)
+        out[(FAST == 2 ? (q0 + q) * K + o : o * K + q0 + q) * ld + r0 + x] = tile[q][x];
+    }
+    __syncthreads();
+  }
+}
+int64_t panel_ld(int64_t rows) { return (rows + 15) / 16 * 16; }
+
+template <class T>
+void run_stream_pack(const GemmArgs& g, int which, int fast, int64_t ld, void* panel, cudaStream_t st) {
+  const bool a = which == 0;
+  const int64_t rows = a ? g.M : g.N;
+  const int64_t tiles = ((rows + 31) / 32) * (fast == 2 ? (g.H + 31) / 32 * g.K : (g.K + 31) / 32 * g.H);
+  const unsigned grid = (unsigned)(tiles < 8192 ? tiles : 8192);
+  auto kern = fast == 2 ? stream_pack_kernel<T, 2> : fast == 1 ? stream_pack_kernel<T, 1> : stream_pack_kernel<T, 0>;
+  kern<<<grid, 256, 0, st>>>(static_cast<const T*>(a ? g.A : g.B), a ? g.s.a_m : g.s.b_n, a ? g.s.a_k : g.s.b_k,
+                             a ? g.s.h_a : g.s.h_b, rows, g.K, g.H, ld, static_cast<T*>(panel));
+}
+
+}  // namespace
+
+bool is_tc_stream(int kernel) { return kernel == PLAIN_F32_TC_STREAM || kernel == PLAIN_C32_TC_STREAM; }
+
+size_t stream_panel_bytes(int dtype, int64_t rows, int64_t K, int64_t H) {
+  return (size_t)H * K * panel_ld(rows) * (dtype == 0 ? 4 : 8) + 256;
+}
+
+cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, int fast, void* panel, cudaStream_t st) {
+  const bool a = which == 0;
+  const int64_t ld = panel_ld(a ? g.M : g.N);
+  if (dtype == 0)
+    run_stream_pack<float>(g, which, fast, ld, panel, st);
+  else if (dtype == 2)
+    run_stream_pack<float2>(g, which, fast, ld, panel, st);
+  else
+    return cudaErrorInvalidValue;
+  if (a) {
+    g.A = panel;
+    g.a_ld = ld;
+    g.a_kfast = 0;
+    g.a_vec = 1;
+  } else {
+    g.B = panel;
+    g.b_ld = ld;
+    g.b_kfast = 0;
+    g.b_vec = 1;
+  }
+  return cudaGetLastError();
+}
+
+// Index arithmetic of the kernel: rows, depths and tiles in 32 bits, and an
+// operand's row plus depth offset (in its panel, where it is packed) as well.
+bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints) {
+  constexpr int64_t most = (int64_t)1 << 30;
+  if (dtype != 0 && dtype != 2) return false;
+  if (!hints.known || !hints.off32 || K <= 0 || K >= most || M >= most || N >= most || H >= most) return false;
+  if ((!hints.a_gather && (double)panel_ld(M) * (double)K >= 2.0 * most - (double)M) ||
+      (!hints.b_gather && (double)panel_ld(N) * (double)K >= 2.0 * most - (double)N))
+    return false;
+  const int64_t em = dtype == 2 ? TS_BM / 2 : TS_BM;
+  return ((double)(M / em) + 1) * ((double)(N / TS_BN) + 1) * (double)H < (double)most &&
+         ((double)(N / em) + 1) * ((double)(M / TS_BN) + 1) * (double)H < (double)most;
+}
+
+// Against the FFMA families by estimated microseconds, fitted on B200. Here: 8, per
+// wave of tiles 4 (1.5 for outputs of at most 64 columns) and 1.1 (c32 1.25) per 32-deep
+// stage, 4 per panel; there: 12 (26 from K = 64 on, with packs) + 2 M N K / 50e6 (c32 /
+// 40e6) over whole tiles + 1 per MB of D. Measured here against there: f32 6144^2 x 24
+// in six indexes 89 against 235, 2048^2 x 64 17 against 32, x 1024 87 against 217,
+// 120000 x 31 x 33 37 against 90, 16 x 100^3 batch innermost 26 against 17, 300 x 260 x
+// 2000 (63 stages on nine SMs) 76 against 40 with split-K; c32 2048^2 x 512 178 against
+// 402, 700^2 x 2500 226 against 373. Below 2^23 products the launches decide; beyond K = 1024 the
+// packed panels' single pass over the operands is kept.
+bool use_tc_stream(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
+  if (!tc_stream_fits(dtype, M, N, K, H, hints)) return false;
+  const bool cplx = dtype == 2;
+  const int64_t m = hints.d_mfast ? M : N, n = hints.d_mfast ? N : M;  // the launch's roles
+  const int64_t em = cplx ? TS_BM / 2 : TS_BM, ek = cplx ? TS_BK / 2 : TS_BK, pad = cplx ? 64 : 128;
+  const int64_t tiles = ((m + em - 1) / em) * ((n + TS_BN - 1) / TS_BN) * H;
+  const double outs = (double)M * (double)N * (double)H, per = cplx ? 4 : 1;
+  if (K > 1024 || tiles < 16 || outs * (double)K * per < (double)(1 << 23)) return false;
+  const double waves = (double)((tiles + num_sms - 1) / num_sms), stages = (double)((K + ek - 1) / ek);
+  const double here = 8 + waves * ((n <= 64 ? 1.5 : 4) + (cplx ? 1.25 : 1.1) * stages) +
+                      4 * ((hints.a_gather ? 0 : 1) + (hints.b_gather ? 0 : 1));
+  const double whole = (double)((M + pad - 1) / pad * pad) * (double)((N + pad - 1) / pad * pad) * (double)H;
+  const double there = (K >= 64 ? 26 : 12) + 2 * per * whole * (double)K / (cplx ? 40e6 : 50e6) +
+                       outs * (cplx ? 8e-6 : 4e-6);
+  return here < there;
+}
+
+// The caller has checked tc_stream_fits.
+cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st) {
+  if (dtype != 0 && dtype != 2) return cudaErrorInvalidValue;
+  const int64_t em = dtype == 2 ? TS_BM / 2 : TS_BM;
+  const int64_t tm = (g.M + em - 1) / em, tn = (g.N + TS_BN - 1) / TS_BN, tiles = tm * tn * g.H;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
+  auto kern = dtype == 2 ? tc_stream_kernel<true> : tc_stream_kernel<false>;
+  const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TsSmem::BYTES);
+  if (r != cudaSuccess) return r;
+  kern<<<grid, TS_THREADS, TsSmem::BYTES, st>>>(g, (int)tiles, (int)tm, (int)tn);
+  return cudaGetLastError();
+}
+
+}  // namespace dev
+}  // namespace tprims

@@ -62,7 +62,7 @@ struct __align__(16) GemmArgs {
   // (16-byte gathers).
   int a_vec, b_vec;
   // Non-zero: the operand is a dense panel [H][K][ld], rows fastest, and its
-  // scatter vectors are not read (stream tiles after a pack pass).
+  // scatter vectors are not read (tensor-core stream tiles after a pack pass).
   int64_t a_ld, b_ld;
   Epilogue e;
   unsigned* status;
@@ -108,13 +108,10 @@ enum PlainKernel : int {
   PLAIN_F64_STREAM_128x32 = 22,
   PLAIN_F64_STREAM_64x48 = 23,
   PLAIN_F64_STREAM_32x128 = 24,
-  PLAIN_F32_STREAM_128x64 = 25,
-  PLAIN_F32_STREAM_128x48 = 26,
-  PLAIN_F32_STREAM_128x32 = 27,
-  PLAIN_C32_STREAM_64x64 = 28,
-  PLAIN_C32_STREAM_64x32 = 29,
-  PLAIN_C32_STREAM_64x24 = 30,
-  PLAIN_STREAM_LAST = 30,
+  // Tensor cores, f32 split on the way into shared memory (k_tcstream.cu).
+  PLAIN_F32_TC_STREAM = 25,
+  PLAIN_C32_TC_STREAM = 26,
+  PLAIN_STREAM_LAST = 26,
   // Batches of small products (k_small.cu): chosen by the model, never pinned.
   PLAIN_SMALL_BATCHED = 40,
 };
@@ -123,19 +120,25 @@ enum PlainKernel : int {
 cudaError_t launch_output_pass(int dtype, const GemmArgs& g, cudaStream_t st);
 cudaError_t launch_plain_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
 // Gather-fed stream tiles (k_stream.cu): persistent, one producer warp per CTA.
+struct LaunchHints;
 bool is_stream_kernel(int kernel);
 int stream_dtype(int kernel);
 void stream_tile_shape(int kernel, int* bm, int* bn);
 const char* stream_kernel_name(int kernel);
 // The stream family of least padded work for a shape (0: none of the dtype),
 // and its padded outputs per output.
-struct LaunchHints;
 int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste);
 cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
-// Dense panel of one operand (0 = A', 1 = B') for the stream tiles: its bytes, and
-// the pass that writes it and points `g` at it.
+// f32 and c32 on the tensor cores without a pack pass (k_tcstream.cu).
+bool is_tc_stream(int kernel);
+cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st);
+bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints);
+bool use_tc_stream(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
+// Dense panel of one operand (0 = A', 1 = B') whose gather is not coalesced: its
+// bytes, and the pass that writes it and points `g` at it. `fast`: the index of
+// the operand's smallest stride (0 rows, 1 depth, 2 batch).
 size_t stream_panel_bytes(int dtype, int64_t rows, int64_t K, int64_t H);
-cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, void* panel, cudaStream_t st);
+cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, int fast, void* panel, cudaStream_t st);
 static_assert(sizeof(GemmArgs) % 16 == 0, "grouped kernels copy GemmArgs in 16-byte words");
 
 // One item of a grouped launch: its arguments and its tile grid.
@@ -170,6 +173,7 @@ struct LaunchHints {
   bool known = false;
   bool a_gather = false, b_gather = false, a_vec = false, b_vec = false, d_mfast = true;
   bool h_inner = false;  // the batch index has the smallest stride of A', B' and D
+  bool off32 = false;    // row plus depth offsets of A' and of B' fit 32 bits
 };
 // The family the autotuner would pick for a shape (no launch).
 int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);

@@ -160,12 +160,14 @@ bool mostly_unit(const std::vector<int64_t>& fast) {
 // multiple of `v`, and every other offset is a multiple of `v`.
 bool vector_groups(const std::vector<int64_t>& fast, const std::vector<int64_t>& slow, const std::vector<int64_t>& h,
                    int64_t v) {
+  if (v == 1) return true;
+  const int64_t mask = v - 1;  // v is a power of two
+  int64_t low = 0;
+  for (int64_t x : slow) low |= x & mask;
+  for (int64_t x : h) low |= x & mask;
+  if (low) return false;
   for (size_t i = 0; i < fast.size(); ++i)
-    if (i % v == 0 ? fast[i] % v != 0 : fast[i] != fast[i - 1] + 1) return false;
-  for (int64_t x : slow)
-    if (x % v != 0) return false;
-  for (int64_t x : h)
-    if (x % v != 0) return false;
+    if ((i & mask) == 0 ? (fast[i] & mask) != 0 : fast[i] != fast[i - 1] + 1) return false;
   return true;
 }
 }  // namespace
@@ -214,6 +216,19 @@ Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1))
   hints.h_inner = step(view.h_a) < std::min(step(view.a_m), step(view.a_k)) &&
                   step(view.h_b) < std::min(step(view.b_n), step(view.b_k)) &&
                   step(view.h_d) < std::min(step(view.d_m), step(view.d_n));
+  const auto reach = [](const std::vector<int64_t>& x) {
+    uint64_t m = 0;
+    for (int64_t v : x) m = std::max<uint64_t>(m, (uint64_t)std::llabs(v));
+    return m;
+  };
+  const bool single = problem.dtype == DType::F32 || problem.dtype == DType::C32;
+  hints.off32 = single && reach(view.a_m) + reach(view.a_k) < (uint64_t(1) << 31) &&
+                reach(view.b_n) + reach(view.b_k) < (uint64_t(1) << 31);
+  const auto fastest = [&](const std::vector<int64_t>& rows, const std::vector<int64_t>& k, const std::vector<int64_t>& h) {
+    return step(h) < std::min(step(rows), step(k)) ? 2 : step(k) < step(rows) ? 1 : 0;
+  };
+  a_fast = fastest(view.a_m, view.a_k, view.h_a);
+  b_fast = fastest(view.b_n, view.b_k, view.h_b);
   signature = problem_signature(*this);
 }
 
@@ -602,7 +617,7 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const Plai
     }
     return;
   }
-  if (dev::is_stream_kernel(c.kernel)) {
+  if (dev::is_tc_stream(c.kernel)) {
     // Complex elements are gathered whole: operands off their natural alignment
     // take the direct tile.
     if (dt == 2 && ((reinterpret_cast<uintptr_t>(g0.A) | reinterpret_cast<uintptr_t>(g0.B)) & 7) != 0) {
@@ -616,7 +631,7 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const Plai
       char* panel = reinterpret_cast<char*>(align_up((uintptr_t)scratch, 256));
       if (panel + bytes > scratch_end) throw Error(ERR_INTERNAL, "stream panel workspace too small");
       Timed t(ex, "stream_pack");
-      check_cuda(dev::launch_stream_pack(dt, g, which, panel, ex.stream), "stream pack launch");
+      check_cuda(dev::launch_stream_pack(dt, g, which, which == 0 ? pr.a_fast : pr.b_fast, panel, ex.stream), "stream pack launch");
       scratch = panel + bytes;
     }
     scratch_bytes = (size_t)(scratch_end - scratch);
@@ -904,9 +919,10 @@ TuneEntry autotune_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, char
     check_cuda(cudaMemcpyAsync(snapshot, d_span, span_bytes, cudaMemcpyDeviceToDevice, ex.stream),
                "autotune snapshot of D");
   EventPair ev;
-  const std::vector<PlainChoice> cands =
-      plain_candidates((int)pr.problem.dtype, pr.view.M, pr.view.N, pr.view.K, pr.view.H, ex.num_sms,
-                       pr.hints);
+  std::vector<PlainChoice> cands = plain_candidates((int)pr.problem.dtype, pr.view.M, pr.view.N, pr.view.K, pr.view.H,
+                                                    ex.num_sms, pr.hints);
+  const PlainChoice model = model_choice(pr, ex.num_sms);
+  if (!(cands.front() == model)) cands.insert(cands.begin(), model);
   TuneEntry best;
   best.ms = 0;
   for (size_t i = 0; i < cands.size(); ++i) {
@@ -1119,7 +1135,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
       if (dev::is_packed_kernel(pc.kernel))
         scratch = std::max(scratch,
                            dev::packed_workspace_bytes(dev::packed_layout(pc.kernel, mc, ncols, v.K, v.H)) + 512);
-      if (dev::is_stream_kernel(pc.kernel)) scratch = std::max(scratch, stream_scratch(pr, mc, ncols));
+      if (dev::is_tc_stream(pc.kernel)) scratch = std::max(scratch, stream_scratch(pr, mc, ncols));
     }
     return true;
   };

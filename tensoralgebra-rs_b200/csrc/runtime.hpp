@@ -151,6 +151,7 @@ struct Product {
   // Layout facts of the oriented view for the launch choice (a_vec, b_vec: whole
   // aligned 16-byte groups relative to the operand's origin).
   dev::LaunchHints hints;
+  int a_fast = 0, b_fast = 0;  // index of the smallest stride: 0 rows, 1 depth, 2 batch
   // Unique over the process lifetime (never reused, unlike the address), so a
   // cached grouped graph can never be replayed for a newer plan.
   const uint64_t uid;
@@ -253,7 +254,7 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
 // The model's choice (heuristics), honouring the tile and split pins.
 // `general`: without the layout's hints (the families that take any layout).
 PlainChoice model_choice(const Product& p, int num_sms, bool general = false);
-// Dense panels of the operands whose gather is not coalesced (stream tiles).
+// Dense panels of the operands whose gather is not coalesced (tensor-core stream tiles).
 size_t stream_scratch(const Product& p, int64_t M, int64_t N);
 // Scratch bytes a plain choice needs (split-K partials).
 size_t plain_scratch(const PlainChoice& c, const Product& p);

