@@ -214,6 +214,13 @@ int grouped_family(const Product& p, int policy) {
       break;
     default: break;
   }
+  // f64 items with coalesced gathers: the stream tiles (256 environment updates of
+  // uneven bonds 2.07 ms on the direct and skinny tiles, 1.81 with stream tiles in
+  // place of the direct ones, 1.63 in place of both).
+  if (dt == 1 && p.hints.known && p.hints.a_gather && p.hints.b_gather) {
+    double waste = 0;
+    return dev::choose_stream_kernel(dt, p.view.M, p.view.N, p.hints, &waste);
+  }
   return dev::choose_grouped_kernel(dt, p.view.M, p.view.N, p.view.K);
 }
 

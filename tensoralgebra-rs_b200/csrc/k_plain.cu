@@ -1611,6 +1611,7 @@ using GSkinny32s = SkinnyTileOp<32, 32>;
 // Loads the family's grouped kernel (module loading is lazy) and records its
 // occupancy, so that the launch inside a stream capture needs neither.
 cudaError_t prepare_grouped(int kernel) {
+  if (is_stream_kernel(kernel)) return prepare_stream_grouped(kernel);
   switch (kernel) {
     case PLAIN_F32_SIMT_128x128: return grouped_prepare_op<GSimtF32L>(kernel);
     case PLAIN_F32_SIMT_64x64: return grouped_prepare_op<GSimtF32S>(kernel);
@@ -1635,6 +1636,8 @@ cudaError_t launch_grouped(int kernel, const GroupItem* items, const int64_t* ti
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   if (nitems <= 0) return cudaSuccess;
+  if (is_stream_kernel(kernel))
+    return launch_stream_grouped(kernel, items, tile_start, nitems, counter, status, num_sms, st);
   switch (kernel) {
     case PLAIN_F32_SIMT_128x128:
       grouped_launch_op<GSimtF32L>(kernel, items, tile_start, nitems, counter, status, num_sms, st);

@@ -613,6 +613,20 @@ cudaError_t run_stream(const GemmArgs& g, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// The grouped kernel's image is loaded and its attribute set before any capture.
+template <class Op>
+cudaError_t prepare_group() {
+  return cudaFuncSetAttribute(stream_kernel<Op, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              StreamSmem<Op>::BYTES);
+}
+template <class Op>
+cudaError_t run_group(const GroupItem* items, const int64_t* tile_start, int nitems, unsigned long long* counter,
+                      unsigned* status, int num_sms, cudaStream_t st) {
+  stream_kernel<Op, true><<<num_sms * Op::MINB, Op::WARPS * 32 + 32, StreamSmem<Op>::BYTES, st>>>(
+      GemmArgs{}, items, tile_start, nitems, counter, status);
+  return cudaGetLastError();
+}
+
 using SF64_64x64 = StreamF64<2, 2, 2, 4, 4, 3>;
 using SF64_128x32 = StreamF64<4, 1, 2, 4, 3, 3>;
 using SF64_64x48 = StreamF64<4, 1, 1, 6, 4, 3>;
@@ -695,11 +709,34 @@ int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hin
   return best;
 }
 
+// Rows of the tile run along D's unit-stride index (the lanes' stores).
+GemmArgs stream_oriented(const GemmArgs& g) { return !g.d_mfast && !g.partial ? swapped(g) : g; }
+
+cudaError_t prepare_stream_grouped(int kernel) {
+  switch (kernel) {
+    case PLAIN_F64_STREAM_64x64: return prepare_group<SF64_64x64>();
+    case PLAIN_F64_STREAM_128x32: return prepare_group<SF64_128x32>();
+    case PLAIN_F64_STREAM_64x48: return prepare_group<SF64_64x48>();
+    case PLAIN_F64_STREAM_32x128: return prepare_group<SF64_32x128>();
+  }
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_stream_grouped(int kernel, const GroupItem* items, const int64_t* tile_start, int nitems,
+                                  unsigned long long* counter, unsigned* status, int num_sms, cudaStream_t st) {
+  switch (kernel) {
+    case PLAIN_F64_STREAM_64x64: return run_group<SF64_64x64>(items, tile_start, nitems, counter, status, num_sms, st);
+    case PLAIN_F64_STREAM_128x32: return run_group<SF64_128x32>(items, tile_start, nitems, counter, status, num_sms, st);
+    case PLAIN_F64_STREAM_64x48: return run_group<SF64_64x48>(items, tile_start, nitems, counter, status, num_sms, st);
+    case PLAIN_F64_STREAM_32x128: return run_group<SF64_32x128>(items, tile_start, nitems, counter, status, num_sms, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
 cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g0, cudaStream_t st) {
   if (g0.M <= 0 || g0.N <= 0 || g0.H <= 0) return cudaSuccess;
   if (g0.K <= 0 || stream_dtype(kernel) != dtype) return cudaErrorInvalidValue;
-  // Rows of the tile run along D's unit-stride index (the lanes' stores).
-  const GemmArgs g = !g0.d_mfast && !g0.partial ? swapped(g0) : g0;
+  const GemmArgs g = stream_oriented(g0);
   switch (kernel) {
     case PLAIN_F32_TC_STREAM:
     case PLAIN_C32_TC_STREAM: return launch_tc_stream(dtype, g, st);

@@ -121,6 +121,7 @@ cudaError_t launch_output_pass(int dtype, const GemmArgs& g, cudaStream_t st);
 cudaError_t launch_plain_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
 // Gather-fed stream tiles (k_stream.cu): persistent, one producer warp per CTA.
 struct LaunchHints;
+struct GroupItem;
 bool is_stream_kernel(int kernel);
 int stream_dtype(int kernel);
 void stream_tile_shape(int kernel, int* bm, int* bn);
@@ -129,6 +130,11 @@ const char* stream_kernel_name(int kernel);
 // and its padded outputs per output.
 int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste);
 cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g, cudaStream_t st);
+// Grouped lists: items in the kernel's orientation (of A' and B').
+GemmArgs stream_oriented(const GemmArgs& g);
+cudaError_t prepare_stream_grouped(int kernel);
+cudaError_t launch_stream_grouped(int kernel, const GroupItem* items, const int64_t* tile_start, int nitems,
+                                  unsigned long long* counter, unsigned* status, int num_sms, cudaStream_t st);
 // f32 and c32 on the tensor cores without a pack pass (k_tcstream.cu).
 bool is_tc_stream(int kernel);
 cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st);

@@ -1516,8 +1516,9 @@ GroupSet build_group_set(Executor& ex, const std::vector<int>& idx, int policy, 
       gi.g = build_args(pr, ex, alpha[i], beta[i], c_read, static_cast<const char*>(items[i].a),
                         static_cast<const char*>(items[i].b),
                         c_read ? static_cast<const char*>(items[i].c) : nullptr, static_cast<char*>(items[i].d));
-      gi.tiles_m = (pr.view.M + bm - 1) / bm;
-      gi.tiles_n = (pr.view.N + bn - 1) / bn;
+      if (dev::is_stream_kernel(kv.first)) gi.g = dev::stream_oriented(gi.g);
+      gi.tiles_m = (gi.g.M + bm - 1) / bm;
+      gi.tiles_n = (gi.g.N + bn - 1) / bn;
       host_items.push_back(gi);
       host_starts.push_back(acc);
       acc += gi.tiles_m * gi.tiles_n * pr.view.H;

@@ -118,3 +118,47 @@ def test_uncoalesced_operands_keep_the_other_families(tp, ex, torch_cuda, orc):
     D = Op(d0, [h, m, n], [1, h, h * m], [9, 0, 1])
     p = make_product(tp, "float64", A, B, None, D)
     assert ".stream." not in p.report()["family"]
+
+
+def test_grouped_list_of_stream_tiles(tp, torch_cuda):
+    """A list of f64 contractions over either fast index, either output
+    orientation, 16-byte groups or not, extents around a tile's edges, K from 1 to
+    past a stage, with C in place: grouped (captured and replayed) against the same
+    plans one by one on the direct tile and against float64 einsum."""
+    torch = torch_cuda
+    ex = tp.Executor()
+    rng = np.random.default_rng(12)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda n: torch.randn(n, dtype=torch.float64, device="cuda", generator=gen)
+    cases = [(m, n, k) for m in (1, 17, 64, 65, 200) for n in (3, 48, 64, 130) for k in (1, 4, 13, 16, 50)]
+    items, singles, outs = [], [], []
+    for i, (m, n, k) in enumerate(cases):
+        akf, bkf, dnf = (bool(x) for x in rng.integers(0, 2, 3))
+        beta = 0.5 if i % 3 == 0 else 0.0
+        sa, sb, sd = [k, 1] if akf else [1, m], [1, k] if bkf else [n, 1], [n, 1] if dnf else [1, m]
+        a, b, d0 = rand(m * k), rand(k * n), rand(m * n)
+        spec = [tp.OperandSpec(tp.LayoutSpec(e, s)) for e, s in (([m, k], sa), ([k, n], sb), ([m, n], sd))]
+        prob = tp.Problem.from_labels(tp.F64, *spec, [0, 2], [2, 1], [0, 1])
+        want = a.as_strided([m, k], sa) @ b.as_strided([k, n], sb) + beta * d0.as_strided([m, n], sd)
+        d1, d2 = d0.clone(), d0.clone()
+        for d, plan, to in ((d1, tp.Plan(prob), items), (d2, tp.Plan(prob, tp.PlanConfig(kernel=3)), singles)):
+            c = d.data_ptr() if beta else None
+            to.append(tp.Item(plan, 1.0, a.data_ptr(), b.data_ptr(), d.data_ptr(), beta, c))
+        outs.append((a, b, d0, d1, d2, want, sd, [m, n]))
+    torch.cuda.synchronize()
+    batch = tp.PreparedBatch(items)
+    for rep in range(2):  # captured, then replayed
+        for o in outs:
+            o[3].copy_(o[2])
+        torch.cuda.synchronize()
+        batch.run(ex)
+        ex.synchronize()
+        for o, c in zip(outs, cases):
+            got = o[3].as_strided(o[7], o[6])
+            assert float((got - o[5]).norm() / o[5].norm()) <= 1e-13, (c, rep)
+    ex.set_grouping(False)
+    tp.PreparedBatch(singles).run(ex)
+    ex.synchronize()
+    for o, c in zip(outs, cases):
+        assert float((o[3] - o[4]).norm() / o[4].norm()) <= 1e-13, c
+    ex.close()
