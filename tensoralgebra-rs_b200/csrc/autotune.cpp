@@ -165,8 +165,10 @@ PlainChoice model_choice(const Product& p, int num_sms, bool general) {
   return c;
 }
 
-size_t stream_scratch(const Product& p, int64_t M, int64_t N) {
+size_t tc_scratch(int kernel, const Product& p, int64_t M, int64_t N) {
   const int dt = (int)p.problem.dtype;
+  if (dev::is_tc_split(kernel)) return dev::plain_split_bytes(dt, M, N, p.view.K, p.view.H) + 256;
+  if (!dev::is_tc_stream(kernel)) return 0;
   return (p.hints.a_gather ? 0 : dev::stream_panel_bytes(dt, M, p.view.K, p.view.H) + 256) +
          (p.hints.b_gather ? 0 : dev::stream_panel_bytes(dt, N, p.view.K, p.view.H) + 256);
 }
@@ -176,7 +178,7 @@ size_t plain_scratch(const PlainChoice& c, const Product& p) {
   size_t s = 0;
   if (dev::is_packed_kernel(c.kernel))
     s += dev::packed_workspace_bytes(dev::packed_layout(c.kernel, p.view.M, p.view.N, p.view.K, p.view.H)) + 512;
-  if (dev::is_tc_stream(c.kernel)) s += stream_scratch(p, p.view.M, p.view.N);
+  s += tc_scratch(c.kernel, p, p.view.M, p.view.N);
   if (c.splits > 1) s += (size_t)c.splits * p.view.H * p.view.M * p.view.N * dtype_size(p.problem.dtype) + 256;
   return s;
 }
@@ -188,7 +190,9 @@ bool choice_fits(const PlainChoice& c, const Product& p) {
   for (int f : kFamilies[(int)p.problem.dtype & 3]) fam_ok = fam_ok || (f != 0 && f == c.kernel);
   fam_ok = fam_ok || (dev::is_stream_kernel(c.kernel) && dev::stream_dtype(c.kernel) == (int)p.problem.dtype && K > 0 &&
                        (!dev::is_tc_stream(c.kernel) ||
-                        (c.splits == 1 && dev::tc_stream_fits((int)p.problem.dtype, M, N, K, H, p.hints))));
+                        (c.splits == 1 && dev::tc_stream_fits((int)p.problem.dtype, M, N, K, H, p.hints))) &&
+                       (!dev::is_tc_split(c.kernel) ||
+                        (c.splits == 1 && dev::tc_split_fits((int)p.problem.dtype, M, N, K, H))));
   if (c.kernel == dev::PLAIN_SMALL_BATCHED) return dev::small_batched_fits(M, N, K, H) && c.splits == 1;
   if (!fam_ok || c.splits < 1) return false;
   if (dev::is_packed_kernel(c.kernel) && !dev::packed_fits(c.kernel, M, N, K, H)) return false;

@@ -1379,10 +1379,7 @@ void choose_plain_launch(int dtype, int pinned, int64_t M, int64_t N, int64_t K,
                                 PLAIN_C64_PACKED_3M_64x32};
   *splits = 1;
   *k_chunk = 0;
-  if (!pinned && use_tc_stream(dtype, M, N, K, H, num_sms, hints)) {
-    *kernel = dtype == 0 ? PLAIN_F32_TC_STREAM : PLAIN_C32_TC_STREAM;
-    return;
-  }
+  if (!pinned && (*kernel = choose_tc_kernel(dtype, M, N, K, H, num_sms, hints)) != 0) return;
   const int64_t min_chunk = 512;  // K per split
   // Small f64 products (at most 64 large tiles, K up to 1024): the small direct
   // tile, K split until about two CTAs run per SM, without a pack pass (399 x 108

@@ -23,8 +23,16 @@
 //    (pack/writeback.rs:311-486). Every mbarrier wait is bounded by
 //    %globaltimer; a timeout sets a status bit and the kernel drains and
 //    returns. No cluster, no multicast.
+//
+// The same GEMM serves plain f32 and c32 contractions that are large enough to pay
+// for the planes' pass through HBM (PLAIN 1 and 2; smaller ones split on the way into
+// shared memory, k_tcstream.cu). c32 is embedded as the real product of 2M x N x 2K.
+// plain_split_pack_kernel also notes the range of the values it splits; outputs that
+// the planes may not carry to f32 rounding (split_guard) are computed again by FFMA.
 #include <cuda.h>
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "tc_common.cuh"
 
@@ -139,6 +147,111 @@ __global__ void __launch_bounds__(256) split_pack_kernel(const float* __restrict
   }
 }
 
+// Planes of a plain f32 or c32 operand: one 32-row x 64-deep (c32: 32 complex k)
+// tile per CTA, split into three planes [H][rows_pad][k_pad], K-major. c32: A' as
+// rows (re, -im) and (im, re), B' as (re, im), conjugation in the sign of im. The
+// tile's largest and smallest non-zero magnitudes (as bits) go to stat.
+template <bool CPLX, bool IS_A>
+__global__ void __launch_bounds__(256)
+plain_split_pack_kernel(const void* __restrict__ X, const int64_t* __restrict__ rows_scat,
+                        const int64_t* __restrict__ k_scat, const int64_t* __restrict__ h_scat,
+                        const int64_t* __restrict__ rows_blk, const int64_t* __restrict__ k_blk, int64_t nrows,
+                        int64_t K, int64_t rows_pad, int64_t k_pad, int64_t H, int kfast, int conj,
+                        __nv_bfloat16* __restrict__ out, uint2* __restrict__ stat) {
+  using T = typename std::conditional<CPLX, float2, float>::type;
+  constexpr int E = CPLX ? 2 : 1, EK = 64 / E, PR = CPLX && IS_A ? 2 : 1;
+  __shared__ float tile[32][65];
+  __shared__ uint2 part[8];
+  const int tid = threadIdx.x;
+  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * EK, h = blockIdx.z;
+  const T* base = static_cast<const T*>(X) + h_scat[h];
+  int64_t rs = SCATTER_IRREGULAR, ks = SCATTER_IRREGULAR;
+  if (rows_blk && k_blk && r0 + 32 <= nrows && k0 + EK <= K) {
+    rs = rows_blk[blockIdx.y];
+    ks = k_blk[k0 / SCATTER_BLOCK];
+    if (EK == 64 && ks != SCATTER_IRREGULAR &&
+        (k_blk[k0 / SCATTER_BLOCK + 1] != ks || k_scat[k0 + 32] - k_scat[k0] != 32 * ks))
+      ks = SCATTER_IRREGULAR;
+  }
+  const auto put = [&](int rr, int kk, T v) {
+    if constexpr (CPLX) {
+      tile[rr][2 * kk] = v.x;
+      tile[rr][2 * kk + 1] = conj ? -v.y : v.y;
+    } else {
+      tile[rr][kk] = v;
+    }
+  };
+  if (rs != SCATTER_IRREGULAR && ks != SCATTER_IRREGULAR) {
+    const T* tb = base + rows_scat[r0] + k_scat[k0];
+    const int64_t fs = kfast ? ks : rs, ss = kfast ? rs : ks;
+    constexpr int V = 16 / (int)sizeof(T);
+    if (fs == 1 && (reinterpret_cast<uintptr_t>(tb) & 15) == 0 && (ss & (V - 1)) == 0) {
+      const int tpr = (kfast ? EK : 32) / V;  // threads along the fast index
+#pragma unroll
+      for (int j = 0; j < 32 * EK / V / 256; ++j) {
+        const int a0 = (tid % tpr) * V, q = tid / tpr + j * (256 / tpr);
+        const float4 x = __ldg(reinterpret_cast<const float4*>(tb + q * ss + a0));
+        const T* e = reinterpret_cast<const T*>(&x);
+#pragma unroll
+        for (int i = 0; i < V; ++i) put(kfast ? q : a0 + i, kfast ? a0 + i : q, e[i]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32 * EK / 256; ++j) {
+        const int idx = tid + 256 * j, rr = kfast ? idx / EK : idx % 32, kk = kfast ? idx % EK : idx / 32;
+        put(rr, kk, __ldg(tb + rr * rs + kk * ks));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32 * EK / 256; ++j) {
+      const int idx = tid + 256 * j, rr = kfast ? idx / EK : idx % 32, kk = kfast ? idx % EK : idx / 32;
+      const int64_t r = r0 + rr, k = k0 + kk;
+      T v{};
+      if (r < nrows && k < K) v = base[rows_scat[r] + k_scat[k]];
+      put(rr, kk, v);
+    }
+  }
+  __syncthreads();
+  const int64_t plane = H * rows_pad * k_pad;
+  uint32_t mx = 0, mn = 0xffffffffu;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int p = tid + 256 * j, rr = p / 32, kp = p % 32;
+    const float x = tile[rr][2 * kp], y = tile[rr][2 * kp + 1];
+    const uint32_t bx = __float_as_uint(x) & 0x7fffffffu, by = __float_as_uint(y) & 0x7fffffffu;
+    mx = max(mx, max(bx, by));
+    mn = min(mn, min(bx - 1, by - 1));  // zero: the largest
+    __nv_bfloat16 a[3], c[3];
+    split3(x, a[0], a[1], a[2]);
+    split3(y, c[0], c[1], c[2]);
+    const int64_t off = (h * rows_pad + PR * (r0 + rr)) * k_pad + blockIdx.x * 64 + 2 * kp;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + q * plane + off);
+      if constexpr (CPLX && IS_A) {
+        if (PR * (r0 + rr) < rows_pad) {
+          o[0] = __halves2bfloat162(a[q], __hneg(c[q]));
+          o[k_pad / 2] = __halves2bfloat162(c[q], a[q]);
+        }
+      } else {
+        o[0] = __halves2bfloat162(a[q], c[q]);
+      }
+    }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  if ((tid & 31) == 0) part[tid >> 5] = make_uint2(mx, mn);
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < 8; ++w) {
+      mx = max(mx, part[w].x);
+      mn = min(mn, part[w].y);
+    }
+    stat[(h * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = make_uint2(mx, mn);
+  }
+}
+
 template <int S>
 struct Pairs;
 template <>
@@ -175,6 +288,49 @@ __host__ __device__ inline void tile_coords(int64_t tile, int64_t tiles_m, int64
   nt = local / gm;
 }
 
+// split_guard of every tile from the pack's ranges: arb, brb pack rows of a tile of
+// an_rb, bn_rb in all, nkb depth blocks.
+__global__ void __launch_bounds__(128) split_guard_kernel(const uint2* __restrict__ sa, const uint2* __restrict__ sb,
+                                                          int64_t tiles_m, int64_t tiles_n, int64_t an_rb, int64_t bn_rb,
+                                                          int arb, int brb, int nkb, float* __restrict__ thr) {
+  int64_t h, mt, nt;
+  tile_coords(blockIdx.x, tiles_m, tiles_n, h, mt, nt);
+  uint32_t m[2] = {0, 0}, l[2] = {0xffffffffu, 0xffffffffu};
+  const int64_t a0 = mt * arb, b0 = nt * brb;
+  const int na = (int)(a0 + arb < an_rb ? arb : an_rb - a0) * nkb, nb = (int)(b0 + brb < bn_rb ? brb : bn_rb - b0) * nkb;
+  for (int i = threadIdx.x; i < na; i += 128) {
+    const uint2 v = sa[(h * an_rb + a0) * nkb + i];
+    m[0] = max(m[0], v.x);
+    l[0] = min(l[0], v.y);
+  }
+  for (int i = threadIdx.x; i < nb; i += 128) {
+    const uint2 v = sb[(h * bn_rb + b0) * nkb + i];
+    m[1] = max(m[1], v.x);
+    l[1] = min(l[1], v.y);
+  }
+  __shared__ uint32_t part[4][4];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    m[q] = __reduce_max_sync(0xffffffffu, m[q]);
+    l[q] = __reduce_min_sync(0xffffffffu, l[q]);
+    if ((threadIdx.x & 31) == 0) {
+      part[threadIdx.x >> 5][q] = m[q];
+      part[threadIdx.x >> 5][2 + q] = l[q];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      for (int w = 1; w < 4; ++w) {
+        m[q] = max(m[q], part[w][q]);
+        l[q] = min(l[q], part[w][2 + q]);
+      }
+    const auto low = [](uint32_t x) { return x == 0xffffffffu ? 999 : (int)((x + 1) >> 23) - 127; };
+    thr[blockIdx.x] = split_guard((int)(m[0] >> 23) - 127, low(l[0]), (int)(m[1] >> 23) - 127, low(l[1]));
+  }
+}
+
 template <int S, int BN>
 struct TcCfg {
   static constexpr int A_TILE = TC_BM * TC_BK * 2;  // bytes of one A plane tile
@@ -204,10 +360,13 @@ struct TcCfg {
 // tail CTA writes its FP32 sum to partial[(tail tile * parts + part) * TC_BM
 // * BN + col * TC_BM + row] and split_tail_reduce_kernel adds the parts in
 // order and applies the epilogue.
-template <int S, int BN, int CK>
+//
+// PLAIN 0: the split schemes; 1 and 2: plain f32 and c32, with the tiles' thresholds.
+template <int S, int BN, int CK, int PLAIN>
 __global__ void __launch_bounds__(TcCfg<S, BN>::THREADS, 1)
 tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g,
-                    int64_t m_pad, int64_t n_pad, int64_t k_pad, int64_t whole, int parts, float* partial) {
+                    int64_t m_pad, int64_t n_pad, int64_t k_pad, int64_t whole, int parts, float* partial,
+                    const float* __restrict__ thr_of) {
   using Cfg = TcCfg<S, BN>;
   constexpr int CPT = Cfg::COLS_PER_THREAD;
   extern __shared__ uint8_t smem_raw[];
@@ -359,12 +518,16 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_before();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(main_empty)) : "memory");
     }
-    const int64_t m = m0 + lane_base + lane;
+    constexpr bool CPLX = PLAIN == 2;
+    const int64_t m = CPLX ? (m0 + lane_base + lane) >> 1 : m0 + lane_base + lane;
     const bool mok = ok && m < g.M;
     const int64_t dm = mok ? g.s.d_m[m] : 0;
     const int64_t cm = (mok && !g.e.beta_zero) ? g.s.c_m[m] : 0;
-    const float* Cb = static_cast<const float*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h]) + cm;
-    float* Db = static_cast<float*>(g.D) + g.s.h_d[h] + dm;
+    using T = typename Elem<float, CPLX>::type;
+    const T* Cb = static_cast<const T*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h]) + cm;
+    T* Db = static_cast<T*>(g.D) + g.s.h_d[h] + dm;
+    const float thr = PLAIN ? thr_of[tile] : 0.f;
+    uint32_t again[CPT / 32] = {};
     float* Pb = part >= 0 ? partial + ((tile - whole) * parts + part) * (int64_t)(TC_BM * BN) + lane_base + lane
                           : nullptr;
     // The last main_full commit also covers every cross-term MMA.
@@ -377,15 +540,59 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         // Tail part: the raw FP32 sum, column-major in the tile (coalesced).
 #pragma unroll
         for (int j = 0; j < 16; ++j) Pb[(col0 + 16 * q + j) * TC_BM] = run[16 * q + j] + __uint_as_float(r[j]);
+      } else if constexpr (PLAIN != 0) {
+        const int comp = CPLX ? lane & 1 : 0;
+        constexpr int CG = CPLX ? 4 : 8;
+        if (thr == 0.f && g.e.plain) {
+          if (mok) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const int nn = col0 + 16 * q + j;
+              if (n0 + nn < g.N)
+                reinterpret_cast<float*>(Db + dn_s[nn])[comp] = run[16 * q + j] + __uint_as_float(r[j]);
+            }
+          }
+          __syncwarp();
+          continue;
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < 16; j0 += CG) {
+          T cv[CG];  // C of the group, on its way before the first of it is used
+          if (!g.e.beta_zero) {
+#pragma unroll
+            for (int j = 0; j < CG; ++j)
+              if (mok && n0 + col0 + 16 * q + j0 + j < g.N && !comp) cv[j] = Cb[cn_s[col0 + 16 * q + j0 + j]];
+          }
+#pragma unroll
+          for (int j = 0; j < CG; ++j) {
+            const int jj = 16 * q + j0 + j, nn = col0 + jj;
+            const float v = run[jj] + __uint_as_float(r[j0 + j]);
+            const float o = CPLX ? __shfl_xor_sync(0xffffffffu, v, 1) : 0.f;
+            if (!mok || n0 + nn >= g.N || comp) continue;
+            if (split_lost(thr, v) || (CPLX && split_lost(thr, o)))
+              again[jj / 32] |= 1u << (jj % 32);
+            else
+              epilogue_store<float, CPLX>(g.e, v, o, &cv[j], Db + dn_s[nn]);
+          }
+        }
       } else if (mok) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int nn = col0 + 16 * q + j;
           if (n0 + nn < g.N)
-            epilogue_store<float, false>(g.e, run[16 * q + j] + __uint_as_float(r[j]), 0.f, Cb + cn_s[nn],
-                                         Db + dn_s[nn]);
+            epilogue_store<float, CPLX>(g.e, run[16 * q + j] + __uint_as_float(r[j]), 0.f, Cb + cn_s[nn],
+                                        Db + dn_s[nn]);
         }
       }
+    }
+    if constexpr (PLAIN != 0) {
+#pragma unroll
+      for (int w = 0; w < CPT / 32; ++w)
+        for (uint32_t bits = again[w]; bits; bits &= bits - 1) {
+          const int nn = col0 + 32 * w + __ffs(bits) - 1;
+          const float2 v = ffma_dot<CPLX>(g, h, m, n0 + nn);
+          epilogue_store<float, CPLX>(g.e, v.x, v.y, Cb + cn_s[nn], Db + dn_s[nn]);
+        }
     }
   }
 
@@ -398,10 +605,12 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // Tail tiles: add the parts in order, then the epilogue through the scatter.
-template <int BN>
+template <int BN, int PLAIN>
 __global__ void __launch_bounds__(256) split_tail_reduce_kernel(GemmArgs g, const float* __restrict__ partial,
                                                                 int64_t whole, int parts, int64_t tail, int64_t m_pad,
-                                                                int64_t n_pad) {
+                                                                int64_t n_pad, const float* __restrict__ thr_of) {
+  constexpr bool CPLX = PLAIN == 2;
+  using T = typename Elem<float, CPLX>::type;
   const int64_t tiles_n = n_pad / BN, tiles_m = m_pad / TC_BM;
   const int64_t total = tail * TC_BM * BN;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -411,13 +620,21 @@ __global__ void __launch_bounds__(256) split_tail_reduce_kernel(GemmArgs g, cons
     const int64_t tile = whole + t;
     int64_t h, mt, nt;
     tile_coords(tile, tiles_m, tiles_n, h, mt, nt);
-    const int64_t m = mt * TC_BM + row, n = nt * BN + col;
-    if (m >= g.M || n >= g.N) continue;
-    float v = 0.f;
-    for (int p = 0; p < parts; ++p) v += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within];
-    const float* c = static_cast<const float*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h] + g.s.c_m[m] + g.s.c_n[n]);
-    float* d = static_cast<float*>(g.D) + g.s.h_d[h] + g.s.d_m[m] + g.s.d_n[n];
-    epilogue_store<float, false>(g.e, v, 0.f, c, d);
+    const int64_t m = CPLX ? (mt * TC_BM + row) >> 1 : mt * TC_BM + row, n = nt * BN + col;
+    if (m >= g.M || n >= g.N || (CPLX && (row & 1))) continue;
+    float v = 0.f, o = 0.f;
+    for (int p = 0; p < parts; ++p) {
+      v += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within];
+      if (CPLX) o += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within + 1];
+    }
+    if (PLAIN && (split_lost(thr_of[tile], v) || (CPLX && split_lost(thr_of[tile], o)))) {
+      const float2 x = ffma_dot<CPLX>(g, h, m, n);
+      v = x.x;
+      o = x.y;
+    }
+    const T* c = static_cast<const T*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h] + g.s.c_m[m] + g.s.c_n[n]);
+    T* d = static_cast<T*>(g.D) + g.s.h_d[h] + g.s.d_m[m] + g.s.d_n[n];
+    epilogue_store<float, CPLX>(g.e, v, o, c, d);
   }
 }
 
@@ -428,12 +645,14 @@ struct TailSplit {
   int64_t whole, tail;
   int parts;
 };
-inline TailSplit tail_split(int64_t tiles, int sms, int nk, int ck) {
+// `deep`: also a first wave that is partly filled (up to 16 parts).
+inline TailSplit tail_split(int64_t tiles, int sms, int nk, int ck, bool deep = false) {
   TailSplit t{tiles, 0, 1};
   const int64_t rem = tiles % sms;
-  if (rem == 0 || tiles < sms) return t;  // full waves, or one partial wave of whole tiles
+  if (rem == 0 || (tiles < sms && !deep)) return t;  // full waves, or one partial wave of whole tiles
   int parts = (int)(sms / rem);
-  parts = parts < 4 ? parts : 4;
+  const int most = tiles < sms ? 16 : 4;
+  parts = parts < most ? parts : most;
   // Each part keeps at least two CK chunks and the last part is not empty.
   auto fits = [&](int p) {
     const int per = ((nk + p - 1) / p + ck - 1) / ck * ck;
@@ -447,9 +666,11 @@ inline TailSplit tail_split(int64_t tiles, int sms, int nk, int ck) {
   return t;
 }
 
-template <int S, int BN, int CK>
+constexpr int TC_PLAIN_SMS = 148;  // what the plain path's workspace is sized for
+
+template <int S, int BN, int CK, int PLAIN = 0>
 cudaError_t run_tc(const GemmArgs& g, const SplitLayout& L, const void* ap, const void* bp, float* tail_partial,
-                   cudaStream_t st) {
+                   cudaStream_t st, const float* thr = nullptr) {
   using Cfg = TcCfg<S, BN>;
   CUtensorMap ma, mb;
   if (!make_map_2d(&ma, ap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, L.k_pad, (int64_t)S * L.H * L.m_pad, TC_BK, TC_BM))
@@ -458,24 +679,25 @@ cudaError_t run_tc(const GemmArgs& g, const SplitLayout& L, const void* ap, cons
     return cudaErrorInvalidValue;
   // Per call: the attribute belongs to the current device's context.
   cudaError_t e =
-      cudaFuncSetAttribute(tc_bf16_gemm_kernel<S, BN, CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+      cudaFuncSetAttribute(tc_bf16_gemm_kernel<S, BN, CK, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
   if (e != cudaSuccess) return e;
   const int64_t tiles = (L.n_pad / BN) * (L.m_pad / TC_BM) * L.H;
   TailSplit ts{tiles, 0, 1};
   if (tail_partial) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ts = tail_split(tiles, sms, (int)(L.k_pad / TC_BK), CK);
+    if (PLAIN && sms > TC_PLAIN_SMS) sms = TC_PLAIN_SMS;
+    ts = tail_split(tiles, sms, (int)(L.k_pad / TC_BK), CK, PLAIN != 0);
   }
   const int64_t grid = ts.whole + ts.tail * ts.parts;
-  tc_bf16_gemm_kernel<S, BN, CK><<<(unsigned)grid, Cfg::THREADS, Cfg::SMEM, st>>>(
-      ma, mb, g, L.m_pad, L.n_pad, L.k_pad, ts.whole, ts.parts, tail_partial);
+  tc_bf16_gemm_kernel<S, BN, CK, PLAIN><<<(unsigned)grid, Cfg::THREADS, Cfg::SMEM, st>>>(
+      ma, mb, g, L.m_pad, L.n_pad, L.k_pad, ts.whole, ts.parts, tail_partial, thr);
   e = cudaGetLastError();
   if (e != cudaSuccess || ts.tail == 0) return e;
   const int64_t elems = ts.tail * TC_BM * BN;
   const unsigned blocks = (unsigned)((elems + 255) / 256 < 4096 ? (elems + 255) / 256 : 4096);
-  split_tail_reduce_kernel<BN><<<blocks, 256, 0, st>>>(g, tail_partial, ts.whole, ts.parts, ts.tail, L.m_pad,
-                                                       L.n_pad);
+  split_tail_reduce_kernel<BN, PLAIN><<<blocks, 256, 0, st>>>(g, tail_partial, ts.whole, ts.parts, ts.tail, L.m_pad,
+                                                              L.n_pad, thr);
   return cudaGetLastError();
 }
 
@@ -527,6 +749,82 @@ cudaError_t launch_tc_bf16_gemm(const GemmArgs& g, const SplitLayout& L, const v
   float* tp = static_cast<float*>(tail_partial);
   if (scheme == 2) return run_tc<3, 256, 4>(g, L, ap, bp, tp, st);
   return run_tc<2, 256, 4>(g, L, ap, bp, tp, st);
+}
+
+// ---- plain f32 / c32 --------------------------------------------------------
+
+namespace {
+// The workspace: A' planes, B' planes, their ranges, the tiles' thresholds, the tail
+// parts.
+struct PlainSplitSpace {
+  size_t b, sa, sb, thr, tail, bytes;
+  int64_t a_rb, b_rb, nkb;
+};
+PlainSplitSpace plain_split_space(int dtype, const SplitLayout& L) {
+  const auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+  PlainSplitSpace s;
+  s.a_rb = L.m_pad / (dtype == 2 ? 64 : 32);
+  s.b_rb = L.n_pad / 32;
+  s.nkb = L.k_pad / 64;
+  s.b = up((size_t)3 * L.H * L.m_pad * L.k_pad * 2);
+  s.sa = s.b + up((size_t)3 * L.H * L.n_pad * L.k_pad * 2);
+  s.sb = s.sa + up((size_t)L.H * s.a_rb * s.nkb * 8);
+  s.thr = s.sb + up((size_t)L.H * s.b_rb * s.nkb * 8);
+  s.tail = s.thr + up((size_t)(L.m_pad / TC_BM) * (L.n_pad / 256) * L.H * 4);
+  s.bytes = s.tail + up(split_tail_bytes(L, TC_PLAIN_SMS));
+  return s;
+}
+}  // namespace
+
+bool is_tc_split(int kernel) { return kernel == PLAIN_F32_TC_SPLIT || kernel == PLAIN_C32_TC_SPLIT; }
+
+SplitLayout plain_split_layout(int dtype, int64_t M, int64_t N, int64_t K, int64_t H) {
+  return split_layout(2, dtype == 2 ? 2 * M : M, N, dtype == 2 ? 2 * K : K, H);
+}
+size_t plain_split_bytes(int dtype, int64_t M, int64_t N, int64_t K, int64_t H) {
+  const SplitLayout a = plain_split_layout(dtype, M, N, K, H), b = plain_split_layout(dtype, N, M, K, H);
+  const size_t x = plain_split_space(dtype, a).bytes, y = plain_split_space(dtype, b).bytes;
+  return (x > y ? x : y) + 256;  // either orientation
+}
+
+bool tc_split_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H) {
+  if ((dtype != 0 && dtype != 2) || K <= 0 || H > 65535) return false;
+  const int64_t most = (int64_t)1 << 30;
+  if (M >= most / 8 || N >= most / 8 || K >= most / 8) return false;
+  const int64_t rows = (M > N ? M : N) * 2 + 256;
+  return rows / 32 <= 65535 && 3 * H * rows < 2 * most && (M / 64 + 2) * (N / 64 + 2) * H < most;
+}
+
+cudaError_t launch_plain_split_pack(int dtype, const GemmArgs& g, int which, void* ws, cudaStream_t st) {
+  const SplitLayout L = plain_split_layout(dtype, g.M, g.N, g.K, g.H);
+  const PlainSplitSpace S = plain_split_space(dtype, L);
+  char* w = static_cast<char*>(ws);
+  const bool a = which == 0;
+  const dim3 grid((unsigned)S.nkb, (unsigned)(a ? S.a_rb : S.b_rb), (unsigned)L.H);
+  auto kern = dtype == 2 ? (a ? plain_split_pack_kernel<true, true> : plain_split_pack_kernel<true, false>)
+                         : (a ? plain_split_pack_kernel<false, true> : plain_split_pack_kernel<false, false>);
+  kern<<<grid, 256, 0, st>>>(a ? g.A : g.B, a ? g.s.a_m : g.s.b_n, a ? g.s.a_k : g.s.b_k, a ? g.s.h_a : g.s.h_b,
+                             a ? g.s.blk_a_m : g.s.blk_b_n, a ? g.s.blk_a_k : g.s.blk_b_k, a ? g.M : g.N, g.K,
+                             a ? L.m_pad : L.n_pad, L.k_pad, L.H, a ? g.a_kfast : g.b_kfast, a ? g.conj_a : g.conj_b,
+                             reinterpret_cast<__nv_bfloat16*>(a ? w : w + S.b),
+                             reinterpret_cast<uint2*>(w + (a ? S.sa : S.sb)));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_plain_split_gemm(int dtype, const GemmArgs& g, void* ws, cudaStream_t st) {
+  const SplitLayout L = plain_split_layout(dtype, g.M, g.N, g.K, g.H);
+  const PlainSplitSpace S = plain_split_space(dtype, L);
+  char* w = static_cast<char*>(ws);
+  const int64_t tm = L.m_pad / TC_BM, tn = L.n_pad / 256;
+  float* thr = reinterpret_cast<float*>(w + S.thr);
+  split_guard_kernel<<<(unsigned)(tm * tn * L.H), 128, 0, st>>>(
+      reinterpret_cast<const uint2*>(w + S.sa), reinterpret_cast<const uint2*>(w + S.sb), tm, tn, S.a_rb, S.b_rb,
+      dtype == 2 ? 2 : 4, 8, (int)S.nkb, thr);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  float* tail = reinterpret_cast<float*>(w + S.tail);
+  return dtype == 2 ? run_tc<3, 256, 4, 2>(g, L, w, w + S.b, tail, st, thr)
+                    : run_tc<3, 256, 4, 1>(g, L, w, w + S.b, tail, st, thr);
 }
 
 }  // namespace dev

@@ -673,6 +673,7 @@ const StreamFamily kStream[] = {
     {1, 64, 64, "sm100.f64.dmma884.stream.64x64x16"},   {1, 128, 32, "sm100.f64.dmma884.stream.128x32x16"},
     {1, 64, 48, "sm100.f64.dmma884.stream.64x48x16"},   {1, 32, 128, "sm100.f64.dmma884.stream.32x128x16"},
     {0, 128, 128, "sm100.f32.tcgen05.stream.128x128x32"}, {2, 64, 128, "sm100.c32.tcgen05.stream.64x128x32"},
+    {0, 128, 256, "sm100.f32.tcgen05.tma.split.128x256x32"}, {2, 64, 256, "sm100.c32.tcgen05.tma.split.64x256x32"},
 };
 
 }  // namespace

@@ -32,6 +32,9 @@
 // and so is an output small enough to have lost bits to underflow.
 //
 // Every wait is bounded (a status bit, then the role ends). No cluster, no multicast.
+#include <algorithm>
+#include <cmath>
+
 #include "tc_common.cuh"
 
 namespace tprims {
@@ -563,21 +566,23 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
               }
             }
           } else {
-#pragma unroll 1
-            for (int j = 0; j < 8; ++j) {
-              // v[j] without a dynamic register index.
-              float y = v[0];
+            // C of four columns is on its way before the first of it is used.
 #pragma unroll
-              for (int i = 1; i < 8; ++i) y = j == i ? v[i] : y;
-              const int jj = 8 * q + j;
-              const float o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
-              bool low = split_lost(thr, y);
-              if (CPLX) low = low || split_lost(thr, o);
-              if (jj >= nrem || !mok || comp) continue;
-              if (low)
-                again |= (uint64_t)1 << jj;
-              else
-                epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
+            for (int j0 = 0; j0 < 8; j0 += 4) {
+              T cv[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (!e.beta_zero && mok && !comp && 8 * q + j0 + j < nrem) cv[j] = Cb[cn_s[8 * q + j0 + j]];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int jj = 8 * q + j0 + j;
+                const float y = v[j0 + j], o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
+                if (jj >= nrem || !mok || comp) continue;
+                if (split_lost(thr, y) || (CPLX && split_lost(thr, o)))
+                  again |= (uint64_t)1 << jj;
+                else
+                  epilogue_store<float, CPLX>(e, y, o, &cv[j], Db + dn_s[jj]);
+              }
             }
           }
           __syncwarp();
@@ -707,23 +712,37 @@ bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const
 // in six indexes 89 against 235, 2048^2 x 64 17 against 32, x 1024 87 against 217,
 // 120000 x 31 x 33 37 against 90, 16 x 100^3 batch innermost 26 against 17, 300 x 260 x
 // 2000 (63 stages on nine SMs) 76 against 40 with split-K; c32 2048^2 x 512 178 against
-// 402, 700^2 x 2500 226 against 373. Below 2^23 products the launches decide; beyond K = 1024 the
-// packed panels' single pass over the operands is kept.
-bool use_tc_stream(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
-  if (!tc_stream_fits(dtype, M, N, K, H, hints)) return false;
+// 402, 700^2 x 2500 226 against 373. Below 2^23 products the launches decide.
+// Over planes packed first (k_split.cu) the split is paid once, not once per tile: 16,
+// the planes' bytes at 4 TB/s, and 20 + 0.038 per plane depth for a wave of 128 x 256
+// tiles, whose depth is split where the wave is partly filled (f32 4096^3 0.67 ms
+// against 1.21 here and 2.70 there, 2048^2 x 512 55 against 51 here; c32 2048^3 0.41
+// ms against 0.66 here and 1.53 there; f32 700^2 x 2500 against 108 here, 94 there).
+int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
+  if (!tc_stream_fits(dtype, M, N, K, H, hints)) return 0;
   const bool cplx = dtype == 2;
   const int64_t m = hints.d_mfast ? M : N, n = hints.d_mfast ? N : M;  // the launch's roles
   const int64_t em = cplx ? TS_BM / 2 : TS_BM, ek = cplx ? TS_BK / 2 : TS_BK, pad = cplx ? 64 : 128;
   const int64_t tiles = ((m + em - 1) / em) * ((n + TS_BN - 1) / TS_BN) * H;
   const double outs = (double)M * (double)N * (double)H, per = cplx ? 4 : 1;
-  if (K > 1024 || tiles < 16 || outs * (double)K * per < (double)(1 << 23)) return false;
+  if (tiles < 16 || outs * (double)K * per < (double)(1 << 23)) return 0;
   const double waves = (double)((tiles + num_sms - 1) / num_sms), stages = (double)((K + ek - 1) / ek);
   const double here = 8 + waves * ((n <= 64 ? 1.5 : 4) + (cplx ? 1.25 : 1.1) * stages) +
                       4 * ((hints.a_gather ? 0 : 1) + (hints.b_gather ? 0 : 1));
   const double whole = (double)((M + pad - 1) / pad * pad) * (double)((N + pad - 1) / pad * pad) * (double)H;
   const double there = (K >= 64 ? 26 : 12) + 2 * per * whole * (double)K / (cplx ? 40e6 : 50e6) +
                        outs * (cplx ? 8e-6 : 4e-6);
-  return here < there;
+  double split = 1e30;
+  if (tc_split_fits(dtype, M, N, K, H)) {
+    const double mp = (double)((m * (cplx ? 2 : 1) + 127) / 128 * 128), np = (double)((n + 255) / 256 * 256);
+    const double kp = (double)((K * (cplx ? 2 : 1) + 63) / 64 * 64), t = mp / 128 * np / 256 * (double)H;
+    const double parts = t < num_sms ? std::min(std::min(16.0, std::floor(num_sms / t)), std::floor(kp / 256)) : 1;
+    const double w = t <= num_sms ? 1 : t / num_sms + 0.15;
+    split = 16 + ((mp + np) * kp * 6 + (double)(m + n) * (double)K * (cplx ? 8 : 4)) * (double)H / 4e6 +
+            (parts > 1 ? 25 + 0.038 * kp / parts : w * (20 + 0.038 * kp));
+  }
+  if (split < here && split < there) return cplx ? PLAIN_C32_TC_SPLIT : PLAIN_F32_TC_SPLIT;
+  return here < there ? (cplx ? PLAIN_C32_TC_STREAM : PLAIN_F32_TC_STREAM) : 0;
 }
 
 // The caller has checked tc_stream_fits.

@@ -111,7 +111,10 @@ enum PlainKernel : int {
   // Tensor cores, f32 split on the way into shared memory (k_tcstream.cu).
   PLAIN_F32_TC_STREAM = 25,
   PLAIN_C32_TC_STREAM = 26,
-  PLAIN_STREAM_LAST = 26,
+  // Tensor cores over BF16 planes packed first (k_split.cu).
+  PLAIN_F32_TC_SPLIT = 27,
+  PLAIN_C32_TC_SPLIT = 28,
+  PLAIN_STREAM_LAST = 28,
   // Batches of small products (k_small.cu): chosen by the model, never pinned.
   PLAIN_SMALL_BATCHED = 40,
 };
@@ -139,7 +142,8 @@ cudaError_t launch_stream_grouped(int kernel, const GroupItem* items, const int6
 bool is_tc_stream(int kernel);
 cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st);
 bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints);
-bool use_tc_stream(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
+// The tensor-core family the model takes for a plain f32 or c32 contraction (0: none).
+int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
 // Dense panel of one operand (0 = A', 1 = B') whose gather is not coalesced: its
 // bytes, and the pass that writes it and points `g` at it. `fast`: the index of
 // the operand's smallest stride (0 rows, 1 depth, 2 batch).
@@ -303,6 +307,15 @@ int split_tail_parts(const SplitLayout& L, int num_sms);
 // Bytes of packed workspace a split scheme needs.
 size_t split_workspace_bytes(const SplitLayout& L);
 SplitLayout split_layout(int scheme, int64_t M, int64_t N, int64_t K, int64_t H);
+
+// Plain f32 / c32 over three packed planes: workspace bytes, the pack of A' (which 0)
+// and B' (1), then the thresholds and the GEMM. `g` in the kernel's orientation
+// (stream_oriented).
+bool is_tc_split(int kernel);
+bool tc_split_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H);
+size_t plain_split_bytes(int dtype, int64_t M, int64_t N, int64_t K, int64_t H);
+cudaError_t launch_plain_split_pack(int dtype, const GemmArgs& g, int which, void* ws, cudaStream_t st);
+cudaError_t launch_plain_split_gemm(int dtype, const GemmArgs& g, void* ws, cudaStream_t st);
 
 // ---- Ozaki INT8 slices (f64 / c64 on tensor cores) -------------------------
 

@@ -617,13 +617,29 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const Plai
     }
     return;
   }
-  if (dev::is_tc_stream(c.kernel)) {
-    // Complex elements are gathered whole: operands off their natural alignment
+  if (dev::is_tc_stream(c.kernel) || dev::is_tc_split(c.kernel)) {
+    // Complex elements are loaded whole: operands off their natural alignment
     // take the direct tile.
     if (dt == 2 && ((reinterpret_cast<uintptr_t>(g0.A) | reinterpret_cast<uintptr_t>(g0.B)) & 7) != 0) {
       PlainChoice d = c;
       d.kernel = dev::PLAIN_C32_SIMT_64x64;
       return launch_plain(pr, ex, g0, d, scratch, scratch_bytes);
+    }
+    if (dev::is_tc_split(c.kernel)) {
+      if (dev::plain_split_bytes(dt, g.M, g.N, g.K, g.H) > scratch_bytes)
+        throw Error(ERR_INTERNAL, "split plane workspace too small");
+      g = dev::stream_oriented(g);
+      char* ws = reinterpret_cast<char*>(align_up((uintptr_t)scratch, 256));
+      {
+        Timed t(ex, "split_pack");
+        cudaStream_t side = fork_side(ex);  // B' packs on a side stream, joined back below
+        check_cuda(dev::launch_plain_split_pack(dt, g, 1, ws, side), "split pack B");
+        check_cuda(dev::launch_plain_split_pack(dt, g, 0, ws, ex.stream), "split pack A");
+        join_side(ex);
+      }
+      Timed t(ex, dev::plain_kernel_name(c.kernel));
+      check_cuda(dev::launch_plain_split_gemm(dt, g, ws, ex.stream), "tcgen05 contraction launch");
+      return;
     }
     for (int which = 0; which < 2; ++which) {
       if (which == 0 ? pr.hints.a_gather : pr.hints.b_gather) continue;
@@ -1135,7 +1151,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
       if (dev::is_packed_kernel(pc.kernel))
         scratch = std::max(scratch,
                            dev::packed_workspace_bytes(dev::packed_layout(pc.kernel, mc, ncols, v.K, v.H)) + 512);
-      if (dev::is_tc_stream(pc.kernel)) scratch = std::max(scratch, stream_scratch(pr, mc, ncols));
+      scratch = std::max(scratch, tc_scratch(pc.kernel, pr, mc, ncols));
     }
     return true;
   };

@@ -254,8 +254,9 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
 // The model's choice (heuristics), honouring the tile and split pins.
 // `general`: without the layout's hints (the families that take any layout).
 PlainChoice model_choice(const Product& p, int num_sms, bool general = false);
-// Dense panels of the operands whose gather is not coalesced (tensor-core stream tiles).
-size_t stream_scratch(const Product& p, int64_t M, int64_t N);
+// Workspace of a tensor-core family: the panels of operands whose gather is not
+// coalesced, or the packed planes.
+size_t tc_scratch(int kernel, const Product& p, int64_t M, int64_t N);
 // Scratch bytes a plain choice needs (split-K partials).
 size_t plain_scratch(const PlainChoice& c, const Product& p);
 // Whether a choice (from a tuning-cache file, say) is valid for a product: a

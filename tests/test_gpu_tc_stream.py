@@ -1,5 +1,6 @@
 """f32 and c32 contractions on the tensor cores with the operands split on the way
-into shared memory (csrc/k_tcstream.cu), through the C ABI on a B200.
+into shared memory (csrc/k_tcstream.cu) or, where large, into BF16 planes first (csrc/k_split.cu), on a
+B200.
 
 Against the extended-precision label oracle at the plain bound (relative Frobenius
 1e-6) over the forms the rule accepts: either index fast in each operand, 16-byte
@@ -204,3 +205,101 @@ def test_values_outside_the_planes(tp, ex, torch_cuda, orc, dt, case):
         assert np.all(np.abs(x.astype("float64") - y.astype("float64")) <= 2 * lim)
     else:
         assert orc.rel_frobenius(x[ok], y[ok].astype("float64")) <= plain_tol(dt)
+
+
+# (spec, extents, A conj, D permuted strides, beta): rows and columns past a tile, K past a
+# chunk, an only wave whose depth is split, a last wave that is, batches, strided gathers.
+SPLIT_FORMS = [
+    ("km,kn->mn", dict(m=1100, n=1300, k=2500), True, False, 0.0),
+    ("mk,nk->nm", dict(m=1025, n=1281, k=2411), False, False, 0.5),
+    ("mk,kn->mn", dict(m=4100, n=2309, k=1530), True, False, 0.5),
+    ("mkh,knh->mnh", dict(m=700, n=900, k=2090, h=9), False, False, 0.0),
+    ("kmlo,nlpk->mnop", dict(k=47, m=40, l=50, o=36, n=33, p=40), True, False, 0.0),
+]
+
+
+def split_case(torch, tp, dt, form, seed=5):
+    spec, e, conj, _, beta = form
+    if dt == "float32":
+        e = dict(e, m=2 * e["m"])  # enough work for the planes' pass
+    ta, tb, td = spec.replace("->", ",").split(",")
+    tdt = getattr(torch, dt)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+
+    def make(term):
+        ext = [e[x] for x in term]
+        st = np.cumprod([1] + ext[:-1]).tolist()
+        return torch.randn(int(np.prod(ext)), dtype=tdt, device="cuda", generator=gen).as_strided(ext, st)
+
+    A, B, D = make(ta), make(tb), make(td)
+    conj = conj and dt.startswith("complex")
+    lay = lambda t, c=False: tp.OperandSpec(tp.LayoutSpec(list(t.shape), list(t.stride())), c)
+    code = {"float32": tp.F32, "complex64": tp.C32}[dt]
+    lab = lambda t: [ord(x) for x in t]
+    prob = tp.Problem.from_labels(code, lay(A, conj), lay(B), lay(D), lab(ta), lab(tb), lab(td))
+    return A, B, D, conj, prob
+
+
+@pytest.mark.parametrize("dt", sorted(DIRECT))
+@pytest.mark.parametrize("form", SPLIT_FORMS, ids=lambda f: f[0])
+def test_planes_packed_first(tp, torch_cuda, dt, form):
+    torch = torch_cuda
+    ex = tp.Executor(device=0, stream=torch.cuda.current_stream().cuda_stream, sync=False)
+    A, B, D, conj, prob = split_case(torch, tp, dt, form)
+    plan = tp.Plan(prob)
+    assert ".tma.split." in plan.report()["family"], plan.report()["family"]
+    wide = torch.complex128 if dt.startswith("complex") else torch.float64
+    a = A.to(wide).conj() if conj else A.to(wide)
+    want = torch.einsum(form[0], a, B.to(wide)) + form[4] * D.to(wide)
+    if form[4]:
+        plan.execute_into_accum(ex, 1.0, A, B, form[4], D, c=D)
+    else:
+        plan.execute_into(ex, 1.0, A, B, D)
+    torch.cuda.synchronize()
+    assert float((D.to(wide) - want).norm() / want.norm()) <= plain_tol(dt)
+    ex.close()
+
+
+@pytest.mark.parametrize("case", ["inf", "nan", "overflow", "tiny", "denormal"])
+@pytest.mark.parametrize("form", [SPLIT_FORMS[0], SPLIT_FORMS[2]], ids=["split wave", "split tail"])
+@pytest.mark.parametrize("dt", sorted(DIRECT))
+def test_values_outside_the_packed_planes(tp, torch_cuda, dt, form, case):
+    """As from the direct tile; a few rows and columns hold the values, so that the
+    other tiles stay on the tensor cores."""
+    torch = torch_cuda
+    ex = tp.Executor(device=0, stream=torch.cuda.current_stream().cuda_stream, sync=False)
+    A, B, D, conj, prob = split_case(torch, tp, dt, form[:4] + (0.0,))
+    ta = form[0].split(",")[0]
+    rows = A if ta[0] == "m" else A.transpose(0, 1)  # [m, k]
+    cols = B.transpose(0, 1)                         # [n, k] of "kn"
+    if case == "inf":
+        rows[3, 5], rows[1000, 77] = float("inf"), float("-inf")
+    elif case == "nan":
+        rows[130, 1], cols[7, 9] = float("nan"), float("nan")
+    elif case == "overflow":
+        rows[64:70] *= 3e37
+        cols[:9] *= 40.0
+    elif case == "tiny":
+        rows[200:300] *= 1e-17
+        cols[100:200] *= 1e-17
+    else:
+        rows[:150] *= 1e-40
+    res = []
+    for kernel in (0, DIRECT[dt]):
+        plan = tp.Plan(prob, tp.PlanConfig(kernel=kernel))
+        D.zero_()
+        plan.execute_into(ex, 1.0, A, B, D)
+        torch.cuda.synchronize()
+        res.append(torch.view_as_real(D).double() if dt.startswith("complex") else D.double())
+    x, y = res
+    assert torch.equal(torch.isnan(x), torch.isnan(y))
+    inf = torch.isinf(y)
+    assert torch.equal(torch.isinf(x), inf) and torch.equal(x[inf], y[inf])
+    wide = torch.complex128 if dt.startswith("complex") else torch.float64
+    mag = torch.einsum(form[0], A.abs().double(), B.abs().double())
+    if dt.startswith("complex"):
+        mag = mag.unsqueeze(-1).expand(x.shape)
+    # Each output within 60 roundings of the sum of its products' magnitudes.
+    ok = torch.isfinite(y) & torch.isfinite(mag)
+    assert bool(((x - y).abs()[ok] <= 60 * (2.0 ** -24 * mag[ok] + 2.0 ** -149)).all())
+    ex.close()
