@@ -566,23 +566,19 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
               }
             }
           } else {
-            // C of four columns is on its way before the first of it is used.
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+              // v[j] without a dynamic register index.
+              float y = v[0];
 #pragma unroll
-            for (int j0 = 0; j0 < 8; j0 += 4) {
-              T cv[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (!e.beta_zero && mok && !comp && 8 * q + j0 + j < nrem) cv[j] = Cb[cn_s[8 * q + j0 + j]];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int jj = 8 * q + j0 + j;
-                const float y = v[j0 + j], o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
-                if (jj >= nrem || !mok || comp) continue;
-                if (split_lost(thr, y) || (CPLX && split_lost(thr, o)))
-                  again |= (uint64_t)1 << jj;
-                else
-                  epilogue_store<float, CPLX>(e, y, o, &cv[j], Db + dn_s[jj]);
-              }
+              for (int i = 1; i < 8; ++i) y = j == i ? v[i] : y;
+              const int jj = 8 * q + j;
+              const float o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
+              if (jj >= nrem || !mok || comp) continue;
+              if (split_lost(thr, y) || (CPLX && split_lost(thr, o)))
+                again |= (uint64_t)1 << jj;
+              else
+                epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
             }
           }
           __syncwarp();
