@@ -36,9 +36,9 @@ struct Scatters {
 // D = op_D(alpha * acc + beta * op_C(C)); beta_zero means C is never read.
 struct Epilogue {
   double alpha_re, alpha_im, beta_re, beta_im;
-  int beta_zero;  // C not read
-  int plain;      // alpha == 1, beta == 0, no conj on D: store acc as is
-  int conj_c, conj_d;
+  int8_t beta_zero;  // C not read
+  int8_t plain;      // alpha == 1, beta == 0, no conj on D: store acc as is
+  int8_t conj_c, conj_d;
 };
 
 // Bits of the device status word an executor owns. A kernel that gives up on a
@@ -56,11 +56,11 @@ struct __align__(16) GemmArgs {
   const void* C;
   void* D;
   int64_t M, N, K, H;
-  int conj_a, conj_b;
-  int a_kfast, b_kfast, d_mfast;
+  int8_t conj_a, conj_b;
+  int8_t a_kfast, b_kfast, d_mfast;
   // Every 16-byte group of the operand's fast index is contiguous and aligned
   // (16-byte gathers).
-  int a_vec, b_vec;
+  int8_t a_vec, b_vec;
   // Non-zero: the operand is a dense panel [H][K][ld], rows fastest, and its
   // scatter vectors are not read (tensor-core stream tiles after a pack pass).
   int64_t a_ld, b_ld;
@@ -150,6 +150,9 @@ int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int 
 size_t stream_panel_bytes(int dtype, int64_t rows, int64_t K, int64_t H);
 cudaError_t launch_stream_pack(int dtype, GemmArgs& g, int which, int fast, void* panel, cudaStream_t st);
 static_assert(sizeof(GemmArgs) % 16 == 0, "grouped kernels copy GemmArgs in 16-byte words");
+// Kernel parameters: 304 bytes cost a launch 0.6 us more than 288 (host time of a small
+// call 8.9 us against 9.6 on the B200 machines).
+static_assert(sizeof(GemmArgs) <= 288, "launch cost");
 
 // One item of a grouped launch: its arguments and its tile grid.
 struct GroupItem {
