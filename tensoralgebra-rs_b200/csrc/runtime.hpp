@@ -89,7 +89,8 @@ struct Executor {
   size_t pool_size = 0, budget = 1;  // recorded for the pooled-executor extension
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  unsigned* status = nullptr;  // device word
+  unsigned* status = nullptr;  // status word as kernels address it
+  unsigned* status_host = nullptr;  // the same word (mapped host memory)
   int num_sms = 148;
   std::mutex mu;
   std::atomic<int> inflight{0};
