@@ -18,7 +18,7 @@
 //               matrices, no swizzle; the 16-byte step between depth groups keeps
 //               the stores free of bank conflicts).
 //   warp 24     issues tcgen05.mma: x0 y0 into a main accumulator, restarted every
-//               128 k and added up in FP32 registers, the five cross products into
+//               32 k (64 where that is all of K) and added up in FP32, the five cross products into
 //               a correction accumulator (the accumulate of the tensor core
 //               truncates; see k_split.cu).
 //
@@ -44,7 +44,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int TS_BM = 128, TS_BN = 128, TS_BK = 32, TS_STAGES = 4, TS_CK = 4;
+constexpr int TS_BM = 128, TS_BN = 128, TS_BK = 32, TS_STAGES = 4;
 constexpr int TS_LBO = TS_BM * 16 + 16;     // bytes between 8-deep groups of a plane
 constexpr int TS_PLANE = 4 * TS_LBO;        // 128 rows x 32 k
 constexpr int TS_STAGE = 6 * TS_PLANE;      // three planes of A', three of B'
@@ -384,11 +384,14 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
   // Tensor memory, 128 columns each: main 0, main 1, then the corrections of two
   // tiles, or (K of several chunks) one and the running sums.
   const uint32_t tmem = *tmem_slot;
-  const bool multi = nk > TS_CK;
+  // Blocks per restart of the leading sum (see the top of the file): two where that is
+  // all of K, so that the corrections of two tiles fit; else one.
+  const int ck = nk <= 2 ? 2 : 1;
+  const bool multi = nk > ck;
 
-  // Registers a thread: 56 x 256 + 88 x 512 + 40 x 128 = the 72 x 896 of the launch.
+  // Registers a thread: 64 x 256 + 80 x 512 + 40 x 128 = 62464 of the launch's 72 x 896.
   if (warp >= 8 && warp < 24) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     if ((warp & 7) < 4)
       ts_produce<CPLX, true>(g, ring, full, empty, stats, stat_full, stat_empty, tiles, tm, tn, warp - 8, lane);
     else
@@ -408,7 +411,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
         const uint32_t corr = tmem + 256 + 128 * cb;
         if (!ts_wait(&corr_empty[cb], ((uint32_t)(multi ? it : it >> 1) & 1u) ^ 1u)) ok = false;
         for (int kb = 0; ok && kb < nk; ++kb) {
-          const int in_chunk = kb % TS_CK;
+          const int in_chunk = kb % ck;
           if (!ts_wait(&full[stage], round & 1u) ||
               (in_chunk == 0 && !ts_wait(&main_empty[chunk & 1], ((chunk >> 1) & 1u) ^ 1u))) {
             ok = false;
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
             umma_bf16(mainacc, a[0], b[0], idesc, (in_chunk | kk) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
-          if (in_chunk == TS_CK - 1 || kb == nk - 1) {
+          if (in_chunk == ck - 1 || kb == nk - 1) {
             umma_commit(&main_full[chunk & 1]);
             ++chunk;
           }
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     }
     __syncwarp();
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const int col0 = (warp >> 2) * TS_CPT;
     int64_t* cols_w = cols + warp * 4 * TS_CPT;
     const uint32_t lane_addr = ((uint32_t)(32 * (warp & 3)) << 16) + col0;
@@ -488,7 +491,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       if (t + (int)gridDim.x < tiles) fetch(ts_tile<CPLX>(g, t + gridDim.x, tm, tn), (it + 1) & 1);
       const int cb = multi ? 0 : it & 1;
       const uint32_t corr = tmem + 256 + 128 * cb + lane_addr, total = tmem + 384 + lane_addr;
-      for (int kb = 0; kb + TS_CK < nk; kb += TS_CK, ++chunk) {
+      for (int kb = 0; kb + ck < nk; kb += ck, ++chunk) {
         if (!ts_wait(&main_full[chunk & 1], (chunk >> 1) & 1u)) {
           ok = false;
           break;
