@@ -18,8 +18,7 @@
 //   compute:  full[stage] -> fragments -> empty[stage]; after the last stage
 //             the epilogue from the slot, then slot_empty.
 //
-// Only the k of the last stage that exist are multiplied (k steps of four on
-// the DMMA pipe, single k on the FFMA pipe), so a short odd K costs no padded
+// Only the k of the last stage that exist are multiplied (in steps of four), so a short odd K costs no padded
 // depth. Every mbarrier wait is bounded by %globaltimer (a status bit, then the
 // role ends); the producer drains its own copies before it exits.
 #include "tc_common.cuh"
@@ -37,19 +36,9 @@ __device__ __forceinline__ void cpa8(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cpa8z(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
 }
-__device__ __forceinline__ void cpa4z(uint32_t dst, const void* src, bool ok) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
-}
 // 16-byte copy of `bytes` (0, a multiple of the element, or 16), the rest zero-filled.
 __device__ __forceinline__ void cpa16z(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-template <int ES>
-__device__ __forceinline__ void cpa_elem(uint32_t dst, const void* src, bool ok) {
-  if constexpr (ES == 4)
-    cpa4z(dst, src, ok);
-  else
-    cpa8z(dst, src, ok);
 }
 // The barrier's pending count drops by one when this thread's earlier cp.async
 // copies have landed.
@@ -60,7 +49,7 @@ __device__ __forceinline__ void cpa_drain() { asm volatile("cp.async.wait_all;" 
 
 // Shared-memory order of an operand's stage (16 deep):
 //   rows-fast operands: [k][row], row stride LD elements;
-//   k-fast f64 operands (SWZ): 128-byte rows of 16 k, the 16-byte chunk c of row
+//   k-fast operands: 128-byte rows of 16 k, the 16-byte chunk c of row
 //   r at chunk c xor (r mod 8) (the order TMA's SWIZZLE_128B gives the packed
 //   panels): a copy of 16 consecutive k of a row is one contiguous write, and the
 //   fragment reads (8 rows x 4 k) are free of bank conflicts.
@@ -69,11 +58,11 @@ __device__ __forceinline__ void cpa_drain() { asm volatile("cp.async.wait_all;" 
 // covers 32 rows of one k (rows fast) or 16 consecutive k of two rows (k fast),
 // so it touches two or three 128-byte lines; with `vec` (the host found every
 // offset a multiple of 16 bytes and the fast index contiguous) the copies are
-// 16 bytes wide and half (a quarter) as many. The row offsets of the tile stay
+// 16 bytes wide and half as many. The row offsets of the tile stay
 // in registers, one row per lane, and reach the lanes by shuffles, as the
 // stage's k offsets do. Rows past the operand's end are left as they are (their
 // products are never stored); k past the range are zero-filled.
-template <int ES, int ROWS, int LD, bool SWZ>
+template <int ES, int ROWS, int LD>
 struct StageGather {
   static constexpr int RREG = (ROWS + 31) / 32, V = 16 / ES;
   int64_t off[RREG];  // row lane + 32 j
@@ -86,38 +75,21 @@ struct StageGather {
       off[j] = __ldg(rows + r0 + (r < last ? r : last)) * ES;
     }
   }
-  __device__ __forceinline__ int64_t row_off(int r) const {  // r / 32 uniform and known at compile time
-    return __shfl_sync(0xffffffffu, off[RREG > 1 ? r / 32 : 0], r & 31);
-  }
-
   // kreg: lanes 0..15 (and 16..31 again) hold the stage's k offsets in bytes;
   // kv: k of the stage that exist; rv: rows of the tile that exist.
   __device__ __forceinline__ void issue(const char* base, uint32_t dst, int64_t kreg, int kv, int rv, int kfast,
                                         int vec, int lane) const {
     if (kfast) {
-      if constexpr (SWZ) {
-        if (vec) {
-          const int c = lane & 7, rl = lane >> 3;  // chunk of two k, row of four
-          const int64_t ko = __shfl_sync(0xffffffffu, kreg, 2 * c);
-          const char* p = base + ko;
-          const int sz = min(max(kv - 2 * c, 0), 2) * 8;
+      if (vec) {
+        const int c = lane & 7, rl = lane >> 3;  // chunk of two k, row of four
+        const int64_t ko = __shfl_sync(0xffffffffu, kreg, 2 * c);
+        const char* p = base + ko;
+        const int sz = min(max(kv - 2 * c, 0), 2) * 8;
 #pragma unroll
-          for (int j = 0; j < ROWS / 4; ++j) {
-            const int64_t ro = __shfl_sync(0xffffffffu, off[RREG > 1 ? j / 8 : 0], (4 * j + rl) & 31);
-            const int row = 4 * j + rl;
-            if (row < rv) cpa16z(dst + (uint32_t)(row * 128 + ((c ^ (row & 7)) << 4)), p + ro, sz);
-          }
-        } else {
-          const int kk = lane & 15, rl = lane >> 4;
-          const char* p = base + kreg;
-          const bool ok = kk < kv;
-#pragma unroll
-          for (int j = 0; j < ROWS / 2; ++j) {
-            const int64_t ro = __shfl_sync(0xffffffffu, off[RREG > 1 ? j / 16 : 0], (2 * j + rl) & 31);
-            const int row = 2 * j + rl;
-            if (row < rv)
-              cpa_elem<ES>(dst + (uint32_t)(row * 128 + ((((kk >> 1) ^ (row & 7)) << 4) | ((kk & 1) << 3))), p + ro, ok);
-          }
+        for (int j = 0; j < ROWS / 4; ++j) {
+          const int64_t ro = __shfl_sync(0xffffffffu, off[RREG > 1 ? j / 8 : 0], (4 * j + rl) & 31);
+          const int row = 4 * j + rl;
+          if (row < rv) cpa16z(dst + (uint32_t)(row * 128 + ((c ^ (row & 7)) << 4)), p + ro, sz);
         }
       } else {
         const int kk = lane & 15, rl = lane >> 4;
@@ -126,7 +98,9 @@ struct StageGather {
 #pragma unroll
         for (int j = 0; j < ROWS / 2; ++j) {
           const int64_t ro = __shfl_sync(0xffffffffu, off[RREG > 1 ? j / 16 : 0], (2 * j + rl) & 31);
-          if (2 * j + rl < rv) cpa_elem<ES>(dst + (uint32_t)(kk * LD + 2 * j + rl) * ES, p + ro, ok);
+          const int row = 2 * j + rl;
+          if (row < rv)
+            cpa8z(dst + (uint32_t)(row * 128 + ((((kk >> 1) ^ (row & 7)) << 4) | ((kk & 1) << 3))), p + ro, ok);
         }
       }
       return;
@@ -155,16 +129,6 @@ struct StageGather {
           if (sz > 0) cpa16z(d + (uint32_t)(k0 * LD) * ES, p + ko, kk < kv ? sz : 0);
         }
       }
-    } else if constexpr (ROWS < 32) {
-      constexpr int KP = 32 / ROWS;
-      const int64_t ro = __shfl_sync(0xffffffffu, off[0], lane % ROWS);
-#pragma unroll
-      for (int k0 = 0; k0 < 16; k0 += KP) {
-        const int kk = k0 + lane / ROWS;
-        const int64_t ko = __shfl_sync(0xffffffffu, kreg, kk);
-        if (lane < KP * ROWS && lane % ROWS < rv)
-          cpa_elem<ES>(dst + (uint32_t)(kk * LD + lane % ROWS) * ES, base + ko + ro, kk < kv);
-      }
     } else {
 #pragma unroll
       for (int kk = 0; kk < 16; ++kk) {
@@ -174,7 +138,7 @@ struct StageGather {
         const uint32_t d = dst + (uint32_t)(kk * LD + lane) * ES;
 #pragma unroll
         for (int j = 0; j < RREG; ++j)
-          if (lane + 32 * j < rv) cpa_elem<ES>(d + 32 * j * ES, p + off[j], ok);
+          if (lane + 32 * j < rv) cpa8z(d + 32 * j * ES, p + off[j], ok);
       }
     }
   }
@@ -208,7 +172,6 @@ struct __align__(16) TileSlot {
 template <int WGM, int WGN, int TI, int TJ, int STG, int MINB_>
 struct StreamF64 {
   using R = double;
-  static constexpr bool SWZ = true;
   static constexpr int ES = 8, WARPS = WGM * WGN, BM = WGM * TI * 16, BN = WGN * TJ * 8, BK = 16;
   // Row strides of 4 (mod 16) doubles: the fragment reads (8 rows x 4 k) are
   // free of bank conflicts.
@@ -461,8 +424,8 @@ stream_kernel(const __grid_constant__ GemmArgs gp, const GroupItem* __restrict__
       }
       const GemmArgs& g = GROUPED ? items[item].g : gp;
       int64_t kb = 0, kspan = 0, m0 = 0, n0 = 0;
-      StageGather<ES, BM, Op::SA, Op::SWZ> ga;
-      StageGather<ES, BN, Op::SB, Op::SWZ> gb;
+      StageGather<ES, BM, Op::SA> ga;
+      StageGather<ES, BN, Op::SB> gb;
       const int klane = lane & 15;
       int64_t ka = 0, kbr = 0, ha = 0, hb = 0;
       if (!end) {
