@@ -219,19 +219,20 @@ struct TsProducer {
     }
   }
 
-  // Splits one row's eight values into the planes; mx, mn: the largest and smallest
-  // non-zero leading halves (mn less one, zero as 0x7fff).
+  // Splits one row's eight values into the planes. mx: the largest leading halves; mn:
+  // the smallest non-zero magnitude as f32 bits, twice and less one (zero: the
+  // largest). From the f32 bits: values of 2^-134 and below are zero in every plane.
   __device__ __forceinline__ void row(const float (&v)[8], char* d, uint32_t flip, uint32_t& mx, uint32_t& mn) const {
     uint32_t w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float x = v[2 * j], y = v[2 * j + 1];
+      mn = min(mn, min(2 * __float_as_uint(x) - 1, 2 * __float_as_uint(y) - 1));
       w[0][j] = ts_split(x, y);
       w[1][j] = ts_split(x, y);
       w[2][j] = ts_split(x, y);
       const uint32_t a = w[0][j] & 0x7fff7fffu;
       asm("max.u16x2 %0, %0, %1;" : "+r"(mx) : "r"(a));
-      asm("min.s16x2 %0, %0, %1;" : "+r"(mn) : "r"(a + 0x7fff7fffu));
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
@@ -274,7 +275,7 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
   uint32_t block = (uint32_t)warp >> 3;  // the set's blocks: every other one of the CTA's sequence
   int t = blockIdx.x, reported = t;  // the block's tile; the first tile whose range is not reported
   int kb = 0, it = 0;
-  uint32_t mx = 0, mn = 0x7fff7fffu;
+  uint32_t mx = 0, mn = 0xffffffffu;
   bool act = false, ok = true;
   const auto advance = [&](int n) {
     kb += n;
@@ -303,14 +304,14 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
       const int s = it % TS_STATS;
       ok = __all_sync(0xffffffffu, ts_wait(&stat_empty[s], ((uint32_t)(it / TS_STATS) & 1u) ^ 1u));
       const int hi = (int)__reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
-      const int lo = __reduce_min_sync(0xffffffffu, min((int)(int16_t)(mn & 0xffffu), (int)(int16_t)(mn >> 16)));
+      const uint32_t lo = __reduce_min_sync(0xffffffffu, mn);
       if (lane == 0 && ok) {
-        stats[s * 16 + warp] = make_int2(hi, lo == 0x7fff ? 0x7fff : (lo - 0x7fff) & 0xffff);
+        stats[s * 16 + warp] = make_int2(hi, lo == 0xffffffffu ? 0x7fff : (int)((lo + 1) >> 17));
         mbar_arrive(&stat_full[s]);
       }
       __syncwarp();
       mx = 0;
-      mn = 0x7fff7fffu;
+      mn = 0xffffffffu;
     }
   };
   advance((int)block);
