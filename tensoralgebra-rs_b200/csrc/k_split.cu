@@ -331,7 +331,44 @@ __global__ void __launch_bounds__(128) split_guard_kernel(const uint2* __restric
   }
 }
 
-template <int S, int BN>
+// 32 lanes x 64 columns, and the wait tied to its registers.
+__device__ __forceinline__ void tmem_ld_x64(uint32_t taddr, uint32_t (&r)[64]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
+      "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+      "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), 
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), 
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), 
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), 
+        "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), 
+        "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), 
+        "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), 
+        "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_x64(uint32_t (&r)[64]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), 
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), 
+                 "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), 
+                 "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]), 
+                 "+r"(r[32]), "+r"(r[33]), "+r"(r[34]), "+r"(r[35]), "+r"(r[36]), "+r"(r[37]), "+r"(r[38]), "+r"(r[39]), 
+                 "+r"(r[40]), "+r"(r[41]), "+r"(r[42]), "+r"(r[43]), "+r"(r[44]), "+r"(r[45]), "+r"(r[46]), "+r"(r[47]), 
+                 "+r"(r[48]), "+r"(r[49]), "+r"(r[50]), "+r"(r[51]), "+r"(r[52]), "+r"(r[53]), "+r"(r[54]), "+r"(r[55]), 
+                 "+r"(r[56]), "+r"(r[57]), "+r"(r[58]), "+r"(r[59]), "+r"(r[60]), "+r"(r[61]), "+r"(r[62]), "+r"(r[63])::"memory");
+}
+
+__device__ __forceinline__ void add_pair(float& x, float& y, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\t"
+      "add.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+      : "+f"(x), "+f"(y)
+      : "r"(a), "r"(b));
+}
+
+template <int S, int BN, int PLAIN = 0>
 struct TcCfg {
   static constexpr int A_TILE = TC_BM * TC_BK * 2;  // bytes of one A plane tile
   static constexpr int B_TILE = BN * TC_BK * 2;
@@ -342,7 +379,9 @@ struct TcCfg {
   static constexpr int BAR = (2 * STAGES + 3) * 8 + 16;
   static constexpr int SMEM = 1024 + RING + SCAT + BAR;
   static constexpr int EPI_WARPS = 8;  // two per TMEM lane quarter, each half of the columns
-  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  // Plain: whole warpgroups, so that the drain warps can take the registers of the others.
+  static constexpr int EPI_FIRST = PLAIN ? 4 : 2;
+  static constexpr int THREADS = 32 * (EPI_FIRST + EPI_WARPS);
   static constexpr int COLS_PER_THREAD = BN / 2;
 };
 
@@ -362,12 +401,22 @@ struct TcCfg {
 // order and applies the epilogue.
 //
 // PLAIN 0: the split schemes; 1 and 2: plain f32 and c32, with the tiles' thresholds.
+// There the main accumulator restarts every 16-deep step: 16 16-bit products mostly add
+// up exactly, so values of one sign gather no bias from the truncation (x1 y2, x2 y1 and
+// x2 y2 are left out, up to 2^-24 of a product and 2^-26 typically; with all of them the
+// error is the same from K = 512 on). The cross terms of a step cover the drain of the
+// one before; the drain warps take the registers of the other roles and release the
+// accumulator before they add. The FP32 sums of 16 or 32 steps go to a second sum per
+// output (in local memory, an eighth of the columns at a time), so that the roundings
+// of a long K do not pile up. f32 4096^3 on B200: 626 us with restarts every 64 k and
+// one sum, 775 so (731 without the second sum); error on uniform [0, 1) 1.3e-7 -> 0.6e-7
+// (FFMA tiles 1.1e-7), on [-1, 1) 1.7e-7 -> 1.25e-7 (2.1e-7).
 template <int S, int BN, int CK, int PLAIN>
-__global__ void __launch_bounds__(TcCfg<S, BN>::THREADS, 1)
+__global__ void __launch_bounds__(TcCfg<S, BN, PLAIN>::THREADS, 1)
 tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g,
                     int64_t m_pad, int64_t n_pad, int64_t k_pad, int64_t whole, int parts, float* partial,
                     const float* __restrict__ thr_of) {
-  using Cfg = TcCfg<S, BN>;
+  using Cfg = TcCfg<S, BN, PLAIN>;
   constexpr int CPT = Cfg::COLS_PER_THREAD;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -415,8 +464,8 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tmem_alloc(tmem_slot, 2 * BN);
     tmem_relinquish();
   }
-  if (warp >= 2) {
-    for (int i = tid - 64; i < BN; i += 32 * Cfg::EPI_WARPS) {
+  if (warp >= Cfg::EPI_FIRST) {
+    for (int i = tid - 32 * Cfg::EPI_FIRST; i < BN; i += 32 * Cfg::EPI_WARPS) {
       const int64_t n = n0 + i;
       const bool ok = n < g.N;
       dn_s[i] = ok ? g.s.d_n[n] : 0;
@@ -429,78 +478,164 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const uint32_t tmem = *tmem_slot;
   const uint32_t tmem_main = tmem, tmem_corr = tmem + BN;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      for (int kb = 0; kb < nk; ++kb) {
-        const int st = kb % Cfg::STAGES;
-        const uint32_t round = (uint32_t)(kb / Cfg::STAGES);
-        if (!mbar_wait(&empty[st], (round & 1u) ^ 1u)) {
-          atomicOr(g.status, STATUS_WAIT_TIMEOUT);
-          break;
+  // Plain: registers a thread 40 x 128 + 232 x 256 = 64512 of the launch's 168 x 384.
+  if (warp < Cfg::EPI_FIRST) {
+    if constexpr (PLAIN != 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 0) {
+      if (lane == 0) {
+        for (int kb = 0; kb < nk; ++kb) {
+          const int st = kb % Cfg::STAGES;
+          const uint32_t round = (uint32_t)(kb / Cfg::STAGES);
+          if (!mbar_wait(&empty[st], (round & 1u) ^ 1u)) {
+            atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+            break;
+          }
+          mbar_arrive_expect_tx(&full[st], (uint32_t)Cfg::STAGE);
+          uint8_t* sbase = ring + st * Cfg::STAGE;
+          const int kx = (kb_lo + kb) * TC_BK;
+#pragma unroll
+          for (int p = 0; p < S; ++p)
+            tma_load_2d(sbase + p * Cfg::A_TILE, &tmA, &full[st], kx, (int)((p * g.H + h) * m_pad + m0));
+#pragma unroll
+          for (int p = 0; p < S; ++p)
+            tma_load_2d(sbase + S * Cfg::A_TILE + p * Cfg::B_TILE, &tmB, &full[st], kx,
+                        (int)((p * g.H + h) * n_pad + n0));
         }
-        mbar_arrive_expect_tx(&full[st], (uint32_t)Cfg::STAGE);
-        uint8_t* sbase = ring + st * Cfg::STAGE;
-        const int kx = (kb_lo + kb) * TC_BK;
-#pragma unroll
-        for (int p = 0; p < S; ++p)
-          tma_load_2d(sbase + p * Cfg::A_TILE, &tmA, &full[st], kx, (int)((p * g.H + h) * m_pad + m0));
-#pragma unroll
-        for (int p = 0; p < S; ++p)
-          tma_load_2d(sbase + S * Cfg::A_TILE + p * Cfg::B_TILE, &tmB, &full[st], kx,
-                      (int)((p * g.H + h) * n_pad + n0));
       }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t IDESC = idesc_bf16(TC_BM, BN);
-      bool ok = true;
-      for (int kb = 0; kb < nk && ok; ++kb) {
-        const int st = kb % Cfg::STAGES;
-        const uint32_t round = (uint32_t)(kb / Cfg::STAGES);
-        if (!mbar_wait(&full[st], round & 1u)) {
-          atomicOr(g.status, STATUS_WAIT_TIMEOUT);
-          break;
-        }
-        tc_fence_after();
-        const uint32_t sbase = smem_u32(ring + st * Cfg::STAGE);
-        // Cross terms first: they overlap the drain of the previous chunk.
+    } else if (warp == 1) {
+      if (lane == 0) {
+        constexpr uint32_t IDESC = idesc_bf16(TC_BM, BN);
+        bool ok = true;
+        for (int kb = 0; kb < nk && ok; ++kb) {
+          const int st = kb % Cfg::STAGES;
+          const uint32_t round = (uint32_t)(kb / Cfg::STAGES);
+          if (!mbar_wait(&full[st], round & 1u)) {
+            atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sbase = smem_u32(ring + st * Cfg::STAGE);
+          if constexpr (PLAIN != 0) {
 #pragma unroll
-        for (int p = 1; p < Pairs<S>::N; ++p) {
-          const uint64_t ad = sdesc_sw64(sbase + Pairs<S>::a(p) * Cfg::A_TILE);
-          const uint64_t bd = sdesc_sw64(sbase + S * Cfg::A_TILE + Pairs<S>::b(p) * Cfg::B_TILE);
+            for (int kk = 0; kk < 2; ++kk) {
+              uint64_t a[3], b[3];
 #pragma unroll
-          for (int kk = 0; kk < TC_BK / 16; ++kk)
-            umma_bf16(tmem_corr, ad + 2 * kk, bd + 2 * kk, IDESC, (kb | (p - 1) | kk) != 0 ? 1u : 0u);
-        }
-        const int chunk = kb / CK, in_chunk = kb % CK;
-        if (in_chunk == 0 && !mbar_wait(main_empty, ((uint32_t)chunk & 1u) ^ 1u)) {
-          atomicOr(g.status, STATUS_WAIT_TIMEOUT);
-          ok = false;
-        }
-        tc_fence_after();
-        {
-          const uint64_t ad = sdesc_sw64(sbase);
-          const uint64_t bd = sdesc_sw64(sbase + S * Cfg::A_TILE);
+              for (int p = 0; p < 3; ++p) {
+                a[p] = sdesc_sw64(sbase + p * Cfg::A_TILE) + 2 * kk;
+                b[p] = sdesc_sw64(sbase + S * Cfg::A_TILE + p * Cfg::B_TILE) + 2 * kk;
+              }
+              umma_bf16(tmem_corr, a[0], b[2], IDESC, (kb | kk) != 0 ? 1u : 0u);
+              umma_bf16(tmem_corr, a[2], b[0], IDESC, 1u);
+              umma_bf16(tmem_corr, a[1], b[1], IDESC, 1u);
+              umma_bf16(tmem_corr, a[0], b[1], IDESC, 1u);
+              umma_bf16(tmem_corr, a[1], b[0], IDESC, 1u);
+              if (!mbar_wait_polls(main_empty, (uint32_t)kk ^ 1u)) {
+                atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              umma_bf16(tmem_main, a[0], b[0], IDESC, 0u);
+              umma_commit(main_full);
+            }
+            umma_commit(&empty[st]);
+          } else {
+            // Cross terms first: they overlap the drain of the previous chunk.
 #pragma unroll
-          for (int kk = 0; kk < TC_BK / 16; ++kk)
-            umma_bf16(tmem_main, ad + 2 * kk, bd + 2 * kk, IDESC, (in_chunk | kk) != 0 ? 1u : 0u);
+            for (int p = 1; p < Pairs<S>::N; ++p) {
+              const uint64_t ad = sdesc_sw64(sbase + Pairs<S>::a(p) * Cfg::A_TILE);
+              const uint64_t bd = sdesc_sw64(sbase + S * Cfg::A_TILE + Pairs<S>::b(p) * Cfg::B_TILE);
+#pragma unroll
+              for (int kk = 0; kk < TC_BK / 16; ++kk)
+                umma_bf16(tmem_corr, ad + 2 * kk, bd + 2 * kk, IDESC, (kb | (p - 1) | kk) != 0 ? 1u : 0u);
+            }
+            const int chunk = kb / CK, in_chunk = kb % CK;
+            if (in_chunk == 0 && !mbar_wait(main_empty, ((uint32_t)chunk & 1u) ^ 1u)) {
+              atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+              ok = false;
+            }
+            tc_fence_after();
+            {
+              const uint64_t ad = sdesc_sw64(sbase);
+              const uint64_t bd = sdesc_sw64(sbase + S * Cfg::A_TILE);
+#pragma unroll
+              for (int kk = 0; kk < TC_BK / 16; ++kk)
+                umma_bf16(tmem_main, ad + 2 * kk, bd + 2 * kk, IDESC, (in_chunk | kk) != 0 ? 1u : 0u);
+            }
+            umma_commit(&empty[st]);
+            if (in_chunk == CK - 1 || kb == nk - 1) umma_commit(main_full);
+          }
         }
-        umma_commit(&empty[st]);
-        if (in_chunk == CK - 1 || kb == nk - 1) umma_commit(main_full);
+        if (PLAIN == 0 && !ok) umma_commit(main_full);
       }
-      if (!ok) umma_commit(main_full);
     }
   } else {
+    if constexpr (PLAIN != 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
     // Epilogue: warp w reads TMEM lanes 32*(w%4) .. +31 (tile rows) and half
     // of the columns; it keeps the running FP32 sum of its 128 outputs.
     const int lane_base = 32 * (warp & 3);
-    const int col0 = ((warp - 2) >> 2) * CPT;
+    const int col0 = ((warp - Cfg::EPI_FIRST) >> 2) * CPT;
     const uint32_t lane_addr = (uint32_t)lane_base << 16;
     float run[CPT];
 #pragma unroll
     for (int j = 0; j < CPT; ++j) run[j] = 0.f;
     bool ok = true;
-    for (int c = 0; c < nchunks; ++c) {
+    if constexpr (PLAIN != 0) {
+      constexpr int GROUPS = CPT / 16;
+      const int every = nk > 32 ? 4 : 2;  // steps per group of columns whose sums move
+      __align__(16) float kept[CPT];
+      float* sums = kept;
+      asm volatile("" : "+l"(sums));  // in local memory
+      for (int c = 0; c < 2 * nk; ++c) {
+        // The group whose sums move after this step, fetched ahead of the wait.
+        const int group = c % every == every - 1 ? c / every % GROUPS : -1;
+        float p[16];
+        if (group >= 0 && c >= every * GROUPS) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(p + j) = *reinterpret_cast<float4*>(sums + 16 * group + j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) p[j] = 0.f;
+        }
+        if (!mbar_wait_polls(main_full, (uint32_t)c & 1u)) {
+          atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < CPT / 64; ++q) {
+          uint32_t r[64];
+          tmem_ld_x64(tmem_main + lane_addr + (uint32_t)(col0 + 64 * q), r);
+          tmem_wait_x64(r);
+          if (q == CPT / 64 - 1) {  // read: the next step may fill it again
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(main_empty);
+          }
+#pragma unroll
+          for (int j = 0; j < 64; j += 2) add_pair(run[64 * q + j], run[64 * q + j + 1], r[j], r[j + 1]);
+        }
+#pragma unroll
+        for (int q = 0; q < GROUPS; ++q)
+          if (group == q) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+              *reinterpret_cast<float4*>(sums + 16 * q + j) =
+                  make_float4(p[j] + run[16 * q + j], p[j + 1] + run[16 * q + j + 1], p[j + 2] + run[16 * q + j + 2],
+                              p[j + 3] + run[16 * q + j + 3]);
+              run[16 * q + j] = run[16 * q + j + 1] = run[16 * q + j + 2] = run[16 * q + j + 3] = 0.f;
+            }
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < GROUPS; ++q)
+        if (2 * nk >= every * (q + 1)) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) run[16 * q + j] += sums[16 * q + j];
+        }
+    }
+    for (int c = 0; PLAIN == 0 && c < nchunks; ++c) {
       if (!mbar_wait(main_full, (uint32_t)c & 1u)) {
         atomicOr(g.status, STATUS_WAIT_TIMEOUT);
         ok = false;
@@ -535,7 +670,7 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     for (int q = 0; q < CPT / 16; ++q) {
       uint32_t r[16];
       tmem_ld_32x32b_x16(tmem_corr + lane_addr + (uint32_t)(col0 + 16 * q), r);
-      tmem_ld_wait();
+      tmem_ld_wait(r);
       if (part >= 0) {
         // Tail part: the raw FP32 sum, column-major in the tile (coalesced).
 #pragma unroll
@@ -671,7 +806,7 @@ constexpr int TC_PLAIN_SMS = 148;  // what the plain path's workspace is sized f
 template <int S, int BN, int CK, int PLAIN = 0>
 cudaError_t run_tc(const GemmArgs& g, const SplitLayout& L, const void* ap, const void* bp, float* tail_partial,
                    cudaStream_t st, const float* thr = nullptr) {
-  using Cfg = TcCfg<S, BN>;
+  using Cfg = TcCfg<S, BN, PLAIN>;
   CUtensorMap ma, mb;
   if (!make_map_2d(&ma, ap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, L.k_pad, (int64_t)S * L.H * L.m_pad, TC_BK, TC_BM))
     return cudaErrorInvalidValue;
@@ -823,13 +958,6 @@ cudaError_t launch_plain_split_gemm(int dtype, const GemmArgs& g, void* ws, cuda
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   float* tail = reinterpret_cast<float*>(w + S.tail);
-  // The leading sum restarts every 32 k: the tensor core truncates as it accumulates, a
-  // bias that values of one sign do not average out (K = 1024, uniform on [0, 1): 1.5e-7
-  // with 128 k, 0.6e-7 with 32 and in the FFMA tiles; 4096^3 605 against 632 us). Past
-  // 2048 the roundings of the restarts outweigh it, and 64 k are taken.
-  if (L.k_pad > 2048)
-    return dtype == 2 ? run_tc<3, 256, 2, 2>(g, L, w, w + S.b, tail, st, thr)
-                      : run_tc<3, 256, 2, 1>(g, L, w, w + S.b, tail, st, thr);
   return dtype == 2 ? run_tc<3, 256, 1, 2>(g, L, w, w + S.b, tail, st, thr)
                     : run_tc<3, 256, 1, 1>(g, L, w, w + S.b, tail, st, thr);
 }

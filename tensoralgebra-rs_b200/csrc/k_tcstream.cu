@@ -1,10 +1,9 @@
 // f32 and c32 contractions on the tensor cores without a pack pass.
 //
 // The FFMA pipe (72 TFLOP/s) bounds plain f32 tiles; BF16 products run 20 times
-// faster, and an f32 value is exactly the sum of three BF16 values (8 significant
-// bits each), so six BF16 products with FP32 accumulation carry a product to the
-// rounding of f32 (the terms left out are below 2^-26 of it; error against 64 bits
-// at K = 4096: 1.7e-7 against 2.1e-7 of the FFMA tiles, see k_split.cu). Packing the
+// faster, and an f32 value is exactly the sum of three BF16 values x0 + x1 + x2 (8
+// significant bits each; x1 up to 2^-8 and x2 up to 2^-17 of x). Eight of the nine
+// BF16 products are formed, all but x2 y2 (at most 2^-34 of the product). Packing the
 // planes through HBM costs 1.5 times the operand's bytes twice, which a short or
 // moderate K does not win back, so here the split happens on the way into shared
 // memory. One persistent CTA per SM, 128 x 128 tiles, 32-deep stages:
@@ -17,10 +16,18 @@
 //               stores the planes in the tensor core's order (K-major core
 //               matrices, no swizzle; the 16-byte step between depth groups keeps
 //               the stores free of bank conflicts).
-//   warp 24     issues tcgen05.mma: x0 y0 into a main accumulator, restarted every
-//               32 k (64 where that is all of K) and added up in FP32, the five cross products into
-//               a correction accumulator (the accumulate of the tensor core
-//               truncates; see k_split.cu).
+//   warp 24     issues tcgen05.mma, eight products per 16-deep step.
+//
+// Accumulation. The tensor core truncates each sum it forms, a bias that values of one
+// sign do not average out. So the leading products x0 y0 of a step, whose 16 16-bit
+// products mostly add up exactly, get an accumulator that starts from zero, and the
+// seven cross products (2^-8 of them) one of their own over all of K; the epilogue adds
+// the steps in FP32, two at a time, into a running sum that starts again every
+// TS_FLUSH blocks of 32. Relative error of 2048^2 f32 products on B200 (FFMA tiles ->
+// here), uniform on [-1, 1): K = 64 1.4e-7 -> 0.45e-7, K = 512 1.6e-7 -> 0.7e-7; uniform
+// on [0, 1): K = 64 1.15e-7 -> 0.5e-7, K = 512 0.61e-7 -> 0.56e-7; u^8 (one sign, heavy
+// tail, where the products of a step do not add up exactly): K = 16 0.59e-7 -> 0.75e-7,
+// K = 512 0.68e-7 -> 0.83e-7.
 //
 // c32 runs as the real product of 2M x N x 2K (rows 2m, 2m + 1 of A' hold [re, -im]
 // and [im, re], depths 2k, 2k + 1 of B' re and im): the embedding is a sign flip and
@@ -51,6 +58,7 @@ constexpr int TS_STAGE = 6 * TS_PLANE;      // three planes of A', three of B'
 constexpr int TS_THREADS = 896;
 constexpr int TS_CPT = TS_BN / 2;           // columns of an epilogue warp
 constexpr int TS_STATS = 4;                 // tiles whose value ranges are kept
+constexpr int TS_FLUSH = 8;                 // 32-deep blocks in a running sum
 
 struct TsSmem {
   static constexpr int RING = TS_STAGES * TS_STAGE;
@@ -80,17 +88,6 @@ __device__ __forceinline__ uint32_t ts_split(float& x, float& y) {
   return w;
 }
 
-// mbar_wait with the clock read only every 64 polls.
-__device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  for (;;) {
-#pragma unroll 1
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
-  }
-}
 __device__ __forceinline__ void ts_tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -302,7 +299,7 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
   const auto report = [&](int end) {
     for (; ok && reported < end; reported += gridDim.x, ++it) {
       const int s = it % TS_STATS;
-      ok = __all_sync(0xffffffffu, ts_wait(&stat_empty[s], ((uint32_t)(it / TS_STATS) & 1u) ^ 1u));
+      ok = __all_sync(0xffffffffu, mbar_wait_polls(&stat_empty[s], ((uint32_t)(it / TS_STATS) & 1u) ^ 1u));
       const int hi = (int)__reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
       const uint32_t lo = __reduce_min_sync(0xffffffffu, mn);
       if (lane == 0 && ok) {
@@ -320,7 +317,7 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
   while (t < tiles) {
     report(t);
     const uint32_t stage = block % TS_STAGES, round = block / TS_STAGES;
-    ok = ok && ts_wait(&empty[stage], (round & 1u) ^ 1u);
+    ok = ok && mbar_wait_polls(&empty[stage], (round & 1u) ^ 1u);
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) break;
     if (act) p.split(v, ring + stage * TS_STAGE + (IS_A ? 0 : 3 * TS_PLANE), mx, mn);
@@ -337,7 +334,8 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
   if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
 }
 
-template <bool CPLX>
+// STEPS: steps of 16 plane depths (one MMA each) in all of K: 1, 2 or (3) more.
+template <bool CPLX, int STEPS>
 __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_constant__ GemmArgs g, int tiles, int tm,
                                                                   int tn) {
   using T = typename Elem<float, CPLX>::type;
@@ -382,13 +380,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // Tensor memory, 128 columns each: main 0, main 1, then the corrections of two
-  // tiles, or (K of several chunks) one and the running sums.
+  // Tensor memory, 128 columns each, per STEPS. 1: two sets of the leading products and
+  // the cross products. 2: the leading products of either step, and the cross products
+  // of two tiles. 3: those of a block's steps, the cross products, the running sum.
+  constexpr bool MULTI = STEPS == 3;
+  const int steps_all = (int)((g.K * (CPLX ? 2 : 1) + 15) / 16);
   const uint32_t tmem = *tmem_slot;
-  // Blocks per restart of the leading sum (see the top of the file): two where that is
-  // all of K, so that the corrections of two tiles fit; else one.
-  const int ck = nk <= 2 ? 2 : 1;
-  const bool multi = nk > ck;
 
   // Registers a thread: 64 x 256 + 80 x 512 + 40 x 128 = 62464 of the launch's 72 x 896.
   if (warp >= 8 && warp < 24) {
@@ -401,28 +398,26 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 24 && lane == 0) {
       int stage = 0;
-      uint32_t round = 0, chunk = 0;
+      uint32_t round = 0, blocks = 0;
       bool ok = true;
       int it = 0;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++it) {
         const TsTile x = ts_tile<CPLX>(g, t, tm, tn);
         const int n = min(TS_BN, ((int)g.N - x.n0 + 15) / 16 * 16);
         const uint32_t idesc = ts_idesc(n);
-        const int cb = multi ? 0 : it & 1;
-        const uint32_t corr = tmem + 256 + 128 * cb;
-        if (!ts_wait(&corr_empty[cb], ((uint32_t)(multi ? it : it >> 1) & 1u) ^ 1u)) ok = false;
-        for (int kb = 0; ok && kb < nk; ++kb) {
-          const int in_chunk = kb % ck;
-          if (!ts_wait(&full[stage], round & 1u) ||
-              (in_chunk == 0 && !ts_wait(&main_empty[chunk & 1], ((chunk >> 1) & 1u) ^ 1u))) {
+        const int set = MULTI ? 0 : it & 1, mset = STEPS == 1 ? set : 0;
+        const uint32_t main0 = tmem + 256 * mset, main1 = main0 + 128,
+                       corr = STEPS == 1 ? main1 : tmem + 256 + 128 * set;
+        const uint32_t tile_turn = (uint32_t)(MULTI ? it : it >> 1);
+        if (!mbar_wait_polls(&corr_empty[set], (tile_turn & 1u) ^ 1u)) ok = false;
+        for (int kb = 0; ok && kb < nk; ++kb, ++blocks) {
+          if (!mbar_wait_polls(&full[stage], round & 1u)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(ring + stage * TS_STAGE), sb = sa + 3 * TS_PLANE;
-          const int left = ((int)g.K - kb * EK) * (CPLX ? 2 : 1);
-          const int steps = left > 16 ? 2 : 1;
-          const uint32_t mainacc = tmem + 128 * (chunk & 1);
+          const int steps = min(2, steps_all - 2 * kb);
           for (int kk = 0; kk < steps; ++kk) {
             uint64_t a[3], b[3];
 #pragma unroll
@@ -430,18 +425,24 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
               a[p] = ts_desc(sa + p * TS_PLANE + 2 * kk * TS_LBO);
               b[p] = ts_desc(sb + p * TS_PLANE + 2 * kk * TS_LBO);
             }
-            umma_bf16(corr, a[0], b[2], idesc, (kb | kk) != 0 ? 1u : 0u);
-            umma_bf16(corr, a[1], b[1], idesc, 1u);
+            umma_bf16(corr, a[1], b[2], idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_bf16(corr, a[2], b[1], idesc, 1u);
+            umma_bf16(corr, a[0], b[2], idesc, 1u);
             umma_bf16(corr, a[2], b[0], idesc, 1u);
+            umma_bf16(corr, a[1], b[1], idesc, 1u);
             umma_bf16(corr, a[0], b[1], idesc, 1u);
             umma_bf16(corr, a[1], b[0], idesc, 1u);
-            umma_bf16(mainacc, a[0], b[0], idesc, (in_chunk | kk) != 0 ? 1u : 0u);
           }
+          // The leading products of the block before have been read.
+          if (!mbar_wait_polls(&main_empty[mset], ((STEPS == 1 ? tile_turn : blocks) & 1u) ^ 1u)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          umma_bf16(main0, ts_desc(sa), ts_desc(sb), idesc, 0u);
+          if (steps == 2) umma_bf16(main1, ts_desc(sa + 2 * TS_LBO), ts_desc(sb + 2 * TS_LBO), idesc, 0u);
           umma_commit(&empty[stage]);
-          if (in_chunk == ck - 1 || kb == nk - 1) {
-            umma_commit(&main_full[chunk & 1]);
-            ++chunk;
-          }
+          umma_commit(&main_full[mset]);
           if (++stage == TS_STAGES) {
             stage = 0;
             ++round;
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
       // Nothing of this CTA's tensor work is in flight when it ends.
       umma_commit(done);
-      if (!ts_wait(done, 0)) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+      if (!mbar_wait_polls(done, 0)) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
     }
     __syncwarp();
   } else {
@@ -461,9 +462,10 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     const uint32_t lane_addr = ((uint32_t)(32 * (warp & 3)) << 16) + col0;
     const int prow = 32 * (warp & 3) + lane, comp = CPLX ? prow & 1 : 0;
     const Epilogue e = g.e;
-    uint32_t chunk = 0;
+    uint32_t blocks = 0;
     int it = 0;
     bool ok = true;
+    float sums[MULTI ? TS_CPT : 1];  // of TS_FLUSH blocks each
     // Output offsets of a tile, fetched while the one before it is written back.
     int64_t nd = 0, nc = 0;
     const auto fetch = [&](const TsTile& x, int buf) {
@@ -490,40 +492,46 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
       if (t + (int)gridDim.x < tiles) fetch(ts_tile<CPLX>(g, t + gridDim.x, tm, tn), (it + 1) & 1);
-      const int cb = multi ? 0 : it & 1;
-      const uint32_t corr = tmem + 256 + 128 * cb + lane_addr, total = tmem + 384 + lane_addr;
-      for (int kb = 0; kb + ck < nk; kb += ck, ++chunk) {
-        if (!ts_wait(&main_full[chunk & 1], (chunk >> 1) & 1u)) {
+      const int set = MULTI ? 0 : it & 1, mset = STEPS == 1 ? set : 0;
+      const uint32_t main0 = tmem + 256 * mset + lane_addr, main1 = main0 + 128,
+                     corr = STEPS == 1 ? main1 : tmem + 256 + 128 * set + lane_addr, total = tmem + 384 + lane_addr;
+      // All blocks but the last into the running sum, which starts again every
+      // TS_FLUSH blocks, so that the roundings of a long K do not pile up.
+      for (int kb = 0; MULTI && kb + 1 < nk; ++kb, ++blocks) {
+        if (!mbar_wait_polls(&main_full[0], blocks & 1u)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t acc = tmem + 128 * (chunk & 1) + lane_addr;
+        const bool first = kb % TS_FLUSH == 0, last = kb % TS_FLUSH == TS_FLUSH - 1;
 #pragma unroll 1
         for (int q = 0; 8 * q < nrem; ++q) {
-          uint32_t r[8];
-          ts_tmem_ld(acc + 8 * q, r);
-          if (kb) {
-            uint32_t u[8];
-            ts_tmem_ld(total + 8 * q, u);
-            tmem_ld_wait();
+          uint32_t r[8], u[8], w[8];
+          ts_tmem_ld(main0 + 8 * q, r);
+          ts_tmem_ld(main1 + 8 * q, u);
+          ts_tmem_ld(total + 8 * q, w);
+          tmem_ld_wait(r, u, w);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(r[j]));
+          for (int j = 0; j < 8; ++j)
+            r[j] = __float_as_uint((first ? 0.f : __uint_as_float(w[j])) + (__uint_as_float(r[j]) + __uint_as_float(u[j])));
+          if (last) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              sums[8 * q + j] = (kb == TS_FLUSH - 1 ? 0.f : sums[8 * q + j]) + __uint_as_float(r[j]);
           } else {
-            tmem_ld_wait();
+            ts_tmem_st(total + 8 * q, r);
           }
-          ts_tmem_st(total + 8 * q, r);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&main_empty[chunk & 1]);
+        if (lane == 0) mbar_arrive(&main_empty[0]);
       }
-      // The last chunk's commit covers the cross products; then the value ranges
+      // The last block, whose commit covers the cross products; then the value ranges
       // of the tile's operands.
       const int s = it % TS_STATS;
-      if (ok) ok = ts_wait(&main_full[chunk & 1], (chunk >> 1) & 1u);
-      if (ok) ok = ts_wait(&stat_full[s], (uint32_t)(it / TS_STATS) & 1u);
+      if (ok) ok = mbar_wait_polls(&main_full[mset], (STEPS == 1 ? (uint32_t)(it >> 1) : blocks) & 1u);
+      if (ok) ok = mbar_wait_polls(&stat_full[s], (uint32_t)(it / TS_STATS) & 1u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -540,25 +548,43 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
                                     bmin == 0x7fff ? 999 : (bmin >> 7) - 127);
       const bool guard = thr != 0.f;
       uint64_t again = 0;
-      const uint32_t acc = tmem + 128 * (chunk & 1) + lane_addr;
+      const bool second = steps_all % 2 == 0, more = (nk - 1) % TS_FLUSH != 0, flushed = nk > TS_FLUSH;
 #pragma unroll 1
       for (int q = 0; 8 * q < nrem; ++q) {
         {
-          uint32_t r[8], c[8];
-          ts_tmem_ld(acc + 8 * q, r);
-          ts_tmem_ld(corr + 8 * q, c);
-          tmem_ld_wait();
+          uint32_t r[8], u[8];
           float v[8];
+          ts_tmem_ld(main0 + 8 * q, r);
+          ts_tmem_ld(main1 + 8 * q, u);  // STEPS 1: the cross products
+          if constexpr (MULTI) {
+            uint32_t w[8];
+            ts_tmem_ld(total + 8 * q, w);
+            tmem_ld_wait(r, u, w);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
-          if (multi) {
-            ts_tmem_ld(total + 8 * q, r);
-            tmem_ld_wait();
+            for (int j = 0; j < 8; ++j)
+              v[j] = __uint_as_float(r[j]) + (second ? __uint_as_float(u[j]) : 0.f) + (more ? __uint_as_float(w[j]) : 0.f);
+            ts_tmem_ld(corr + 8 * q, u);
+            if (flushed) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]) + v[j];
+              for (int j = 0; j < 8; ++j) v[j] += sums[8 * q + j];
+            }
+            tmem_ld_wait(u);
+          } else if constexpr (STEPS == 2) {
+            uint32_t w[8];
+            ts_tmem_ld(corr + 8 * q, w);
+            tmem_ld_wait(r, u, w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              v[j] = __uint_as_float(r[j]) + __uint_as_float(u[j]);
+              u[j] = w[j];
+            }
+          } else {
+            tmem_ld_wait(r, u);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(c[j]);
+          for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(u[j]);
           if (!guard && e.plain && 8 * q + 8 <= nrem) {
             float* Df = reinterpret_cast<float*>(Db) + comp;
             if (mok) {
@@ -591,11 +617,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&main_empty[chunk & 1]);
-        mbar_arrive(&corr_empty[cb]);
+        mbar_arrive(&main_empty[mset]);
+        mbar_arrive(&corr_empty[set]);
         mbar_arrive(&stat_empty[s]);
       }
-      ++chunk;
+      ++blocks;
       for (; again; again &= again - 1) {
         const int j = __ffsll((long long)again) - 1;
         const float2 r = ffma_dot<CPLX>(g, x.h, m, n0 + j);
@@ -753,7 +779,11 @@ cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-  auto kern = dtype == 2 ? tc_stream_kernel<true> : tc_stream_kernel<false>;
+  const int64_t steps = (g.K * (dtype == 2 ? 2 : 1) + 15) / 16;
+  auto kern = dtype == 2 ? (steps == 1 ? tc_stream_kernel<true, 1> : steps == 2 ? tc_stream_kernel<true, 2>
+                                                                                : tc_stream_kernel<true, 3>)
+                         : (steps == 1 ? tc_stream_kernel<false, 1> : steps == 2 ? tc_stream_kernel<false, 2>
+                                                                                 : tc_stream_kernel<false, 3>);
   const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TsSmem::BYTES);
   if (r != cudaSuccess) return r;
   kern<<<grid, TS_THREADS, TsSmem::BYTES, st>>>(g, (int)tiles, (int)tm, (int)tn);
