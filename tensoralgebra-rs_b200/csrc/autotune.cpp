@@ -169,7 +169,8 @@ size_t tc_scratch(int kernel, const Product& p, int64_t M, int64_t N) {
   const int dt = (int)p.problem.dtype;
   if (dev::is_tc_split(kernel)) return dev::plain_split_bytes(dt, M, N, p.view.K, p.view.H) + 256;
   if (!dev::is_tc_stream(kernel)) return 0;
-  return (p.hints.a_gather ? 0 : dev::stream_panel_bytes(dt, M, p.view.K, p.view.H) + 256) +
+  return dev::tc_stream_flag_bytes(dt, M, N, p.view.H) + 256 +
+         (p.hints.a_gather ? 0 : dev::stream_panel_bytes(dt, M, p.view.K, p.view.H) + 256) +
          (p.hints.b_gather ? 0 : dev::stream_panel_bytes(dt, N, p.view.K, p.view.H) + 256);
 }
 

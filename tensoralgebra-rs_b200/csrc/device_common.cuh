@@ -81,43 +81,17 @@ __device__ inline void epilogue_store(const Epilogue& e, R acc_re, R acc_im, con
 
 // ---- f32 as sums of BF16 planes: values that they cannot carry --------------
 //
-// One output from the operands: FP32 sums restarted every 16 k, as the direct tiles.
-template <bool CPLX>
-__device__ __forceinline__ float2 ffma_dot(const GemmArgs& g, int64_t h, int64_t m, int64_t n) {
-  using T = typename Elem<float, CPLX>::type;
-  const T* A = static_cast<const T*>(g.A) + (g.a_ld ? h * g.K * g.a_ld + m : g.s.h_a[h] + g.s.a_m[m]);
-  const T* B = static_cast<const T*>(g.B) + (g.b_ld ? h * g.K * g.b_ld + n : g.s.h_b[h] + g.s.b_n[n]);
-  float tr = 0.f, ti = 0.f;
-  for (int64_t k0 = 0; k0 < g.K; k0 += 16) {
-    float cr = 0.f, ci = 0.f;
-    for (int64_t k = k0; k < g.K && k < k0 + 16; ++k) {
-      float ar, ai, br, bi;
-      Elem<float, CPLX>::load(A + (g.a_ld ? k * g.a_ld : g.s.a_k[k]), ar, ai);
-      Elem<float, CPLX>::load(B + (g.b_ld ? k * g.b_ld : g.s.b_k[k]), br, bi);
-      cr = fmaf(ar, br, cr);
-      if (CPLX) {
-        if (g.conj_a) ai = -ai;
-        if (g.conj_b) bi = -bi;
-        cr = fmaf(-ai, bi, cr);
-        ci = fmaf(ar, bi, ci);
-        ci = fmaf(ai, br, ci);
-      }
-    }
-    tr += cr;
-    ti += ci;
-  }
-  return make_float2(tr, ti);
-}
-
 // From the largest (ea, eb) and the smallest non-zero (la, lb; 999: none) exponents
 // of a tile's operands: the magnitude below which an output of the split products may
 // differ from f32 arithmetic's. 0: none; infinity: every output, for an infinity, a
-// NaN, a leading plane that rounds to infinity or products near overflow. With
+// NaN, a leading plane that rounds to infinity or a sum of `k` products that could
+// overflow. With
 // products down to 2^-100 and elements down to 2^-100 every plane and every kept
 // product is a normal number; below that, up to 2^-126 times the other operand is
 // lost per product, which 2^46 times as much leaves below f32 rounding.
-__device__ __forceinline__ float split_guard(int ea, int la, int eb, int lb) {
-  if (ea >= 127 || eb >= 127 || ea + eb > 100) return __uint_as_float(0x7f800000u);
+__device__ __forceinline__ float split_guard(int ea, int la, int eb, int lb, int k) {
+  // |x| < 2^(ea + 1), so the sum is below 2^(ea + eb + 2 + 32 - clz(k)).
+  if (ea >= 127 || eb >= 127 || ea + eb + 34 - __clz(k) > 126) return __uint_as_float(0x7f800000u);
   if (la == 999 || lb == 999 || (la + lb >= -100 && la >= -100 && lb >= -100)) return 0.f;
   const int e = ea > eb ? ea : eb;
   return __uint_as_float((uint32_t)(127 - 80 + (e + 1 > 0 ? e + 1 : 0)) << 23);

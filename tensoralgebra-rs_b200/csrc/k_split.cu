@@ -268,31 +268,12 @@ struct Pairs<3> {
   __device__ static inline int b(int p) { return p == 0 ? 0 : (p == 1 ? 1 : (p == 2 ? 0 : (p == 3 ? 2 : (p == 4 ? 1 : 0)))); }
 };
 
-// Tile order: within a batch entry, tiles go in groups of TILE_GROUP_M m-tiles
-// (the last group may be narrower); inside a group the m-tile is fastest, then
-// the n-tile. A wave of 148 CTAs then covers a block of about 16 A row panels
-// by 9 B column panels instead of 9 row panels by every column panel, so the
-// B planes a wave reads stay in L2 for the next wave of the same group.
-constexpr int TILE_GROUP_M = 16;
-
-__host__ __device__ inline void tile_coords(int64_t tile, int64_t tiles_m, int64_t tiles_n, int64_t& h, int64_t& mt,
-                                            int64_t& nt) {
-  const int64_t per_h = tiles_m * tiles_n;
-  h = tile / per_h;
-  const int64_t t = tile % per_h;
-  const int64_t group = t / (TILE_GROUP_M * tiles_n);
-  const int64_t first_m = group * TILE_GROUP_M;
-  const int64_t gm = tiles_m - first_m < TILE_GROUP_M ? tiles_m - first_m : TILE_GROUP_M;
-  const int64_t local = t - group * TILE_GROUP_M * tiles_n;
-  mt = first_m + local % gm;
-  nt = local / gm;
-}
-
 // split_guard of every tile from the pack's ranges: arb, brb pack rows of a tile of
 // an_rb, bn_rb in all, nkb depth blocks.
 __global__ void __launch_bounds__(128) split_guard_kernel(const uint2* __restrict__ sa, const uint2* __restrict__ sb,
                                                           int64_t tiles_m, int64_t tiles_n, int64_t an_rb, int64_t bn_rb,
-                                                          int arb, int brb, int nkb, float* __restrict__ thr) {
+                                                          int arb, int brb, int nkb, int k, int plain, float* __restrict__ thr,
+                                                          unsigned char* __restrict__ flags) {
   int64_t h, mt, nt;
   tile_coords(blockIdx.x, tiles_m, tiles_n, h, mt, nt);
   uint32_t m[2] = {0, 0}, l[2] = {0xffffffffu, 0xffffffffu};
@@ -327,7 +308,12 @@ __global__ void __launch_bounds__(128) split_guard_kernel(const uint2* __restric
         l[q] = min(l[q], part[w][2 + q]);
       }
     const auto low = [](uint32_t x) { return x == 0xffffffffu ? 999 : (int)((x + 1) >> 23) - 127; };
-    thr[blockIdx.x] = split_guard((int)(m[0] >> 23) - 127, low(l[0]), (int)(m[1] >> 23) - 127, low(l[1]));
+    const float t = split_guard((int)(m[0] >> 23) - 127, low(l[0]), (int)(m[1] >> 23) - 127, low(l[1]), k);
+    // Infinity: the whole tile is computed again; so is one with a threshold where D is
+    // not only written.
+    const bool whole = t == __uint_as_float(0x7f800000u) || (t != 0.f && !plain);
+    thr[blockIdx.x] = whole ? __uint_as_float(0x7f800000u) : t;
+    flags[blockIdx.x] = whole ? 0xff : 0;
   }
 }
 
@@ -415,7 +401,7 @@ template <int S, int BN, int CK, int PLAIN>
 __global__ void __launch_bounds__(TcCfg<S, BN, PLAIN>::THREADS, 1)
 tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g,
                     int64_t m_pad, int64_t n_pad, int64_t k_pad, int64_t whole, int parts, float* partial,
-                    const float* __restrict__ thr_of) {
+                    const float* __restrict__ thr_of, unsigned char* __restrict__ flags) {
   using Cfg = TcCfg<S, BN, PLAIN>;
   constexpr int CPT = Cfg::COLS_PER_THREAD;
   extern __shared__ uint8_t smem_raw[];
@@ -446,7 +432,10 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   int64_t h, mt, nt;
   tile_coords(tile, tiles_m, tiles_n, h, mt, nt);
   const int64_t m0 = mt * TC_BM, n0 = nt * BN;
-  const int nk = kb_hi - kb_lo;  // k-blocks of this CTA (>= 1)
+  // Sums below thr may have lost bits; infinity: the tile is computed by FFMA (k_again.cu).
+  const float thr = PLAIN ? thr_of[tile] : 0.f;
+  const bool whole_tile = PLAIN != 0 && thr == __uint_as_float(0x7f800000u);
+  const int nk = whole_tile ? 0 : kb_hi - kb_lo;  // k-blocks of this CTA
   const int nchunks = (nk + CK - 1) / CK;
 
   if (warp == 0 && lane == 0) {
@@ -661,13 +650,12 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     using T = typename Elem<float, CPLX>::type;
     const T* Cb = static_cast<const T*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h]) + cm;
     T* Db = static_cast<T*>(g.D) + g.s.h_d[h] + dm;
-    const float thr = PLAIN ? thr_of[tile] : 0.f;
-    uint32_t again[CPT / 32] = {};
+    float least = __uint_as_float(0x7f800000u);  // magnitude of what this lane writes
     float* Pb = part >= 0 ? partial + ((tile - whole) * parts + part) * (int64_t)(TC_BM * BN) + lane_base + lane
                           : nullptr;
     // The last main_full commit also covers every cross-term MMA.
 #pragma unroll
-    for (int q = 0; q < CPT / 16; ++q) {
+    for (int q = 0; q < (whole_tile ? 0 : CPT / 16); ++q) {
       uint32_t r[16];
       tmem_ld_32x32b_x16(tmem_corr + lane_addr + (uint32_t)(col0 + 16 * q), r);
       tmem_ld_wait(r);
@@ -678,7 +666,12 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       } else if constexpr (PLAIN != 0) {
         const int comp = CPLX ? lane & 1 : 0;
         constexpr int CG = CPLX ? 4 : 8;
-        if (thr == 0.f && g.e.plain) {
+        if (thr != 0.f) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (n0 + col0 + 16 * q + j < g.N) least = fminf(least, fabsf(run[16 * q + j] + __uint_as_float(r[j])));
+        }
+        if (g.e.plain) {
           if (mok) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -703,11 +696,7 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int jj = 16 * q + j0 + j, nn = col0 + jj;
             const float v = run[jj] + __uint_as_float(r[j0 + j]);
             const float o = CPLX ? __shfl_xor_sync(0xffffffffu, v, 1) : 0.f;
-            if (!mok || n0 + nn >= g.N || comp) continue;
-            if (split_lost(thr, v) || (CPLX && split_lost(thr, o)))
-              again[jj / 32] |= 1u << (jj % 32);
-            else
-              epilogue_store<float, CPLX>(g.e, v, o, &cv[j], Db + dn_s[nn]);
+            if (mok && n0 + nn < g.N && !comp) epilogue_store<float, CPLX>(g.e, v, o, &cv[j], Db + dn_s[nn]);
           }
         }
       } else if (mok) {
@@ -720,15 +709,8 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
     }
-    if constexpr (PLAIN != 0) {
-#pragma unroll
-      for (int w = 0; w < CPT / 32; ++w)
-        for (uint32_t bits = again[w]; bits; bits &= bits - 1) {
-          const int nn = col0 + 32 * w + __ffs(bits) - 1;
-          const float2 v = ffma_dot<CPLX>(g, h, m, n0 + nn);
-          epilogue_store<float, CPLX>(g.e, v.x, v.y, Cb + cn_s[nn], Db + dn_s[nn]);
-        }
-    }
+    if (PLAIN != 0 && part < 0 && thr != 0.f && __any_sync(0xffffffffu, mok && !(least >= thr)) && lane == 0)
+      mark_again(flags, tile, warp - Cfg::EPI_FIRST);
   }
 
   tc_fence_before();
@@ -740,11 +722,35 @@ tc_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // Tail tiles: add the parts in order, then the epilogue through the scatter.
-template <int BN, int PLAIN>
+template <int BN>
 __global__ void __launch_bounds__(256) split_tail_reduce_kernel(GemmArgs g, const float* __restrict__ partial,
                                                                 int64_t whole, int parts, int64_t tail, int64_t m_pad,
-                                                                int64_t n_pad, const float* __restrict__ thr_of) {
-  constexpr bool CPLX = PLAIN == 2;
+                                                                int64_t n_pad) {
+  const int64_t tiles_n = n_pad / BN, tiles_m = m_pad / TC_BM;
+  const int64_t total = tail * TC_BM * BN;
+  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = idx / (TC_BM * BN), within = idx % (TC_BM * BN);
+    const int row = (int)(within % TC_BM), col = (int)(within / TC_BM);
+    const int64_t tile = whole + t;
+    int64_t h, mt, nt;
+    tile_coords(tile, tiles_m, tiles_n, h, mt, nt);
+    const int64_t m = mt * TC_BM + row, n = nt * BN + col;
+    if (m >= g.M || n >= g.N) continue;
+    float v = 0.f;
+    for (int p = 0; p < parts; ++p) v += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within];
+    const float* c = static_cast<const float*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h] + g.s.c_m[m] + g.s.c_n[n]);
+    float* d = static_cast<float*>(g.D) + g.s.h_d[h] + g.s.d_m[m] + g.s.d_n[n];
+    epilogue_store<float, false>(g.e, v, 0.f, c, d);
+  }
+}
+
+// The same for plain f32 and c32, whose sums below the tile's threshold are marked.
+template <int BN, bool CPLX>
+__global__ void __launch_bounds__(256) plain_tail_reduce_kernel(GemmArgs g, const float* __restrict__ partial,
+                                                                int64_t whole, int parts, int64_t tail, int64_t m_pad,
+                                                                int64_t n_pad, const float* __restrict__ thr_of,
+                                                                unsigned char* __restrict__ flags) {
   using T = typename Elem<float, CPLX>::type;
   const int64_t tiles_n = n_pad / BN, tiles_m = m_pad / TC_BM;
   const int64_t total = tail * TC_BM * BN;
@@ -757,16 +763,14 @@ __global__ void __launch_bounds__(256) split_tail_reduce_kernel(GemmArgs g, cons
     tile_coords(tile, tiles_m, tiles_n, h, mt, nt);
     const int64_t m = CPLX ? (mt * TC_BM + row) >> 1 : mt * TC_BM + row, n = nt * BN + col;
     if (m >= g.M || n >= g.N || (CPLX && (row & 1))) continue;
+    const float thr = thr_of[tile];
+    if (thr == __uint_as_float(0x7f800000u)) continue;
     float v = 0.f, o = 0.f;
     for (int p = 0; p < parts; ++p) {
       v += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within];
       if (CPLX) o += partial[(t * parts + p) * (int64_t)(TC_BM * BN) + within + 1];
     }
-    if (PLAIN && (split_lost(thr_of[tile], v) || (CPLX && split_lost(thr_of[tile], o)))) {
-      const float2 x = ffma_dot<CPLX>(g, h, m, n);
-      v = x.x;
-      o = x.y;
-    }
+    if (thr != 0.f && !(fabsf(v) >= thr && (!CPLX || fabsf(o) >= thr))) mark_again(flags, tile, row / 32 + 4 * (col / (BN / 2)));
     const T* c = static_cast<const T*>(g.C) + (g.e.beta_zero ? 0 : g.s.h_c[h] + g.s.c_m[m] + g.s.c_n[n]);
     T* d = static_cast<T*>(g.D) + g.s.h_d[h] + g.s.d_m[m] + g.s.d_n[n];
     epilogue_store<float, CPLX>(g.e, v, o, c, d);
@@ -805,7 +809,7 @@ constexpr int TC_PLAIN_SMS = 148;  // what the plain path's workspace is sized f
 
 template <int S, int BN, int CK, int PLAIN = 0>
 cudaError_t run_tc(const GemmArgs& g, const SplitLayout& L, const void* ap, const void* bp, float* tail_partial,
-                   cudaStream_t st, const float* thr = nullptr) {
+                   cudaStream_t st, const float* thr = nullptr, unsigned char* flags = nullptr) {
   using Cfg = TcCfg<S, BN, PLAIN>;
   CUtensorMap ma, mb;
   if (!make_map_2d(&ma, ap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, L.k_pad, (int64_t)S * L.H * L.m_pad, TC_BK, TC_BM))
@@ -826,13 +830,16 @@ cudaError_t run_tc(const GemmArgs& g, const SplitLayout& L, const void* ap, cons
   }
   const int64_t grid = ts.whole + ts.tail * ts.parts;
   tc_bf16_gemm_kernel<S, BN, CK, PLAIN><<<(unsigned)grid, Cfg::THREADS, Cfg::SMEM, st>>>(
-      ma, mb, g, L.m_pad, L.n_pad, L.k_pad, ts.whole, ts.parts, tail_partial, thr);
+      ma, mb, g, L.m_pad, L.n_pad, L.k_pad, ts.whole, ts.parts, tail_partial, thr, flags);
   e = cudaGetLastError();
   if (e != cudaSuccess || ts.tail == 0) return e;
   const int64_t elems = ts.tail * TC_BM * BN;
   const unsigned blocks = (unsigned)((elems + 255) / 256 < 4096 ? (elems + 255) / 256 : 4096);
-  split_tail_reduce_kernel<BN, PLAIN><<<blocks, 256, 0, st>>>(g, tail_partial, ts.whole, ts.parts, ts.tail, L.m_pad,
-                                                              L.n_pad, thr);
+  if constexpr (PLAIN != 0)
+    plain_tail_reduce_kernel<BN, PLAIN == 2><<<blocks, 256, 0, st>>>(g, tail_partial, ts.whole, ts.parts, ts.tail, L.m_pad,
+                                                                     L.n_pad, thr, flags);
+  else
+    split_tail_reduce_kernel<BN><<<blocks, 256, 0, st>>>(g, tail_partial, ts.whole, ts.parts, ts.tail, L.m_pad, L.n_pad);
   return cudaGetLastError();
 }
 
@@ -889,10 +896,10 @@ cudaError_t launch_tc_bf16_gemm(const GemmArgs& g, const SplitLayout& L, const v
 // ---- plain f32 / c32 --------------------------------------------------------
 
 namespace {
-// The workspace: A' planes, B' planes, their ranges, the tiles' thresholds, the tail
-// parts.
+// The workspace: A' planes, B' planes, their ranges, the tiles' thresholds and flags,
+// the tail parts.
 struct PlainSplitSpace {
-  size_t b, sa, sb, thr, tail, bytes;
+  size_t b, sa, sb, thr, flags, tail, bytes;
   int64_t a_rb, b_rb, nkb;
 };
 PlainSplitSpace plain_split_space(int dtype, const SplitLayout& L) {
@@ -905,7 +912,9 @@ PlainSplitSpace plain_split_space(int dtype, const SplitLayout& L) {
   s.sa = s.b + up((size_t)3 * L.H * L.n_pad * L.k_pad * 2);
   s.sb = s.sa + up((size_t)L.H * s.a_rb * s.nkb * 8);
   s.thr = s.sb + up((size_t)L.H * s.b_rb * s.nkb * 8);
-  s.tail = s.thr + up((size_t)(L.m_pad / TC_BM) * (L.n_pad / 256) * L.H * 4);
+  const size_t tiles = (size_t)(L.m_pad / TC_BM) * (L.n_pad / 256) * L.H;
+  s.flags = s.thr + up(tiles * 4);
+  s.tail = s.flags + up(tiles);
   s.bytes = s.tail + up(split_tail_bytes(L, TC_PLAIN_SMS));
   return s;
 }
@@ -952,14 +961,17 @@ cudaError_t launch_plain_split_gemm(int dtype, const GemmArgs& g, void* ws, cuda
   char* w = static_cast<char*>(ws);
   const int64_t tm = L.m_pad / TC_BM, tn = L.n_pad / 256;
   float* thr = reinterpret_cast<float*>(w + S.thr);
+  unsigned char* flags = reinterpret_cast<unsigned char*>(w + S.flags);
   split_guard_kernel<<<(unsigned)(tm * tn * L.H), 128, 0, st>>>(
       reinterpret_cast<const uint2*>(w + S.sa), reinterpret_cast<const uint2*>(w + S.sb), tm, tn, S.a_rb, S.b_rb,
-      dtype == 2 ? 2 : 4, 8, (int)S.nkb, thr);
-  const cudaError_t e = cudaGetLastError();
+      dtype == 2 ? 2 : 4, 8, (int)S.nkb, (int)L.k_pad, g.e.plain, thr, flags);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   float* tail = reinterpret_cast<float*>(w + S.tail);
-  return dtype == 2 ? run_tc<3, 256, 1, 2>(g, L, w, w + S.b, tail, st, thr)
-                    : run_tc<3, 256, 1, 1>(g, L, w, w + S.b, tail, st, thr);
+  e = dtype == 2 ? run_tc<3, 256, 1, 2>(g, L, w, w + S.b, tail, st, thr, flags)
+                 : run_tc<3, 256, 1, 1>(g, L, w, w + S.b, tail, st, thr, flags);
+  if (e != cudaSuccess) return e;
+  return launch_ffma_again(dtype, g, flags, tm * tn * L.H, tm, tn, 256, true, TC_PLAIN_SMS, st);
 }
 
 }  // namespace dev

@@ -702,8 +702,6 @@ cudaError_t launch_stream_gemm(int dtype, int kernel, const GemmArgs& g0, cudaSt
   if (g0.K <= 0 || stream_dtype(kernel) != dtype) return cudaErrorInvalidValue;
   const GemmArgs g = stream_oriented(g0);
   switch (kernel) {
-    case PLAIN_F32_TC_STREAM:
-    case PLAIN_C32_TC_STREAM: return launch_tc_stream(dtype, g, st);
     case PLAIN_F64_STREAM_64x64: return run_stream<SF64_64x64>(g, st);
     case PLAIN_F64_STREAM_128x32: return run_stream<SF64_128x32>(g, st);
     case PLAIN_F64_STREAM_64x48: return run_stream<SF64_64x48>(g, st);

@@ -34,9 +34,11 @@
 // a swap of the split planes, so a complex element is split once.
 //
 // Values that BF16 planes cannot carry: the producers track the largest and the
-// smallest non-zero magnitude of a tile's operands. A tile with an infinity, a NaN
-// or products near overflow is computed again by FFMA straight from the operands,
-// and so is an output small enough to have lost bits to underflow.
+// smallest non-zero magnitude of a tile's operands. With an infinity, a NaN or sums near
+// overflow, and where outputs are so small that they may have lost bits to underflow, an
+// epilogue warp marks its part of the tile, and a second launch computes the marked parts
+// by FFMA straight from the operands (k_again.cu). Inside this kernel that code cost every
+// call up to a tenth, whichever role ran it, by the register allocation of the others.
 //
 // Every wait is bounded (a status bit, then the role ends). No cluster, no multicast.
 #include <algorithm>
@@ -59,13 +61,14 @@ constexpr int TS_THREADS = 896;
 constexpr int TS_CPT = TS_BN / 2;           // columns of an epilogue warp
 constexpr int TS_STATS = 4;                 // tiles whose value ranges are kept
 constexpr int TS_FLUSH = 8;                 // 32-deep blocks in a running sum
+constexpr int TS_TILES = 15 * 1024;         // tiles of a CTA at most (a byte each)
 
 struct TsSmem {
   static constexpr int RING = TS_STAGES * TS_STAGE;
   static constexpr int COLS = 8 * 4 * TS_CPT * 8;  // per epilogue warp: d_n, c_n of two tiles
   static constexpr int STAT = TS_STATS * 16 * 8;
-  static constexpr int BARS = (2 * TS_STAGES + 2 * 2 + 2 + 2 * TS_STATS + 1) * 8 + 16;
-  static constexpr int BYTES = 128 + RING + COLS + STAT + BARS;
+  static constexpr int BARS = (2 * TS_STAGES + 2 * 2 + 2 + 4 * TS_STATS + 1) * 8 + 8 + 4 * TS_STATS;
+  static constexpr int BYTES = 128 + RING + COLS + STAT + BARS + TS_TILES;
 };
 
 // K-major operand without swizzle: 8-row x 16-byte core matrices, the ones along
@@ -334,10 +337,14 @@ __device__ __forceinline__ void ts_produce(const GemmArgs& g, char* ring, uint64
   if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
 }
 
+__device__ __forceinline__ void ts_mark(unsigned char* again, int tile, int warp) {
+  atomicOr(reinterpret_cast<uint32_t*>(again + (tile & ~3)), 1u << (8 * (tile & 3) + warp));
+}
+
 // STEPS: steps of 16 plane depths (one MMA each) in all of K: 1, 2 or (3) more.
 template <bool CPLX, int STEPS>
 __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_constant__ GemmArgs g, int tiles, int tm,
-                                                                  int tn) {
+                                                                  int tn, unsigned char* __restrict__ flags) {
   using T = typename Elem<float, CPLX>::type;
   constexpr int EK = CPLX ? TS_BK / 2 : TS_BK;
   extern __shared__ unsigned char ts_smem[];
@@ -351,8 +358,14 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
   uint64_t* corr_empty = main_empty + 2;
   uint64_t* stat_full = corr_empty + 2;
   uint64_t* stat_empty = stat_full + TS_STATS;
-  uint64_t* done = stat_empty + TS_STATS;
+  uint64_t* thr_full = stat_empty + TS_STATS;
+  uint64_t* thr_empty = thr_full + TS_STATS;
+  uint64_t* done = thr_empty + TS_STATS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  // Per tile of this CTA, the epilogue warps whose outputs are computed again.
+  volatile float* thresholds = reinterpret_cast<float*>(tmem_slot + 2);  // split_guard of a tile
+  unsigned char* again = reinterpret_cast<unsigned char*>(tmem_slot + 2 + TS_STATS);
+  const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nk = (int)((g.K + EK - 1) / EK);
@@ -368,7 +381,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     }
     for (int s = 0; s < TS_STATS; ++s) {
       mbar_init(&stat_full[s], 16);
-      mbar_init(&stat_empty[s], 8);
+      mbar_init(&stat_empty[s], 1);
+      mbar_init(&thr_full[s], 1);
+      mbar_init(&thr_empty[s], 8);
     }
     mbar_init(done, 1);
     fence_barrier_init();
@@ -377,6 +392,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  for (int i = 4 * threadIdx.x; i < mine; i += 4 * TS_THREADS) *reinterpret_cast<uint32_t*>(again + i) = 0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -387,7 +403,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
   const int steps_all = (int)((g.K * (CPLX ? 2 : 1) + 15) / 16);
   const uint32_t tmem = *tmem_slot;
 
-  // Registers a thread: 64 x 256 + 80 x 512 + 40 x 128 = 62464 of the launch's 72 x 896.
+  // Registers a thread: 64 x 256 + 80 x 512 + 56 x 128 = 64512, the launch's 72 x 896.
   if (warp >= 8 && warp < 24) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     if ((warp & 7) < 4)
@@ -395,7 +411,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
     else
       ts_produce<CPLX, false>(g, ring, full, empty, stats, stat_full, stat_empty, tiles, tm, tn, warp - 8, lane);
   } else if (warp >= 24) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 24 && lane == 0) {
       int stage = 0;
       uint32_t round = 0, blocks = 0;
@@ -455,6 +471,31 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       if (!mbar_wait_polls(done, 0)) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
     }
     __syncwarp();
+    if (warp == 25) {
+      // The tiles' thresholds from the value ranges that the producers found.
+      bool ok = true;
+      for (int it = 0; ok && it < mine; ++it) {
+        const int s = it % TS_STATS;
+        const uint32_t turn = (uint32_t)(it / TS_STATS);
+        ok = mbar_wait_polls(&stat_full[s], turn & 1u) && mbar_wait_polls(&thr_empty[s], (turn & 1u) ^ 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        const int2 r = stats[s * 16 + (lane & 15)];
+        const bool is_a = (lane & 4) == 0;
+        const int amax = (int)__reduce_max_sync(0xffffffffu, (uint32_t)(is_a ? r.x : 0));
+        const int bmax = (int)__reduce_max_sync(0xffffffffu, (uint32_t)(is_a ? 0 : r.x));
+        const int amin = (int)__reduce_min_sync(0xffffffffu, (uint32_t)(is_a ? r.y : 0x7fff));
+        const int bmin = (int)__reduce_min_sync(0xffffffffu, (uint32_t)(is_a ? 0x7fff : r.y));
+        if (lane == 0 && ok) {
+          thresholds[s] = split_guard((amax >> 7) - 127, amin == 0x7fff ? 999 : (amin >> 7) - 127, (bmax >> 7) - 127,
+                                      bmin == 0x7fff ? 999 : (bmin >> 7) - 127, (int)g.K * (CPLX ? 2 : 1));
+          mbar_arrive(&stat_empty[s]);
+          mbar_arrive(&thr_full[s]);
+        }
+        __syncwarp();
+      }
+      if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+      __syncwarp();
+    }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const int col0 = (warp >> 2) * TS_CPT;
@@ -531,26 +572,20 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       // of the tile's operands.
       const int s = it % TS_STATS;
       if (ok) ok = mbar_wait_polls(&main_full[mset], (STEPS == 1 ? (uint32_t)(it >> 1) : blocks) & 1u);
-      if (ok) ok = mbar_wait_polls(&stat_full[s], (uint32_t)(it / TS_STATS) & 1u);
+      if (ok) ok = mbar_wait_polls(&thr_full[s], (uint32_t)(it / TS_STATS) & 1u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      int amax = 0, bmax = 0, amin = 0x7fff, bmin = 0x7fff;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const int2 a = stats[s * 16 + w / 4 * 8 + w % 4], b = stats[s * 16 + w / 4 * 8 + 4 + w % 4];
-        amax = max(amax, a.x);
-        amin = min(amin, a.y);
-        bmax = max(bmax, b.x);
-        bmin = min(bmin, b.y);
-      }
-      const float thr = split_guard((amax >> 7) - 127, amin == 0x7fff ? 999 : (amin >> 7) - 127, (bmax >> 7) - 127,
-                                    bmin == 0x7fff ? 999 : (bmin >> 7) - 127);
-      const bool guard = thr != 0.f;
-      uint64_t again = 0;
+      const float thr = thresholds[s];
       const bool second = steps_all % 2 == 0, more = (nk - 1) % TS_FLUSH != 0, flushed = nk > TS_FLUSH;
+      // Sums that the planes may not carry are computed again: all of them, or (a finite
+      // threshold, and D only written) this warp's once one of them is below it.
+      const bool skip = thr == __uint_as_float(0x7f800000u) || (thr != 0.f && !e.plain);
+      if (skip && lane == 0) ts_mark(again, it, warp);
+      const int ncols = skip ? 0 : nrem;
+      float least = __uint_as_float(0x7f800000u);  // magnitude of what this lane writes
 #pragma unroll 1
-      for (int q = 0; 8 * q < nrem; ++q) {
+      for (int q = 0; 8 * q < ncols; ++q) {
         {
           uint32_t r[8], u[8];
           float v[8];
@@ -585,8 +620,10 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(u[j]);
-          if (!guard && e.plain && 8 * q + 8 <= nrem) {
+          if (e.plain && 8 * q + 8 <= ncols) {
             float* Df = reinterpret_cast<float*>(Db) + comp;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) least = fminf(least, fabsf(v[j]));
             if (mok) {
 #pragma unroll
               for (int j = 0; j < 8; j += 2) {
@@ -604,11 +641,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
               for (int i = 1; i < 8; ++i) y = j == i ? v[i] : y;
               const int jj = 8 * q + j;
               const float o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
-              if (jj >= nrem || !mok || comp) continue;
-              if (split_lost(thr, y) || (CPLX && split_lost(thr, o)))
-                again |= (uint64_t)1 << jj;
-              else
-                epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
+              if (jj < ncols) least = fminf(least, fabsf(y));
+              if (jj >= ncols || !mok || comp) continue;
+              epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
             }
           }
           __syncwarp();
@@ -619,21 +654,20 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       if (lane == 0) {
         mbar_arrive(&main_empty[mset]);
         mbar_arrive(&corr_empty[set]);
-        mbar_arrive(&stat_empty[s]);
       }
-      ++blocks;
-      for (; again; again &= again - 1) {
-        const int j = __ffsll((long long)again) - 1;
-        const float2 r = ffma_dot<CPLX>(g, x.h, m, n0 + j);
-        epilogue_store<float, CPLX>(e, r.x, r.y, Cb + (e.beta_zero ? 0 : cn_s[j]), Db + dn_s[j]);
-      }
+      const float bound = thresholds[s];
+      if (bound != 0.f && !skip && __any_sync(0xffffffffu, !(least >= bound)) && lane == 0) ts_mark(again, it, warp);
       __syncwarp();
+      if (lane == 0) mbar_arrive(&thr_empty[s]);
+      ++blocks;
     }
     if (!ok) atomicOr(g.status, STATUS_WAIT_TIMEOUT);
+    __syncwarp();
   }
 
   tc_fence_before();
   __syncthreads();
+  for (int i = tid; i < mine; i += TS_THREADS) flags[blockIdx.x + i * gridDim.x] = again[i];
   if (warp == 24) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -727,8 +761,9 @@ bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const
       (!hints.b_gather && (double)panel_ld(N) * (double)K >= 2.0 * most - (double)N))
     return false;
   const int64_t em = dtype == 2 ? TS_BM / 2 : TS_BM;
-  return ((double)(M / em) + 1) * ((double)(N / TS_BN) + 1) * (double)H < (double)most &&
-         ((double)(N / em) + 1) * ((double)(M / TS_BN) + 1) * (double)H < (double)most;
+  const double tiles = (double)TS_TILES * 64;  // TS_TILES for each CTA of a grid of 64 or more
+  return ((double)(M / em) + 1) * ((double)(N / TS_BN) + 1) * (double)H < tiles &&
+         ((double)(N / em) + 1) * ((double)(M / TS_BN) + 1) * (double)H < tiles;
 }
 
 // Against the FFMA families by estimated microseconds, fitted on B200. Here: 8, per
@@ -772,7 +807,12 @@ int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int 
 }
 
 // The caller has checked tc_stream_fits.
-cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st) {
+size_t tc_stream_flag_bytes(int dtype, int64_t M, int64_t N, int64_t H) {
+  const auto tiles = [&](int64_t m, int64_t n) { return ((m + (dtype == 2 ? 63 : 127)) / (dtype == 2 ? 64 : 128)) * ((n + TS_BN - 1) / TS_BN) * H; };
+  return (size_t)std::max(tiles(M, N), tiles(N, M)) + 256;  // either orientation
+}
+
+cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, void* flags, cudaStream_t st) {
   if (dtype != 0 && dtype != 2) return cudaErrorInvalidValue;
   const int64_t em = dtype == 2 ? TS_BM / 2 : TS_BM;
   const int64_t tm = (g.M + em - 1) / em, tn = (g.N + TS_BN - 1) / TS_BN, tiles = tm * tn * g.H;
@@ -786,8 +826,10 @@ cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st) {
                                                                                  : tc_stream_kernel<false, 3>);
   const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TsSmem::BYTES);
   if (r != cudaSuccess) return r;
-  kern<<<grid, TS_THREADS, TsSmem::BYTES, st>>>(g, (int)tiles, (int)tm, (int)tn);
-  return cudaGetLastError();
+  kern<<<grid, TS_THREADS, TsSmem::BYTES, st>>>(g, (int)tiles, (int)tm, (int)tn, static_cast<unsigned char*>(flags));
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return launch_ffma_again(dtype, g, static_cast<const unsigned char*>(flags), tiles, tm, tn, TS_BN, false, sms, st);
 }
 
 }  // namespace dev

@@ -140,7 +140,14 @@ cudaError_t launch_stream_grouped(int kernel, const GroupItem* items, const int6
                                   unsigned long long* counter, unsigned* status, int num_sms, cudaStream_t st);
 // f32 and c32 on the tensor cores without a pack pass (k_tcstream.cu).
 bool is_tc_stream(int kernel);
-cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, cudaStream_t st);
+// `flags`: tc_stream_flag_bytes of device memory.
+size_t tc_stream_flag_bytes(int dtype, int64_t M, int64_t N, int64_t H);
+cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, void* flags, cudaStream_t st);
+// FFMA pass over marked tiles (k_again.cu): flags[t] holds a bit per part of tile t, parts
+// of 32 plane rows (c32: 16 rows of D) by half of the tile's `tile_n` columns, rows
+// fastest. `grouped`: tiles in the order of the packed kernel, else column tile fastest.
+cudaError_t launch_ffma_again(int dtype, const GemmArgs& g, const unsigned char* flags, int64_t tiles, int64_t tiles_m,
+                              int64_t tiles_n, int tile_n, bool grouped, int sms, cudaStream_t st);
 bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints);
 // The tensor-core family the model takes for a plain f32 or c32 contraction (0: none).
 int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);

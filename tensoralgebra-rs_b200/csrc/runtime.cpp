@@ -672,7 +672,12 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const Plai
       check_cuda(dev::launch_stream_pack(dt, g, which, which == 0 ? pr.a_fast : pr.b_fast, panel, ex.stream), "stream pack launch");
       scratch = panel + bytes;
     }
-    scratch_bytes = (size_t)(scratch_end - scratch);
+    char* flags = reinterpret_cast<char*>(align_up((uintptr_t)scratch, 256));
+    if (flags + dev::tc_stream_flag_bytes(dt, g.M, g.N, g.H) > scratch_end)
+      throw Error(ERR_INTERNAL, "stream flag workspace too small");
+    Timed t(ex, dev::plain_kernel_name(c.kernel));
+    check_cuda(dev::launch_tc_stream(dt, dev::stream_oriented(g), flags, ex.stream), "tcgen05 contraction launch");
+    return;
   }
   if (c.splits > 1) {
     // Split-K: partial tiles into the scratch, then the reduce + epilogue.

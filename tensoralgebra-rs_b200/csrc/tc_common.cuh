@@ -181,6 +181,31 @@ inline bool make_map_2d(CUtensorMap* map, const void* base, CUtensorMapDataType 
   return r == CUDA_SUCCESS;
 }
 
+// Marks part `which` (0..7) of a tile to be computed again (launch_ffma_again).
+__device__ inline void mark_again(unsigned char* flags, int64_t tile, int which) {
+  atomicOr(reinterpret_cast<uint32_t*>(flags + (tile & ~(int64_t)3)), 1u << (8 * (int)(tile & 3) + which));
+}
+
+// Tile order: within a batch entry, tiles go in groups of TILE_GROUP_M m-tiles
+// (the last group may be narrower); inside a group the m-tile is fastest, then
+// the n-tile. A wave of 148 CTAs then covers a block of about 16 A row panels
+// by 9 B column panels instead of 9 row panels by every column panel, so the
+// B planes a wave reads stay in L2 for the next wave of the same group.
+constexpr int TILE_GROUP_M = 16;
+
+__host__ __device__ inline void tile_coords(int64_t tile, int64_t tiles_m, int64_t tiles_n, int64_t& h, int64_t& mt,
+                                            int64_t& nt) {
+  const int64_t per_h = tiles_m * tiles_n;
+  h = tile / per_h;
+  const int64_t t = tile % per_h;
+  const int64_t group = t / (TILE_GROUP_M * tiles_n);
+  const int64_t first_m = group * TILE_GROUP_M;
+  const int64_t gm = tiles_m - first_m < TILE_GROUP_M ? tiles_m - first_m : TILE_GROUP_M;
+  const int64_t local = t - group * TILE_GROUP_M * tiles_n;
+  mt = first_m + local % gm;
+  nt = local / gm;
+}
+
 }  // namespace tc
 }  // namespace dev
 }  // namespace tprims

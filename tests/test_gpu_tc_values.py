@@ -72,3 +72,79 @@ def test_elements_below_every_plane(tp, ex, torch_cuda, dt, shape, what, side):
     lim = 2.0 ** -20 * np.abs(y.astype("complex128"))
     assert np.all(np.abs(y) > 0)
     assert np.all(np.abs(x.astype("complex128") - y) <= lim)
+
+
+def tiny_block_case(dt, m, n, k, rng):
+    """Ordinary values, but three quarters of the rows and half of the columns are zero,
+    a few rows hold 1e-33 and others an infinity: outputs of every kind side by side."""
+    (A, B), a, b = matrix_pair(dt, m, n, k)
+    for x in (a, b):
+        x[...] = rng.uniform(-1, 1, x.shape)
+    a[:, ::4] = 0
+    a[:, 1::4] *= np.float32(1e-33)
+    b[::2] = 0
+    a[min(5, k - 1), 1000:1003] = np.inf
+    return A, B
+
+
+@pytest.mark.parametrize("cmode", [None, "own", "in place"])
+@pytest.mark.parametrize("shape", SHAPES + [(1100, 2600, 1100, ".split.")], ids=["in flight", "packed", "packed, few tiles"])
+@pytest.mark.parametrize("dt", sorted(DIRECT))
+def test_parts_computed_again(tp, ex, torch_cuda, dt, shape, cmode):
+    """Tiles that are computed again in part, or left out first and computed whole
+    (alpha and beta), give what the direct tile gives."""
+    m, n, k, family = shape
+    rng = np.random.default_rng(m)
+    A, B = tiny_block_case(dt, m, n, k, rng)
+    d0 = rng.uniform(-1, 1, m * n).astype(dt) if cmode else np.zeros(m * n, dtype=dt)
+    D = Op(d0, [m, n], [1, m], [0, 1])
+    C = None if cmode is None else D if cmode == "in place" else Op(rng.uniform(-1, 1, m * n).astype(dt), [m, n], [n, 1], [0, 1])
+    p = make_product(tp, dt, A, B, C, D)
+    assert family in p.report()["family"], p.report()["family"]
+    out = []
+    for kernel in (0, DIRECT[dt]):
+        p.set_kernel(kernel)
+        status, td = execute(torch_cuda, p, ex, dt, A, B, C, D, 1.0 if cmode is None else 1.5, 0.0 if cmode is None else -0.5)
+        assert status == 0, tp.last_error()
+        torch_cuda.cuda.synchronize()
+        out.append(td.cpu().numpy().view("float32").reshape(n, -1))
+    x, y = out
+    assert np.array_equal(np.isfinite(x), np.isfinite(y)) and np.array_equal(np.isnan(x), np.isnan(y))
+    # Each output within 60 roundings of its products' magnitudes, and of C's.
+    a, b = np.abs(A.buf.reshape(k, m)).astype("float64"), np.abs(B.buf.reshape(n, k)).astype("float64")
+    mag = np.repeat(b @ np.where(np.isfinite(a), a, 0), x.shape[1] // m, axis=1)
+    lim = 60 * (2.0 ** -24 * 2 * mag + 2.0 ** -149) + (0 if cmode is None else 2.0 ** -22)
+    ok = np.isfinite(y)
+    assert np.all(np.abs(x[ok].astype("float64") - y[ok]) <= lim[ok])
+
+
+@pytest.mark.parametrize("what", ["one NaN", "2^55"])
+@pytest.mark.parametrize("m,n,k", [(2048, 2048, 256), (2048, 2048, 2048)])
+@pytest.mark.parametrize("dt", sorted(DIRECT))
+def test_values_outside_the_planes_take_no_cliff(tp, torch_cuda, dt, m, n, k, what):
+    """At most twice the time of the FFMA tiles (and some for two small launches)."""
+    torch = torch_cuda
+    A = (torch.rand(k, m, device="cuda", dtype=getattr(torch, dt)) - 0.5).t()
+    B = (torch.rand(n, k, device="cuda", dtype=getattr(torch, dt)) - 0.5).t()
+    if what == "one NaN":
+        A[7, 3] = float("nan")
+    else:
+        A.mul_(2.0 ** 55)
+        B.mul_(2.0 ** 55)
+    D = torch.zeros(n, m, device="cuda", dtype=A.dtype).t()
+    e = tp.Executor(device=0, stream=torch.cuda.current_stream().cuda_stream, sync=False)
+    lay = lambda t: tp.OperandSpec(tp.LayoutSpec(list(t.shape), list(t.stride())))
+    prob = tp.Problem.from_labels({"float32": tp.F32, "complex64": tp.C32}[dt], lay(A), lay(B), lay(D), [0, 2], [2, 1], [0, 1])
+    ms = []
+    for kernel in (0, {"float32": 10, "complex64": 15}[dt]):
+        plan = tp.Plan(prob, tp.PlanConfig(kernel=kernel))
+        for _ in range(2):
+            plan.execute_into(e, 1.0, A, B, D)
+        t = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+        for ev in t:
+            ev.record()
+            plan.execute_into(e, 1.0, A, B, D)
+        torch.cuda.synchronize()
+        ms.append(min(u.elapsed_time(v) for u, v in zip(t, t[1:])))
+    e.close()
+    assert ms[0] <= 2 * ms[1] + 0.05, ms
