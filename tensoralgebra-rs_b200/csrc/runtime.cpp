@@ -572,6 +572,11 @@ void join_side(Executor& ex) {
   check_cuda(cudaStreamWaitEvent(ex.stream, ex.family_events[1], 0), "cudaStreamWaitEvent");
 }
 
+// The tensor-core families load complex elements whole: c32 operands on 8 bytes.
+bool whole_elements(const Product& pr, const void* a, const void* b) {
+  return pr.problem.dtype != DType::C32 || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 7) == 0;
+}
+
 // One plain execution in the configuration `c` (scratch: the split-K partials).
 void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const PlainChoice& c, char* scratch,
                   size_t scratch_bytes) {
@@ -640,13 +645,7 @@ void launch_plain(Product& pr, Executor& ex, const dev::GemmArgs& g0, const Plai
     return;
   }
   if (dev::is_tc_stream(c.kernel) || dev::is_tc_split(c.kernel)) {
-    // Complex elements are loaded whole: operands off their natural alignment
-    // take the direct tile.
-    if (dt == 2 && ((reinterpret_cast<uintptr_t>(g0.A) | reinterpret_cast<uintptr_t>(g0.B)) & 7) != 0) {
-      PlainChoice d = c;
-      d.kernel = dev::PLAIN_C32_SIMT_64x64;
-      return launch_plain(pr, ex, g0, d, scratch, scratch_bytes);
-    }
+    if (!whole_elements(pr, g0.A, g0.B)) throw Error(ERR_INTERNAL, "operands off the alignment of the tensor-core families");
     if (dev::is_tc_split(c.kernel)) {
       if (dev::plain_split_bytes(dt, g.M, g.N, g.K, g.H) > scratch_bytes)
         throw Error(ERR_INTERNAL, "split plane workspace too small");
@@ -948,7 +947,7 @@ int tune_reps(double first_ms) { return first_ms < 0.05 ? 10 : first_ms < 1.0 ? 
 // before every run and at the end, so the caller's execution afterwards sees
 // the original D.
 TuneEntry autotune_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, char* scratch, size_t scratch_bytes,
-                         char* d_span, char* snapshot, size_t span_bytes) {
+                         char* d_span, char* snapshot, size_t span_bytes, const PlainChoice& model) {
   NvtxRange range("tprims.autotune");
   ProfileOff off(ex);
   const auto restore = [&] {
@@ -962,7 +961,6 @@ TuneEntry autotune_plain(Product& pr, Executor& ex, const dev::GemmArgs& g, char
   EventPair ev;
   std::vector<PlainChoice> cands = plain_candidates((int)pr.problem.dtype, pr.view.M, pr.view.N, pr.view.K, pr.view.H,
                                                     ex.num_sms, pr.hints);
-  const PlainChoice model = model_choice(pr, ex.num_sms);
   if (!(cands.front() == model)) cands.insert(cands.begin(), model);
   TuneEntry best;
   best.ms = 0;
@@ -1355,12 +1353,19 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
   ChoiceSource src = ChoiceSource::Model;
   bool tune = false;
   std::string key;
+  // Operands that the tensor-core families cannot take (staged ones are aligned).
+  const auto at = [&](int slot) { return st[slot].staged ? nullptr : st[slot].dev_origin; };
+  const bool whole = whole_elements(pr, at(SA), at(SB));
+  const auto general_if_off = [&] {
+    if (!whole && (dev::is_tc_stream(pc.kernel) || dev::is_tc_split(pc.kernel))) pc = model_choice(pr, ex.num_sms, true);
+  };
   if (pr.scheme == Scheme::Plain && !output_only) {
     pc = model_choice(pr, ex.num_sms);
+    general_if_off();
     if (pr.kernel_pin || pr.split_pin) {
       src = ChoiceSource::Pinned;
     } else if (pr.autotune) {
-      key = tune_key(pr, c_read);
+      key = tune_key(pr, c_read) + (whole ? "" : ";off");
       const auto hit = ex.tune.find(key);
       if (hit != ex.tune.end()) {
         // A loaded entry that does not fit this product (a stale or edited
@@ -1369,6 +1374,7 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
         if (choice_fits(hit->second.choice, pr)) {
           pc = hit->second.choice;
           src = hit->second.tuned ? ChoiceSource::Cached : ChoiceSource::Model;
+          general_if_off();
         }
       } else {
         tune = true;
@@ -1428,7 +1434,7 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
                                      st[SD].dev_origin);
   if (tune) {
     const TuneEntry e = autotune_plain(pr, ex, g, scratch_ptr, scratch, snap ? st[SD].dev_origin + d_lo : nullptr,
-                                       snap_ptr, d_bytes);
+                                       snap_ptr, d_bytes, pc);
     ex.tune[key] = e;
     pc = e.choice;
     src = ChoiceSource::Autotuned;
