@@ -1141,7 +1141,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
   if (!split && pr.scheme != Scheme::Plain) return false;
   std::vector<PlainChoice> pcs;
   size_t scratch = 0;
-  const auto configure = [&](const Side& sd) {
+  const auto configure = [&](const Side& sd, const dev::LaunchHints& hints) {
     const int nc = (int)sd.lo.size();
     const auto cm = [&](int c) { return sd.rows ? (sd.hi[c] - sd.lo[c]) * sd.inner : v.M; };
     const auto cn = [&](int c) { return sd.rows ? v.N : (sd.hi[c] - sd.lo[c]) * sd.inner; };
@@ -1168,7 +1168,7 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
       const int64_t mc = cm(c), ncols = cn(c);
       PlainChoice& pc = pcs[c];
       if (dev::use_tiny_batched(mc, ncols, v.K, v.H)) return false;
-      dev::choose_plain_launch((int)p.dtype, pr.kernel_pin, mc, ncols, v.K, v.H, ex.num_sms, pr.hints, &pc.kernel,
+      dev::choose_plain_launch((int)p.dtype, pr.kernel_pin, mc, ncols, v.K, v.H, ex.num_sms, hints, &pc.kernel,
                                &pc.splits, &pc.chunk);
       if (pc.splits > 1) return false;
       if (dev::is_packed_kernel(pc.kernel))
@@ -1178,20 +1178,6 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
     }
     return true;
   };
-  Side sd;
-  const bool prefer_rows = bytes_y > bytes_x;
-  if (!(plan_side(prefer_rows, sd) && configure(sd)) && !(plan_side(!prefer_rows, sd) && configure(sd)))
-    return false;
-  const bool rows = sd.rows;
-  const int nchunks = (int)sd.lo.size();
-  const std::vector<int64_t>& lo = sd.lo;
-  const std::vector<int64_t>& hi = sd.hi;
-  const int64_t inner = sd.inner;
-  const int chunked = sd.slot, whole = rows ? sx : sy;
-  // Rows and columns of chunk c.
-  const auto chunk_m = [&](int c) { return rows ? (hi[c] - lo[c]) * inner : v.M; };
-  const auto chunk_n = [&](int c) { return rows ? v.N : (hi[c] - lo[c]) * inner; };
-
   // Workspace: the staged spans of A, B and D, then the kernels' scratch.
   Staged st[4];
   const void* origins[4] = {it.a, it.b, nullptr, it.d};
@@ -1202,8 +1188,28 @@ bool enqueue_streamed(Product& pr, Executor& ex, Scalar alpha, const Item& it) {
     span_bytes(p, s, &st[s].lo_bytes, &st[s].bytes);
     total = align_up(total, 256) + st[s].bytes;
   }
+  const auto need = [&] { return align_up(total, 256) + align_up(scratch, 256) + 1024; };
+  Side sd;
+  const bool prefer_rows = bytes_y > bytes_x;
+  const auto pick = [&](const dev::LaunchHints& hints) {
+    return (plan_side(prefer_rows, sd) && configure(sd, hints)) || (plan_side(!prefer_rows, sd) && configure(sd, hints));
+  };
+  bool taken = pick(pr.hints);
+  // Beyond the workspace cap: the choice that needs no layout hints (enqueue_item).
+  if (!split && !pr.kernel_pin && (!taken || need() > ex.ws_limit)) taken = pick(dev::LaunchHints{});
+  if (!taken) return false;
+  const bool rows = sd.rows;
+  const int nchunks = (int)sd.lo.size();
+  const std::vector<int64_t>& lo = sd.lo;
+  const std::vector<int64_t>& hi = sd.hi;
+  const int64_t inner = sd.inner;
+  const int chunked = sd.slot, whole = rows ? sx : sy;
+  // Rows and columns of chunk c.
+  const auto chunk_m = [&](int c) { return rows ? (hi[c] - lo[c]) * inner : v.M; };
+  const auto chunk_n = [&](int c) { return rows ? v.N : (hi[c] - lo[c]) * inner; };
+
   injected_failure_check(ex);
-  char* ws = static_cast<char*>(ex.workspace(align_up(total, 256) + align_up(scratch, 256) + 1024));
+  char* ws = static_cast<char*>(ex.workspace(need()));
   size_t off = 0;
   for (int s : {SA, SB, SD}) {
     off = align_up(off, 256);

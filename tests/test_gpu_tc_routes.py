@@ -57,3 +57,58 @@ def test_c32_operands_off_eight_bytes(tp, torch_cuda, m, n, k, splits, off, auto
         tp.check(p.execute(ex, 1.0, aligned["A"], aligned["B"], 0.0, None, aligned["D"]))
         assert p.report()["family"] == model["family"]
     ex.close()
+
+
+def host_call(tp, torch, dtype, m, n, k, a_lead, limit=None, streaming=True):
+    """D = A B of host operands, A with leading stride `a_lead`; returns the status, D's
+    error against 64 bits, the family and the launches of the call."""
+    gen = torch.Generator().manual_seed(m + n)
+    make = lambda count: torch.randn(count, generator=gen, dtype=torch.complex64 if dtype == tp.C32 else torch.float32)
+    a, b = make(a_lead * m * k).pin_memory(), make(k * n).pin_memory()
+    d = torch.zeros(m * n, dtype=a.dtype).pin_memory()
+    h = tp.Handle()
+    infos = [tp.TensorInfo(dtype, [m, k], [a_lead, a_lead * m]), tp.TensorInfo(dtype, [k, n], [1, k]),
+             tp.TensorInfo(dtype, [m, n], [1, m])]
+    p = tp.TensorProduct.create(h, (0, infos[0], [0, 2]), (0, infos[1], [2, 1]), (0, infos[2], [0, 1]), (0, infos[2], [0, 1]))
+    ex = tp.Executor()
+    ex.set_profiling(True)
+    ex.set_streaming(streaming)
+    if limit:
+        ex.set_workspace_limit(limit)
+    status = p.execute(ex, 1.0, a.data_ptr(), b.data_ptr(), 0.0, None, d.data_ptr())
+    wide = torch.complex128 if dtype == tp.C32 else torch.float64
+    da, db = a.cuda().view(k, m, a_lead)[:, :, 0].to(wide), b.cuda().view(n, k).to(wide)
+    want = db @ da
+    err = float((d.cuda().view(n, m).to(wide) - want).norm() / want.norm())
+    times = ex.kernel_times()
+    ex.close()
+    return status, err, p.report()["family"], times
+
+
+@pytest.mark.parametrize("dtype", ["F32", "C32"])
+@pytest.mark.parametrize("m,n,k,a_lead,what", [(9000, 1000, 64, 1, ".stream."),    # chunks on 16-byte groups
+                                                (9006, 1000, 64, 1, ".stream."),    # and off them (4503 rows first)
+                                                (8194, 1100, 60, 2, ".stream."),    # A through panels
+                                                (6006, 3000, 2000, 1, ".split.")])   # planes packed first
+def test_host_operands_streamed_to_the_tensor_cores(tp, torch_cuda, dtype, m, n, k, a_lead, what):
+    status, err, family, times = host_call(tp, torch_cuda, getattr(tp, dtype), m, n, k, a_lead)
+    assert status == 0, tp.last_error()
+    assert what in family and times[family]["launches"] >= 2, (family, times)
+    assert err <= 1e-6
+
+
+@pytest.mark.parametrize("dtype", ["F32", "C32"])
+def test_host_operands_streamed_under_a_workspace_cap(tp, torch_cuda, dtype):
+    """Room for the operands and for packed panels of a chunk, not for planes: the call
+    runs streamed on the packed family."""
+    m, n, k = (8192, 5120, 960) if dtype == "F32" else (8192, 4096, 512)
+    item = 4 if dtype == "F32" else 8
+    spans = item * (m * k + k * n + m * n)
+    # The first chunk (half the rows): panels of A' and B' (c32: 4 and 2 reals an element).
+    panels = 4 * (4096 * k + k * n) if dtype == "F32" else 4 * (4 * 4096 * k + 2 * k * n)
+    status, err, family, times = host_call(tp, torch_cuda, getattr(tp, dtype), m, n, k, 1, limit=spans + panels + (1 << 20))
+    assert status == 0, tp.last_error()
+    assert ".tcgen05." not in family and times[family]["launches"] >= 2, (family, times)
+    assert err <= 1e-6
+    status, err, family, _ = host_call(tp, torch_cuda, getattr(tp, dtype), m, n, k, 1)
+    assert status == 0 and ".tcgen05." in family and err <= 1e-6
