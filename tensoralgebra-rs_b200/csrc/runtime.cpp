@@ -399,8 +399,11 @@ std::string Product::report() const {
     for (size_t i = 0; i < cands.size(); ++i)
       o << (i ? "," : "") << "\"" << choice_name(cands[i], (int)problem.dtype) << "\"";
   }
-  o << "]"
-    << ",\"choice\":\"" << (scheme == Scheme::Plain ? src_names[(int)src] : "fixed")
+  // The model's own choice, timed beside them where it is a family that cannot be named.
+  o << "]";
+  if (scheme == Scheme::Plain)
+    o << ",\"autotune_model\":\"" << choice_name(model_choice(*this, 148), (int)problem.dtype) << "\"";
+  o << ",\"choice\":\"" << (scheme == Scheme::Plain ? src_names[(int)src] : "fixed")
     << "\",\"autotune\":" << (autotune ? "true" : "false") << ",\"signature\":\"" << signature << "\""
     << ",\"stated_rel_error\":" << stated_bound(problem.dtype, scheme)
     << ",\"regular_rows\":" << regular_fraction(build_block_scatter(view.d_m, 32))
@@ -1392,6 +1395,7 @@ bool enqueue_item(Product& pr, Executor& ex, Scalar alpha, Scalar beta, const It
       align_up(total, 256) + align_up(scratch, 256) + 1024 > ex.ws_limit) {
     // Beyond the workspace cap: the choice that needs no layout hints.
     pc = model_choice(pr, ex.num_sms, true);
+    src = pr.split_pin ? ChoiceSource::Pinned : ChoiceSource::Model;
     scratch = scheme_scratch(pr, pc, ex.num_sms);
   }
   int64_t d_lo = 0;

@@ -112,3 +112,24 @@ def test_host_operands_streamed_under_a_workspace_cap(tp, torch_cuda, dtype):
     assert err <= 1e-6
     status, err, family, _ = host_call(tp, torch_cuda, getattr(tp, dtype), m, n, k, 1)
     assert status == 0 and ".tcgen05." in family and err <= 1e-6
+
+
+def test_a_cached_choice_beyond_the_cap_is_reported_as_the_models(tp, torch_cuda):
+    torch = torch_cuda
+    m, n, k = 2000, 2000, 40
+    a, b = torch.randn(m * k, device="cuda"), torch.randn(k * n, device="cuda")
+    d = torch.zeros(m * n, device="cuda")
+    p = column_major(tp, tp.F32, m, n, k)
+    p.set_autotune(True)
+    ex = tp.Executor()
+    call = lambda: tp.check(p.execute(ex, 1.0, a.data_ptr(), b.data_ptr(), 0.0, None, d.data_ptr()))
+    call()
+    tuned = p.report()
+    assert tuned["choice"] == "autotuned" and ".tcgen05." in tuned["family"]
+    call()
+    assert p.report()["choice"] == "tuning-cache"
+    ex.set_workspace_limit(64)
+    call()
+    rep = p.report()
+    assert ".tcgen05." not in rep["family"] and rep["choice"] == "model"
+    ex.close()
