@@ -96,7 +96,7 @@ std::vector<PlainChoice> plain_candidates(int dtype, int64_t M, int64_t N, int64
       // The families a caller can name; the tensor-core stream tiles, where the
       // model takes them, are timed beside these (autotune_plain).
       dev::LaunchHints named = hints;
-      named.off32 = false;
+      named.tensor = false;
       dev::choose_plain_launch(dtype, 0, M, N, K, H, num_sms, named, &m.kernel, &m.splits, &m.chunk);
     }
     out.push_back(m);

@@ -780,7 +780,7 @@ bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const
 // against 1.21 here and 2.70 there, 2048^2 x 512 55 against 51 here; c32 2048^3 0.41
 // ms against 0.66 here and 1.53 there; f32 700^2 x 2500 against 108 here, 94 there).
 int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
-  if (!tc_stream_fits(dtype, M, N, K, H, hints)) return 0;
+  if (!hints.tensor || !tc_stream_fits(dtype, M, N, K, H, hints)) return 0;
   const bool cplx = dtype == 2;
   const int64_t m = hints.d_mfast ? M : N, n = hints.d_mfast ? N : M;  // the launch's roles
   const int64_t em = cplx ? TS_BM / 2 : TS_BM, ek = cplx ? TS_BK / 2 : TS_BK, pad = cplx ? 64 : 128;

@@ -194,6 +194,7 @@ struct LaunchHints {
   bool a_gather = false, b_gather = false, a_vec = false, b_vec = false, d_mfast = true;
   bool h_inner = false;  // the batch index has the smallest stride of A', B' and D
   bool off32 = false;    // row plus depth offsets of A' and of B' fit 32 bits
+  bool tensor = true;    // the tensor-core families of f32 and c32 may be chosen
 };
 // The family the autotuner would pick for a shape (no launch).
 int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints);
