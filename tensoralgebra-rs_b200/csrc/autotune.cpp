@@ -201,6 +201,47 @@ bool choice_fits(const PlainChoice& c, const Product& p) {
   return c.chunk > 0 && c.chunk % 64 == 0 && (K + c.chunk - 1) / c.chunk == c.splits;
 }
 
+namespace {
+
+// Families of grouped f64 items with coalesced gathers: the stream tiles and, for items
+// of one 32 x 32 tile (which every stream tile pads three times over), the direct one.
+// Weights: time per padded output and k relative to the 64 x 64 stream tile. Lists of
+// 1500 equal items on B200, us, 32 x 32 direct or skinny tile against stream tile: 16 x 16
+// x 256 79 / 101, 32 x 32 x 32 27 / 27, x 128 60 / 66, x 512 151 / 195; 40^3 56 / 32, 64 x
+// 16 x 64 51 / 37, 300 x 16 x 60 206 / 115, 96^3 274 / 154, 100 x 30 x 300 320 / 172.
+const struct {
+  int kernel;
+  double weight;
+} kListFamily[] = {{dev::PLAIN_F64_STREAM_64x64, 1.0},
+                   {dev::PLAIN_F64_STREAM_128x32, 1.15},
+                   {dev::PLAIN_F64_STREAM_64x48, 1.15},
+                   {dev::PLAIN_F64_STREAM_32x128, 1.03},
+                   {dev::PLAIN_F64_DMMA_32x32, 2.3}};
+constexpr int LIST_FAMILIES = sizeof(kListFamily) / sizeof(kListFamily[0]);
+
+bool list_streams(const Product& p, int policy) {
+  return policy != 1 && policy != 2 && !(policy == 3 && p.view.N <= 32) && p.problem.dtype == DType::F64 &&
+         !(p.kernel_pin && !dev::is_packed_kernel(p.kernel_pin)) && p.hints.known && p.hints.a_gather && p.hints.b_gather;
+}
+
+double list_cost(const Product& p, int f) {
+  int bm = 0, bn = 0;
+  dev::plain_tile_shape(kListFamily[f].kernel, &bm, &bn);
+  const bool swap = dev::is_stream_kernel(kListFamily[f].kernel) && !p.hints.d_mfast;
+  const int64_t m = swap ? p.view.N : p.view.M, n = swap ? p.view.M : p.view.N;
+  const double tiles = (double)((m + bm - 1) / bm) * (double)((n + bn - 1) / bn) * (double)p.view.H;
+  return kListFamily[f].weight * tiles * bm * bn * ((double)p.view.K + 24);  // 24 k: a tile's offsets and write-back
+}
+
+int best_list_family(const Product& p) {
+  int best = 0;
+  for (int f = 1; f < LIST_FAMILIES; ++f)
+    if (list_cost(p, f) < list_cost(p, best)) best = f;
+  return kListFamily[best].kernel;
+}
+
+}  // namespace
+
 int grouped_family(const Product& p, int policy) {
   // A packed family pinned on the plan serves its single launches; inside a
   // grouped list the item takes a direct family.
@@ -219,14 +260,48 @@ int grouped_family(const Product& p, int policy) {
       break;
     default: break;
   }
-  // f64 items with coalesced gathers: the stream tiles (256 environment updates of
-  // uneven bonds 2.07 ms on the direct and skinny tiles, 1.81 with stream tiles in
-  // place of the direct ones, 1.63 in place of both).
-  if (dt == 1 && p.hints.known && p.hints.a_gather && p.hints.b_gather) {
-    double waste = 0;
-    return dev::choose_stream_kernel(dt, p.view.M, p.view.N, p.hints, &waste);
-  }
+  if (list_streams(p, policy)) return best_list_family(p);
   return dev::choose_grouped_kernel(dt, p.view.M, p.view.N, p.view.K);
+}
+
+std::vector<int> grouped_families(const std::vector<const Product*>& items, int policy) {
+  std::vector<int> out(items.size());
+  std::vector<size_t> free;  // items that any of the list families can take
+  for (size_t i = 0; i < items.size(); ++i) {
+    out[i] = grouped_family(*items[i], policy);
+    if (list_streams(*items[i], policy)) free.push_back(i);
+  }
+  // Every further family is a launch of its own, whose CTAs wait for SMs of the others.
+  // So: the one family of least cost, and another while it takes a fifth off what is
+  // left. B200, us, the best family of each item against this: 300 items of 16 to 512 per
+  // extent 185 / 116, 100 of 32 to 1024 197 / 128, 500 of 8 to 256 70 / 55, 200 tall ones
+  // (N up to 64) 143 / 138; 256 environment updates of uneven bonds 1540 / 1393 (three lists).
+  bool taken[LIST_FAMILIES] = {};
+  std::vector<double> cost(free.size(), 1e300);
+  double total = 1e300;
+  while (!free.empty()) {
+    int best = -1;
+    double least = total;
+    for (int f = 0; f < LIST_FAMILIES; ++f) {
+      if (taken[f]) continue;
+      double sum = 0;
+      for (size_t j = 0; j < free.size(); ++j) sum += std::min(cost[j], list_cost(*items[free[j]], f));
+      if (sum < least) {
+        least = sum;
+        best = f;
+      }
+    }
+    if (best < 0 || least > 0.8 * total) break;
+    taken[best] = true;
+    total = least;
+    for (size_t j = 0; j < free.size(); ++j) {
+      const double c = list_cost(*items[free[j]], best);
+      if (c >= cost[j]) continue;
+      cost[j] = c;
+      out[free[j]] = kListFamily[best].kernel;
+    }
+  }
+  return out;
 }
 
 std::string choice_name(const PlainChoice& c, int dtype) {

@@ -401,6 +401,8 @@ std::string Product::report() const {
   }
   // The model's own choice, timed beside them where it is a family that cannot be named.
   o << "]";
+  // The tile family of the plan as the only item of a grouped list.
+  if (scheme == Scheme::Plain) o << ",\"list_family\":\"" << dev::plain_kernel_name(grouped_family(*this, 0)) << "\"";
   if (scheme == Scheme::Plain)
     o << ",\"autotune_model\":\"" << choice_name(model_choice(*this, 148), (int)problem.dtype) << "\"";
   o << ",\"choice\":\"" << (scheme == Scheme::Plain ? src_names[(int)src] : "fixed")
@@ -1533,10 +1535,17 @@ struct GroupSet {
   char* starts = nullptr;
 };
 
+std::vector<int> list_families(const std::vector<int>& idx, int policy, Product* const* plans) {
+  std::vector<const Product*> items;
+  for (int i : idx) items.push_back(plans[i]);
+  return grouped_families(items, policy);
+}
+
 GroupSet build_group_set(Executor& ex, const std::vector<int>& idx, int policy, Product* const* plans,
                          const Scalar* alpha, const Scalar* beta, const Item* items) {
   std::map<int, std::vector<int>> by_family;
-  for (int i : idx) by_family[grouped_family(*plans[i], policy)].push_back(i);
+  const std::vector<int> families = list_families(idx, policy, plans);
+  for (size_t j = 0; j < idx.size(); ++j) by_family[families[j]].push_back(idx[j]);
   // Families in decreasing order of work (padded tile volume): the first one
   // runs on the submitting stream and the others fill its tail.
   std::vector<std::pair<int, std::vector<int>>> fam(by_family.begin(), by_family.end());
@@ -1681,8 +1690,7 @@ int list_policy(Executor& ex, const std::vector<int>& idx, Product* const* plans
   EventPair ev;
   std::vector<std::vector<int>> seen;
   for (int policy = 0; policy < GROUP_POLICIES; ++policy) {
-    std::vector<int> fam;
-    for (int i : idx) fam.push_back(grouped_family(*plans[i], policy));
+    const std::vector<int> fam = list_families(idx, policy, plans);
     if (std::find(seen.begin(), seen.end(), fam) != seen.end()) continue;
     seen.push_back(fam);
     GroupSet gs = build_group_set(ex, idx, policy, plans, alpha, beta, items);

@@ -268,6 +268,8 @@ bool choice_fits(const PlainChoice& c, const Product& p);
 // Tile family of a grouped item under a list tile policy (0: model, 1: large
 // tiles, 2: small tiles, 3: tall 128 x 32 tiles for narrow f64/c64 outputs).
 int grouped_family(const Product& p, int policy);
+// The families of a whole list's items (a family more is a launch more).
+std::vector<int> grouped_families(const std::vector<const Product*>& items, int policy);
 constexpr int GROUP_POLICIES = 4;
 // The versioned text form of an executor's cache, and its inverse (entries of
 // another device kind are skipped; a malformed file is an error).
