@@ -143,114 +143,119 @@ std::atomic<uint64_t> g_product_uid{1};
 }
 
 namespace {
-// The stride of a scatter vector that is an arithmetic sequence from 0, else INT64_MIN.
-int64_t sequence_stride(const std::vector<int64_t>& v) {
-  if (v.empty() || v[0] != 0) return INT64_MIN;
-  const int64_t s = v.size() > 1 ? v[1] : 0;
-  for (size_t i = 1; i < v.size(); ++i)
-    if (v[i] != (int64_t)i * s) return INT64_MIN;
-  return s;
-}
+// One operand's offset vector as its folded axes, fastest first: every fact below follows
+// from extents and strides, without a pass over the vector (hundreds of thousands of
+// entries for a large plan). The vector starts at 0.
+struct OffsetAxes {
+  std::vector<std::pair<int64_t, int64_t>> ax;  // (extent >= 2, stride), runs of one progression merged
+  int64_t n = 1;
 
-// Passes over whole offset vectors, free of branches so that they vectorise: a plan's
-// vectors have up to hundreds of thousands of entries.
-//
-// Whether a gather along a fast index is coalesced: three steps in four are 1
-// or -1.
-bool mostly_unit(const std::vector<int64_t>& fast) {
-  const int64_t* x = fast.data();
-  const size_t n = fast.size();
-  uint64_t unit = 0;
-  for (size_t i = 1; i < n; ++i) {
-    const int64_t d = x[i] - x[i - 1];
-    unit += (d == 1) | (d == -1);
+  OffsetAxes(const std::vector<Axis>& axes, int64_t Axis::*stride) {
+    for (const Axis& a : axes) {
+      n *= a.extent;
+      if (a.extent == 1) continue;
+      if (!ax.empty() && a.*stride == ax.back().second * ax.back().first)
+        ax.back().first *= a.extent;
+      else
+        ax.push_back({a.extent, a.*stride});
+    }
   }
-  return n < 2 || 4 * unit >= 3 * (n - 1);
-}
-
-// The bits in which any entry differs from a multiple of 2 * mask.
-int64_t low_bits(const std::vector<int64_t>& v, int64_t mask) {
-  int64_t low = 0;
-  for (const int64_t x : v) low |= x;
-  return low & mask;
-}
-
-// Whether an operand's elements split into aligned 16-byte groups along its
-// fast index: groups of `v` (a power of two) entries of `fast` are consecutive and
-// start at a multiple of `v`, and every other offset is a multiple of `v`.
-bool vector_groups(const std::vector<int64_t>& fast, const std::vector<int64_t>& slow, const std::vector<int64_t>& h,
-                   int64_t v) {
-  if (v == 1) return true;
-  const int64_t mask = v - 1;
-  if (low_bits(slow, mask) | low_bits(h, mask)) return false;
-  const int64_t* x = fast.data();
-  const int64_t n = (int64_t)fast.size();
-  // Entry i is i modulo v, and consecutive inside a group.
-  int64_t bad = n ? x[0] & mask : 0;
-  for (int64_t i = 1; i < n; ++i) bad |= ((x[i] - x[i - 1] - 1) & -(int64_t)((i & mask) != 0)) | ((x[i] - i) & mask);
-  return bad == 0;
-}
-
-// Whether row plus depth offsets fit 32 bits (each side below 2^30 in magnitude).
-bool fit32(const std::vector<int64_t>& rows, const std::vector<int64_t>& k) {
-  uint64_t bits = 0;
-  for (const int64_t x : rows) bits |= (uint64_t)(x ^ (x >> 63));
-  for (const int64_t x : k) bits |= (uint64_t)(x ^ (x >> 63));
-  return bits < ((uint64_t)1 << 30);
-}
+  // First step (0: none).
+  int64_t lead() const { return n > 1 ? ax[0].second : 0; }
+  // The same as a magnitude for comparisons, none being the largest.
+  uint64_t step() const { return n > 1 ? (uint64_t)std::llabs(ax[0].second) : UINT64_MAX; }
+  // The stride of an arithmetic sequence from 0, else INT64_MIN.
+  int64_t sequence() const { return n <= 0 || ax.size() > 1 ? INT64_MIN : lead(); }
+  // Whether a gather along it is coalesced: three steps in four are 1 or -1.
+  bool mostly_unit() const {
+    if (n < 2) return true;
+    int64_t unit = 0, above = n, back = 0;  // back: what the axes below an index step return
+    for (const auto& a : ax) {
+      above /= a.first;
+      const int64_t d = a.second - back;
+      if (d == 1 || d == -1) unit += (a.first - 1) * above;
+      back += (a.first - 1) * a.second;
+    }
+    return 4 * (__int128)unit >= 3 * ((__int128)n - 1);
+  }
+  // Whether every offset is a multiple of `v`.
+  bool multiples(int64_t v) const {
+    if (n <= 0) return true;
+    for (const auto& a : ax)
+      if (a.second % v != 0) return false;
+    return true;
+  }
+  // Whether groups of `v` entries are consecutive offsets that start at a multiple of `v`.
+  bool groups(int64_t v) const {
+    if (n < 2 || v == 1) return true;
+    if (ax[0].second != 1 || (ax.size() > 1 && ax[0].first % v != 0)) return false;
+    for (size_t i = 1; i < ax.size(); ++i)
+      if (ax[i].second % v != 0) return false;
+    return true;
+  }
+  // Whether every offset lies in [-2^30, 2^30).
+  bool fits30() const {
+    __int128 lo = 0, hi = 0;
+    for (const auto& a : ax) (a.second < 0 ? lo : hi) += (__int128)(a.first - 1) * a.second;
+    const __int128 most = (__int128)1 << 30;
+    return n <= 0 || (hi < most && lo >= -most);
+  }
+};
 }  // namespace
 
 Product::Product(const Problem& p) : problem(p), uid(g_product_uid.fetch_add(1)) {
   packed = PackedPlan::from_problem(p);
   const bool swap = packed.transposes_gemm(32);
   view = orient(packed, swap);
-  tiny_h = dev::TinyStrides{sequence_stride(view.h_a), sequence_stride(view.h_b), sequence_stride(view.h_c),
-                            sequence_stride(view.h_d)};
-  const int64_t v = 16 / (int64_t)dtype_size(problem.dtype);
-  const std::vector<int64_t>&af = view.a_kfast ? view.a_k : view.a_m, &as = view.a_kfast ? view.a_m : view.a_k;
-  const std::vector<int64_t>&bf = view.b_kfast ? view.b_k : view.b_n, &bs = view.b_kfast ? view.b_n : view.b_k;
+  // The view's vectors as axes (orient() in plan.cpp): the swap exchanges the operands.
+  const PlanStats& ps = packed.stats;
+  const std::vector<Axis>&rows = swap ? ps.n_axes : ps.m_axes, &columns = swap ? ps.m_axes : ps.n_axes;
+  int64_t Axis::*const ta = swap ? &Axis::sb : &Axis::sa, Axis::*const tb = swap ? &Axis::sa : &Axis::sb;
+  const OffsetAxes a_m(rows, ta), a_k(ps.k_axes, ta), b_k(ps.k_axes, tb), b_n(columns, tb), h_a(ps.h_axes, ta), h_b(ps.h_axes, tb),
+      d_m(rows, &Axis::sd), d_n(columns, &Axis::sd), h_d(ps.h_axes, &Axis::sd), c_m(rows, &Axis::sc), c_n(columns, &Axis::sc),
+      h_c(ps.h_axes, &Axis::sc);
+  tiny_h = dev::TinyStrides{h_a.sequence(), h_b.sequence(), h_c.sequence(), h_d.sequence()};
   small.regular = true;
-  const auto small_index = [&](const std::vector<int64_t>& x) {
-    dev::SmallIndex i;
-    i.n = (int64_t)x.size();
-    i.lead = x.size() > 1 ? x[1] - x[0] : 0;
-    i.stride = sequence_stride(x);
-    small.regular = small.regular && i.stride != INT64_MIN;
-    return i;
-  };
   if (dev::small_batched_fits(view.M, view.N, view.K, view.H)) {
-    small.h_a = small_index(view.h_a);
-    small.a_m = small_index(view.a_m);
-    small.a_k = small_index(view.a_k);
-    small.h_b = small_index(view.h_b);
-    small.b_n = small_index(view.b_n);
-    small.b_k = small_index(view.b_k);
-    small.h_d = small_index(view.h_d);
-    small.d_m = small_index(view.d_m);
-    small.d_n = small_index(view.d_n);
-    small.h_c = small_index(view.h_c);
-    small.c_m = small_index(view.c_m);
-    small.c_n = small_index(view.c_n);
+    const auto index = [&](const OffsetAxes& x) {
+      dev::SmallIndex i;
+      i.n = x.n;
+      i.lead = x.lead();
+      i.stride = x.sequence();
+      small.regular = small.regular && i.stride != INT64_MIN;
+      return i;
+    };
+    small.h_a = index(h_a);
+    small.a_m = index(a_m);
+    small.a_k = index(a_k);
+    small.h_b = index(h_b);
+    small.b_n = index(b_n);
+    small.b_k = index(b_k);
+    small.h_d = index(h_d);
+    small.d_m = index(d_m);
+    small.d_n = index(d_n);
+    small.h_c = index(h_c);
+    small.c_m = index(c_m);
+    small.c_n = index(c_n);
   }
+  const int64_t v = 16 / (int64_t)dtype_size(problem.dtype);
+  const OffsetAxes &af = view.a_kfast ? a_k : a_m, &as = view.a_kfast ? a_m : a_k;
+  const OffsetAxes &bf = view.b_kfast ? b_k : b_n, &bs = view.b_kfast ? b_n : b_k;
   hints.known = true;
-  hints.a_vec = vector_groups(af, as, view.h_a, v);
-  hints.b_vec = vector_groups(bf, bs, view.h_b, v);
-  hints.a_gather = mostly_unit(af);
-  hints.b_gather = mostly_unit(bf);
+  hints.a_vec = af.groups(v) && as.multiples(v) && h_a.multiples(v);
+  hints.b_vec = bf.groups(v) && bs.multiples(v) && h_b.multiples(v);
+  hints.a_gather = af.mostly_unit();
+  hints.b_gather = bf.mostly_unit();
   hints.d_mfast = view.d_mfast;
-  const auto step = [](const std::vector<int64_t>& x) {
-    return x.size() > 1 ? (uint64_t)std::llabs(x[1] - x[0]) : UINT64_MAX;
+  hints.h_inner = h_a.step() < std::min(a_m.step(), a_k.step()) && h_b.step() < std::min(b_n.step(), b_k.step()) &&
+                  h_d.step() < std::min(d_m.step(), d_n.step());
+  hints.off32 = (problem.dtype == DType::F32 || problem.dtype == DType::C32) && a_m.fits30() && a_k.fits30() &&
+                b_n.fits30() && b_k.fits30();
+  const auto fastest = [](const OffsetAxes& r, const OffsetAxes& k, const OffsetAxes& h) {
+    return h.step() < std::min(r.step(), k.step()) ? 2 : k.step() < r.step() ? 1 : 0;
   };
-  hints.h_inner = step(view.h_a) < std::min(step(view.a_m), step(view.a_k)) &&
-                  step(view.h_b) < std::min(step(view.b_n), step(view.b_k)) &&
-                  step(view.h_d) < std::min(step(view.d_m), step(view.d_n));
-  hints.off32 = (problem.dtype == DType::F32 || problem.dtype == DType::C32) && fit32(view.a_m, view.a_k) &&
-                fit32(view.b_n, view.b_k);
-  const auto fastest = [&](const std::vector<int64_t>& rows, const std::vector<int64_t>& k, const std::vector<int64_t>& h) {
-    return step(h) < std::min(step(rows), step(k)) ? 2 : step(k) < step(rows) ? 1 : 0;
-  };
-  a_fast = fastest(view.a_m, view.a_k, view.h_a);
-  b_fast = fastest(view.b_n, view.b_k, view.h_b);
+  a_fast = fastest(a_m, a_k, h_a);
+  b_fast = fastest(b_n, b_k, h_b);
   signature = problem_signature(*this);
 }
 
@@ -401,6 +406,11 @@ std::string Product::report() const {
   }
   // The model's own choice, timed beside them where it is a family that cannot be named.
   o << "]";
+  o << ",\"layout\":{\"a_vec\":" << (hints.a_vec ? "true" : "false") << ",\"b_vec\":" << (hints.b_vec ? "true" : "false")
+    << ",\"a_gather\":" << (hints.a_gather ? "true" : "false") << ",\"b_gather\":" << (hints.b_gather ? "true" : "false")
+    << ",\"off32\":" << (hints.off32 ? "true" : "false") << ",\"h_inner\":" << (hints.h_inner ? "true" : "false")
+    << ",\"small_regular\":" << (small.regular ? "true" : "false") << ",\"a_fast\":" << a_fast << ",\"b_fast\":" << b_fast
+    << "}";
   // The tile family of the plan as the only item of a grouped list.
   if (scheme == Scheme::Plain) o << ",\"list_family\":\"" << dev::plain_kernel_name(grouped_family(*this, 0)) << "\"";
   if (scheme == Scheme::Plain)
