@@ -43,6 +43,7 @@
 // Every wait is bounded (a status bit, then the role ends). No cluster, no multicast.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "tc_common.cuh"
 
@@ -342,11 +343,12 @@ __device__ __forceinline__ void ts_mark(unsigned char* again, int tile, int warp
 }
 
 // STEPS: steps of 16 plane depths (one MMA each) in all of K: 1, 2 or (3) more.
-template <bool CPLX, int STEPS>
+// GEN: D is more than the sums (alpha, C, conjugation), an instantiation of its own, as
+// the registers for C cost the other calls a tenth.
+template <bool CPLX, int STEPS, bool GEN>
 __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_constant__ GemmArgs g, int tiles, int tm,
                                                                   int tn, unsigned char* __restrict__ flags) {
-  using T = typename Elem<float, CPLX>::type;
-  constexpr int EK = CPLX ? TS_BK / 2 : TS_BK;
+  constexpr int E = CPLX ? 2 : 1, EK = TS_BK / E;
   extern __shared__ unsigned char ts_smem[];
   char* ring = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ts_smem) + 127) & ~uintptr_t(127));
   int64_t* cols = reinterpret_cast<int64_t*>(ring + TsSmem::RING);
@@ -527,8 +529,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       const int m = x.m0 + (CPLX ? prow >> 1 : prow), n0 = x.n0 + col0;
       const bool mok = m < (int)g.M;
       const int nrem = max(0, min(TS_CPT, (int)g.N - n0));
-      T* Db = static_cast<T*>(g.D) + nd;
-      const T* Cb = static_cast<const T*>(g.C) + nc;
+      // A lane writes one component of its row.
+      float* const Db = static_cast<float*>(g.D) + nd * E + comp;
+      const float* const Cb = static_cast<const float*>(g.C) + nc * E + comp;
       const int64_t *dn_s = cols_w + (it & 1) * 2 * TS_CPT, *cn_s = dn_s + TS_CPT;
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
@@ -580,15 +583,34 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
       const bool second = steps_all % 2 == 0, more = (nk - 1) % TS_FLUSH != 0, flushed = nk > TS_FLUSH;
       // Sums that the planes may not carry are computed again: all of them, or (a finite
       // threshold, and D only written) this warp's once one of them is below it.
-      const bool skip = thr == __uint_as_float(0x7f800000u) || (thr != 0.f && !e.plain);
+      const bool skip = thr == __uint_as_float(0x7f800000u) || (thr != 0.f && GEN);
       if (skip && lane == 0) ts_mark(again, it, warp);
       const int ncols = skip ? 0 : nrem;
       float least = __uint_as_float(0x7f800000u);  // magnitude of what this lane writes
+      // C of eight columns, a group ahead of its use.
+      float cv[GEN ? 8 : 1], cnext[GEN ? 8 : 1];
+      const auto fetch_c = [&](int q) {
+        if constexpr (GEN) {
+          if (e.beta_zero) return;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) cnext[j] = mok && 8 * q + j < ncols ? Cb[cn_s[8 * q + j] * E] : 0.f;
+        }
+      };
+      if constexpr (GEN) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cnext[j] = 0.f;
+        fetch_c(0);
+      }
 #pragma unroll 1
       for (int q = 0; 8 * q < ncols; ++q) {
         {
           uint32_t r[8], u[8];
           float v[8];
+          if constexpr (GEN) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) cv[j] = cnext[j];
+            fetch_c(q + 1);
+          }
           ts_tmem_ld(main0 + 8 * q, r);
           ts_tmem_ld(main1 + 8 * q, u);  // STEPS 1: the cross products
           if constexpr (MULTI) {
@@ -620,30 +642,39 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tc_stream_kernel(const __grid_c
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(u[j]);
-          if (e.plain && 8 * q + 8 <= ncols) {
-            float* Df = reinterpret_cast<float*>(Db) + comp;
+          if constexpr (GEN) {
+            // D = op(alpha acc + beta op(C)) of this lane's component; the other one of a
+            // complex row sits in the neighbouring lane.
+            const float ar = (float)e.alpha_re, ai = comp ? (float)e.alpha_im : -(float)e.alpha_im;
+            const float br = (float)e.beta_re, bi = comp ? (float)e.beta_im : -(float)e.beta_im;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) least = fminf(least, fabsf(v[j]));
-            if (mok) {
+            for (int j = 0; j < 8; ++j) {
+              float y = v[j] * ar;
+              if constexpr (CPLX) y += __shfl_xor_sync(0xffffffffu, v[j], 1) * ai;
+              if (!e.beta_zero) {
+                const float c = CPLX && e.conj_c && comp ? -cv[j] : cv[j];
+                y += c * br;
+                if constexpr (CPLX) y += __shfl_xor_sync(0xffffffffu, c, 1) * bi;
+              }
+              v[j] = CPLX && e.conj_d && comp ? -y : y;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (8 * q + j < ncols) least = fminf(least, fabsf(v[j]));
+          }
+          if (mok) {
+            if (8 * q + 8 <= ncols) {
 #pragma unroll
               for (int j = 0; j < 8; j += 2) {
                 const longlong2 o = *reinterpret_cast<const longlong2*>(dn_s + 8 * q + j);
-                Df[o.x * (CPLX ? 2 : 1)] = v[j];
-                Df[o.y * (CPLX ? 2 : 1)] = v[j + 1];
+                Db[o.x * E] = v[j];
+                Db[o.y * E] = v[j + 1];
               }
-            }
-          } else {
-#pragma unroll 1
-            for (int j = 0; j < 8; ++j) {
-              // v[j] without a dynamic register index.
-              float y = v[0];
+            } else {
 #pragma unroll
-              for (int i = 1; i < 8; ++i) y = j == i ? v[i] : y;
-              const int jj = 8 * q + j;
-              const float o = CPLX ? __shfl_xor_sync(0xffffffffu, y, 1) : 0.f;
-              if (jj < ncols) least = fminf(least, fabsf(y));
-              if (jj >= ncols || !mok || comp) continue;
-              epilogue_store<float, CPLX>(e, y, o, Cb + (e.beta_zero ? 0 : cn_s[jj]), Db + dn_s[jj]);
+              for (int j = 0; j < 8; ++j)
+                if (8 * q + j < ncols) Db[dn_s[8 * q + j] * E] = v[j];
             }
           }
           __syncwarp();
@@ -820,10 +851,12 @@ cudaError_t launch_tc_stream(int dtype, const GemmArgs& g, void* flags, cudaStre
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
   const int64_t steps = (g.K * (dtype == 2 ? 2 : 1) + 15) / 16;
-  auto kern = dtype == 2 ? (steps == 1 ? tc_stream_kernel<true, 1> : steps == 2 ? tc_stream_kernel<true, 2>
-                                                                                : tc_stream_kernel<true, 3>)
-                         : (steps == 1 ? tc_stream_kernel<false, 1> : steps == 2 ? tc_stream_kernel<false, 2>
-                                                                                 : tc_stream_kernel<false, 3>);
+  const auto pick = [&](auto cplx, auto gen) {
+    constexpr bool C = decltype(cplx)::value, G = decltype(gen)::value;
+    return steps == 1 ? tc_stream_kernel<C, 1, G> : steps == 2 ? tc_stream_kernel<C, 2, G> : tc_stream_kernel<C, 3, G>;
+  };
+  const auto of = [&](auto cplx) { return g.e.plain ? pick(cplx, std::false_type{}) : pick(cplx, std::true_type{}); };
+  auto kern = dtype == 2 ? of(std::true_type{}) : of(std::false_type{});
   const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TsSmem::BYTES);
   if (r != cudaSuccess) return r;
   kern<<<grid, TS_THREADS, TsSmem::BYTES, st>>>(g, (int)tiles, (int)tm, (int)tn, static_cast<unsigned char*>(flags));
