@@ -797,44 +797,78 @@ bool tc_stream_fits(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, const
          ((double)(N / em) + 1) * ((double)(M / TS_BN) + 1) * (double)H < tiles;
 }
 
-// Against the FFMA families by estimated microseconds, fitted on B200. Here: 8, per
-// wave of tiles 4 (1.5 for outputs of at most 64 columns) and 1.1 (c32 1.25) per 32-deep
-// stage, 4 per panel; there: 12 (26 from K = 64 on, with packs) + 2 M N K / 50e6 (c32 /
-// 40e6) over whole tiles + 1 per MB of D. Measured here against there: f32 6144^2 x 24
-// in six indexes 89 against 235, 2048^2 x 64 17 against 32, x 1024 87 against 217,
-// 120000 x 31 x 33 37 against 90, 16 x 100^3 batch innermost 26 against 17, 300 x 260 x
-// 2000 (63 stages on nine SMs) 76 against 40 with split-K; c32 2048^2 x 512 178 against
-// 402, 700^2 x 2500 226 against 373. Below 2^23 products the launches decide.
-// Over planes packed first (k_split.cu) the split is paid once, not once per tile: 16,
-// the planes' bytes at 4 TB/s, and 20 + 0.038 per plane depth for a wave of 128 x 256
-// tiles, whose depth is split where the wave is partly filled (f32 4096^3 0.67 ms
-// against 1.21 here and 2.70 there, 2048^2 x 512 55 against 51 here; c32 2048^3 0.41
-// ms against 0.66 here and 1.53 there; f32 700^2 x 2500 against 108 here, 94 there).
+// Against the FFMA families by estimated microseconds. Fitted on B200 to 600 contractions
+// (matrix products, batches, permuted, six-index and transformation shapes, K from 1 to
+// 4096) timed on all three; typical deviation 7 to 12 %. The family chosen is 4.3 % above
+// the best of the three in the geometric mean (with constants fitted to an earlier state
+// of the kernels 7.7 %). Below 2^23 products the launches decide.
+//
+// FFMA: the choice made without these families, by its tile waves, with the pack pass, the
+// write-back and split K. In flight: waves of tiles, stages of 32 plane depths, panels.
+// Packed: the planes' bytes, waves of 128 x 256 tiles by plane depth (a partial wave in
+// parts). Each with a constant for its launches, and with the operand elements that a
+// panel or the planes read uncoalesced.
+//
+// With tiles for less than a quarter of the SMs, near a tie, the FFMA families' one launch
+// takes the call. From a quarter up these
+// families keep what is estimated within 7 us of FFMA: their sums are the more accurate,
+// and the estimate of a call this short is off by as much (f32 2564 x 129 x 128: estimated
+// 7 apart, measured 14.4 to 16.5 FFMA, 18.5 here).
 int choose_tc_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
   if (!hints.tensor || !tc_stream_fits(dtype, M, N, K, H, hints)) return 0;
   const bool cplx = dtype == 2;
   const int64_t m = hints.d_mfast ? M : N, n = hints.d_mfast ? N : M;  // the launch's roles
-  const int64_t em = cplx ? TS_BM / 2 : TS_BM, ek = cplx ? TS_BK / 2 : TS_BK, pad = cplx ? 64 : 128;
+  const int64_t em = cplx ? TS_BM / 2 : TS_BM, ek = cplx ? TS_BK / 2 : TS_BK, e = cplx ? 2 : 1;
   const int64_t tiles = ((m + em - 1) / em) * ((n + TS_BN - 1) / TS_BN) * H;
-  const double outs = (double)M * (double)N * (double)H, per = cplx ? 4 : 1;
-  if (tiles < 16 || outs * (double)K * per < (double)(1 << 23)) return 0;
+  const double outs = (double)M * (double)N * (double)H, k = (double)K;
+  if (tiles < 16 || outs * k * (cplx ? 4 : 1) < (double)(1 << 23)) return 0;
+
+  LaunchHints general = hints;
+  general.tensor = false;
+  int kernel = 0, splits = 1, bm = 0, bn = 0;
+  int64_t chunk = 0;
+  choose_plain_launch(dtype, 0, M, N, K, H, num_sms, general, &kernel, &splits, &chunk);
+  plain_tile_shape(kernel, &bm, &bn);
+  const double rows = (double)((M + bm - 1) / bm * bm), cols = (double)((N + bn - 1) / bn * bn);
+  const double area = (double)bm * bn, whole = rows / bm * (cols / bn) * (double)H * splits;
+  double ffma;
+  if (is_packed_kernel(kernel)) {
+    const double slots = (cplx ? 2 : 1) * (double)num_sms, w = whole < 3 * slots ? std::ceil(whole / slots) : whole / slots + 0.5;
+    const double bytes = 4 * (rows * (cplx ? 4 : 1) + cols * (cplx ? 2 : 1)) * k * (double)H, part = std::ceil(k / splits);
+    ffma = cplx ? 10.2 + 0.53e-6 * bytes + w * 0.154 * part + (splits > 1 ? 11.2e-6 * splits * outs : 0) + 10.7e-6 * outs
+                : 6.7 + 0.55e-6 * bytes + w * (0.074 * part + 8.3) + (splits > 1 ? 5.6 + 1.6e-6 * splits * outs : 0) + 3.6e-6 * outs;
+  } else {
+    const double w = std::max(1.0, whole / num_sms) * area * k * 1e-6, t = std::max(1.0, whole / num_sms);
+    ffma = cplx ? 5.2 + 8.7 * 4 * w + 3.5 * t + 1.9e-6 * outs
+           : bm == 128 ? 10.8 + 11.2 * w + 5.4 * t + 1.2e-6 * outs
+                       : 5.2 + 15.0 * w + 1.3 * t + 3.3e-6 * outs;
+    ffma = std::max(9.0, ffma);
+  }
+
   const double waves = (double)((tiles + num_sms - 1) / num_sms), stages = (double)((K + ek - 1) / ek);
-  const double here = 8 + waves * ((n <= 64 ? 1.5 : 4) + (cplx ? 1.25 : 1.1) * stages) +
-                      4 * ((hints.a_gather ? 0 : 1) + (hints.b_gather ? 0 : 1));
-  const double whole = (double)((M + pad - 1) / pad * pad) * (double)((N + pad - 1) / pad * pad) * (double)H;
-  const double there = (K >= 64 ? 26 : 12) + 2 * per * whole * (double)K / (cplx ? 40e6 : 50e6) +
-                       outs * (cplx ? 8e-6 : 4e-6);
+  const int panels = (hints.a_gather ? 0 : 1) + (hints.b_gather ? 0 : 1);
+  const double panel = ((hints.a_gather ? 0 : (double)M) + (hints.b_gather ? 0 : (double)N)) * k * (double)H;
+  const double width = std::min(1.0, std::max((double)n, 8.0) / TS_BN);
+  const double here = cplx ? 8.5 + waves * (2.0 * width + 0.27 + 1.64 * stages) + 3.7 * panels + 6.2e-6 * panel + 0.44e-6 * outs
+                           : 9.4 + waves * (1.5 * width + 0.23 + 2.0 * stages) + 3.4 * panels + 5.3e-6 * panel + 0.18e-6 * outs;
+
   double split = 1e30;
   if (tc_split_fits(dtype, M, N, K, H)) {
-    const double mp = (double)((m * (cplx ? 2 : 1) + 127) / 128 * 128), np = (double)((n + 255) / 256 * 256);
-    const double kp = (double)((K * (cplx ? 2 : 1) + 63) / 64 * 64), t = mp / 128 * np / 256 * (double)H;
-    const double parts = t < num_sms ? std::min(std::min(16.0, std::floor(num_sms / t)), std::floor(kp / 256)) : 1;
-    const double w = t <= num_sms ? 1 : t / num_sms + 0.15;
-    split = 16 + ((mp + np) * kp * 6 + (double)(m + n) * (double)K * (cplx ? 8 : 4)) * (double)H / 4e6 +
-            (parts > 1 ? 25 + 0.038 * kp / parts : w * (20 + 0.038 * kp));
+    const int64_t mp = (m * e + 127) / 128 * 128, np = (n + 255) / 256 * 256, kp = (K * e + 63) / 64 * 64;
+    const int64_t t = mp / 128 * (np / 256) * H, rem = t % num_sms;
+    double w;
+    if (t >= num_sms)
+      w = (double)(t / num_sms) + (rem ? 1.0 / (double)std::max<int64_t>(1, std::min<int64_t>(4, num_sms / rem)) : 0.0);
+    else
+      w = 1.0 / (double)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(16, num_sms / t), kp / 64));
+    const double bytes = ((double)(mp + np) * (double)kp * 6 + (double)(m + n) * k * 4 * (double)e) * (double)H;
+    split = cplx ? 19.8 + 0.405e-6 * bytes + 1.55e-6 * panel + 0.0322 * w * (double)kp + 6.8 * std::ceil(w) + 1.9e-6 * outs
+                 : 15.2 + 0.38e-6 * bytes + 2.1e-6 * panel + 0.045 * w * (double)kp + 10.7 * std::ceil(w) + 0.27e-6 * outs;
   }
-  if (split < here && split < there) return cplx ? PLAIN_C32_TC_SPLIT : PLAIN_F32_TC_SPLIT;
-  return here < there ? (cplx ? PLAIN_C32_TC_STREAM : PLAIN_F32_TC_STREAM) : 0;
+  const double bar = tiles * 4 < num_sms ? 0.95 * ffma : ffma + 7.0;
+  if (std::min(here, split) >= bar) return 0;
+  if (split < here) return cplx ? PLAIN_C32_TC_SPLIT : PLAIN_F32_TC_SPLIT;
+  return cplx ? PLAIN_C32_TC_STREAM : PLAIN_F32_TC_STREAM;
 }
 
 // The caller has checked tc_stream_fits.
