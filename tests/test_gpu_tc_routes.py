@@ -133,3 +133,55 @@ def test_a_cached_choice_beyond_the_cap_is_reported_as_the_models(tp, torch_cuda
     rep = p.report()
     assert ".tcgen05." not in rep["family"] and rep["choice"] == "model"
     ex.close()
+
+
+def labelled_call(tp, torch, dtype, spec, ext, beta, limits):
+    """Runs the column-major contraction under each workspace limit (None: none) and yields
+    (status, family, error against 64 bits)."""
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    lhs, out = spec.split("->")
+    la, lb = lhs.split(",")
+    kind = torch.complex64 if dtype == tp.C32 else torch.float32
+
+    def make(labels):
+        shape = [ext[x] for x in labels]
+        t = torch.randn(int(np.prod(shape)), generator=gen, device="cuda", dtype=kind)
+        st = np.cumprod([1] + shape[:-1]).tolist()
+        return t.as_strided(shape, st), tp.TensorInfo(dtype, shape, st), [ord(x) for x in labels]
+
+    (a, ia, na), (b, ib, nb), (d, idd, nd) = make(la), make(lb), make(out)
+    c = d.clone()
+    h = tp.Handle()
+    p = tp.TensorProduct.create(h, (0, ia, na), (0, ib, nb), (0, idd, nd), (0, idd, nd))
+    wide = torch.complex128 if dtype == tp.C32 else torch.float64
+    want = torch.einsum(spec, a.to(wide), b.to(wide)) + beta * c.to(wide)
+    for limit in limits:
+        ex = tp.Executor()
+        if limit:
+            ex.set_workspace_limit(limit)
+        d.copy_(c)
+        torch.cuda.synchronize()
+        status = p.execute(ex, 1.0, a.data_ptr(), b.data_ptr(), beta, d.data_ptr() if beta else None, d.data_ptr())
+        ex.close()
+        yield status, p.report()["family"], float((d.to(wide) - want).norm() / want.norm())
+
+
+# The cap leaves no room for what the tensor-core family lays out (a panel, planes of 6 bytes
+# a real), but for what the general choice needs: nothing for a direct tile, packed panels
+# of 4 bytes a real (tiles enough that it does not split K, which takes partials as well).
+WITHIN = [
+    ("ikmb,mjac->abcijk", dict(a=12, b=11, c=20, i=13, j=11, k=12, m=9), ".stream.", {"F32": 1 << 10, "C32": 1 << 10}),
+    ("cbka,kj->abjc", dict(a=50, b=21, c=22, j=60, k=40), ".stream.", {"F32": 1 << 10, "C32": 1 << 10}),
+    ("ka,kb->ab", dict(a=30000, b=32, k=24), ".stream.", {"F32": 1 << 10, "C32": 1 << 10}),
+    ("mk,kn->mn", dict(m=2000, n=1900, k=700), ".split.", {"F32": 16 << 20, "C32": 40 << 20}),
+    ("km,nk->mn", dict(m=2000, n=1900, k=600), ".split.", {"F32": 12 << 20, "C32": 36 << 20}),
+]
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+@pytest.mark.parametrize("spec,ext,family,limits", WITHIN)
+@pytest.mark.parametrize("dtype", ["F32", "C32"])
+def test_device_operands_under_a_workspace_cap(tp, torch_cuda, dtype, spec, ext, family, limits, beta):
+    (s0, f0, e0), (s1, f1, e1) = labelled_call(tp, torch_cuda, getattr(tp, dtype), spec, ext, beta, (None, limits[dtype]))
+    assert s0 == 0 and family in f0 and e0 <= 1e-6, (s0, f0, e0)
+    assert s1 == 0 and ".tcgen05." not in f1 and e1 <= 1e-6, (s1, f1, e1, tp.last_error())
