@@ -1292,10 +1292,10 @@ bool packed_fits(int kernel, int64_t M, int64_t N, int64_t K, int64_t H) {
 int choose_plain_kernel(int dtype, int64_t M, int64_t N, int64_t K, int64_t H, int num_sms, const LaunchHints& hints) {
   auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * H; };
   // Stream tiles (gathers coalesced on both sides, at least a wave of tiles)
-  // against the packed family, f64 on B200: 177147 x 243 x 50 0.207 ms against
-  // 0.290 (direct tile 0.295); 64 x 256^3 0.089 against 0.120; 2048^2 x 512 0.162
-  // against 0.183; 2048^3 0.622 against 0.604. Above K = 512 they are chosen where
-  // their tile pads less (136856 x 22 x 240: 0.092 against 0.273).
+  // against the packed family, f64 on B200: 177147 x 243 x 50 0.201 ms against
+  // 0.290 (direct tile 0.292); 64 x 256^3 0.086 against 0.119; 2048^2 x 512 0.165
+  // against 0.181; 2048^3 0.622 against 0.607. Above K = 512 they are chosen where
+  // their tile pads less (136856 x 22 x 240: 0.085 against 0.274).
   const bool gather = hints.a_gather && hints.b_gather;
   if (hints.known && dtype == 1 && gather && K > 0) {
     double waste = 0;

@@ -11,8 +11,8 @@
 // A side whose batch entries follow one another in memory moves in 16-byte copies
 // (D in 16-byte stores) and keeps the memory's order in shared memory. About 36 KB
 // of shared memory per CTA keeps six CTAs, and their loads, in flight per SM (24 KB
-// measured 2 to 19 % slower). f64 8192 products of 32 x 4 x 32 on B200: 121 us on
-// 64 x 64 tiles, 13.4 us here (84 MB, 6.3 TB/s).
+// measured 2 to 19 % slower). f64 8192 products of 32 x 4 x 32 on B200: 123 us on
+// 64 x 64 tiles, 16.4 us here in calls one after another (84 MB, 5.1 TB/s).
 #include "device_common.cuh"
 
 namespace tprims {

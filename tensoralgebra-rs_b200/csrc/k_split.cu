@@ -5,8 +5,8 @@
 //   bf16x3: x0*y0 + x0*y1 + x1*y0                       (2 planes, 3 products)
 //   bf16x6: bf16x3 + x0*y2 + x1*y1 + x2*y0              (3 planes, 6 products)
 // Each plane keeps the next 8 significant bits of the remainder, so bf16x6
-// carries 24 bits (the f32 significand) and drops only terms below 2^-24 of
-// the product; bf16x3 carries 16 bits.
+// carries 24 bits (the f32 significand) and drops x1*y2 + x2*y1 and less, at
+// most 2^-24 of the product; bf16x3 carries 16 bits.
 //
 // Two kernels:
 //  * split_pack: gathers A' (or B') through its scatter vectors (the packing of

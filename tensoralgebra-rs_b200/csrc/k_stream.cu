@@ -11,16 +11,18 @@
 // tile's index loads and gathers overlap this tile's products and epilogue.
 //
 //   producer: tile -> row offsets in registers; per stage 16 k offsets in one
-//             register per lane (fetched a stage ahead, passed by shuffles),
-//             one cp.async per element into [k][row] order; the tile's output
-//             offsets go to a double-buffered slot by cp.async with the first
-//             stage.
+//             register per lane (fetched a stage ahead, passed by shuffles);
+//             an operand's copies of 16 bytes where its elements lie side by
+//             side along rows or k, else one cp.async per element, into [k][row]
+//             order; the tile's output offsets go to a double-buffered slot by
+//             cp.async with the first stage.
 //   compute:  full[stage] -> fragments -> empty[stage]; after the last stage
 //             the epilogue from the slot, then slot_empty.
 //
-// Only the k of the last stage that exist are multiplied (in steps of four), so a short odd K costs no padded
-// depth. Every mbarrier wait is bounded by %globaltimer (a status bit, then the
-// role ends); the producer drains its own copies before it exits.
+// Only the k of the last stage that exist are multiplied (in steps of four), so a
+// short odd K costs no padded depth. Every mbarrier wait is bounded by %globaltimer
+// (a status bit, then the role ends); the producer drains its own copies before it
+// exits.
 #include "tc_common.cuh"
 
 namespace tprims {
@@ -666,8 +668,8 @@ int stream_dtype(int kernel) { return kStream[kernel - PLAIN_STREAM_FIRST].dtype
 const char* stream_kernel_name(int kernel) { return kStream[kernel - PLAIN_STREAM_FIRST].name; }
 
 // Each family's padded outputs, weighted by its measured time per padded
-// output relative to 64 x 64 (B200, 177147 x 243 x 50 f64: 64 x 64 0.207
-// ms, 128 x 32 0.238, 64 x 48 0.262 on 1.13 times the padded area, 32 x 128 0.211).
+// output relative to 64 x 64 (B200, 177147 x 243 x 50 f64: 64 x 64 0.201
+// ms, 128 x 32 0.234, 64 x 48 0.259 on 1.13 times the padded area, 32 x 128 0.208).
 int choose_stream_kernel(int dtype, int64_t M, int64_t N, const LaunchHints& hints, double* waste) {
   static const struct {
     int kernel;

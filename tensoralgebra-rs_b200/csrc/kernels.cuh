@@ -226,13 +226,14 @@ inline bool small_batched_fits(int64_t M, int64_t N, int64_t K, int64_t H) {
 }
 // Whether the model takes them. They read each element once where the tiny
 // kernel reads it once per output it enters, and where a tile kernel pads every
-// product to its tile. B200, us per call: f64 65536 products of 4^3 14.6 against
-// 43.8 (tiny), c64 131072 of 3^3 18.7 against 47.6 (tiny), f64 8192 of 32 x 4 x 32
-// 21.9 against 74.8 (tiles), f32 100000 of 5 x 7 x 13 24 against 4312 (tiles). The
-// tiny kernel stays the faster one for products with next to no reuse (f32 200000
-// of 12 x 1 x 1 21 against 36, of 1 x 1 x 30 25 against 31) and where the batch is
-// innermost in all operands, as its lanes then read consecutive elements (f64 65536
-// of 4^3 14.4 against 15.0). Few products do not fill the groups.
+// product to its tile. B200, us per call: f64 65536 products of 4^3 12.9 against
+// 42.7 (tiny), f64 8192 of 32 x 4 x 32 16.4 against 123 (tiles), f32 100000 of 5 x 7
+// x 13 19.4 against 4108 (tiles). The tiny kernel stays the faster one for products
+// with next to no reuse (f32 200000 of 12 x 1 x 1 21 against 36, of 1 x 1 x 30 25
+// against 31) and where the batch is innermost in all operands, as its lanes then read
+// consecutive elements (f64 65536 of 4^3 12.4 against 15.0). Few products do not fill
+// the groups; at 256 the two are within 0.7 us for f64 and c64 (8^3 8.9 on tiles, 9.5
+// here: the larger parameter block) and f32 and c32 gain (15.6 against 9.6).
 inline bool use_small_batched(int64_t M, int64_t N, int64_t K, int64_t H, const LaunchHints& hints) {
   return hints.known && small_batched_fits(M, N, K, H) && H >= 256 && M * N * K >= 48 &&
          !(hints.h_inner && use_tiny_batched(M, N, K, H));
