@@ -148,3 +148,44 @@ def test_values_outside_the_planes_take_no_cliff(tp, torch_cuda, dt, m, n, k, wh
         ms.append(min(u.elapsed_time(v) for u, v in zip(t, t[1:])))
     e.close()
     assert ms[0] <= 2 * ms[1] + 0.05, ms
+
+
+@pytest.mark.parametrize("dt,m,n,k", [("f32", 4000, 1000, 40), ("c32", 3000, 900, 30), ("f32", 2048, 2048, 1024),
+                                      ("c32", 2048, 1024, 600)])
+def test_a_captured_call_marks_its_tiles_anew(tp, dt, m, n, k):
+    """Replays of one captured call: values that the planes carry, then an infinity and an
+    element below 2^-100, then the first again."""
+    import torch
+
+    kind, wide = {"f32": (torch.float32, torch.float64), "c32": (torch.complex64, torch.complex128)}[dt]
+    side = torch.cuda.Stream()
+    ex = tp.Executor(device=0, stream=side.cuda_stream, sync=False)
+    with torch.cuda.stream(side):
+        make = lambda r, c: torch.randn(r * c, device="cuda", dtype=kind).as_strided([r, c], [1, r])
+        A, B, D = make(m, k), make(k, n), make(m, n)
+        first = A.clone()
+    lay = lambda x: tp.OperandSpec(tp.LayoutSpec.col_major(x))
+    plan = tp.Plan(tp.Problem.from_labels({"f32": tp.F32, "c32": tp.C32}[dt], lay([m, k]), lay([k, n]), lay([m, n]),
+                                          [0, 2], [2, 1], [0, 1]))
+    assert ".tcgen05." in plan.report()["family"]
+    with torch.cuda.stream(side):
+        plan.execute_into(ex, 1.0, A, B, D)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        plan.execute_into(ex, 1.0, A, B, D)
+    finite = lambda t: torch.isfinite(torch.view_as_real(t).sum(-1) if t.is_complex() else t)
+    for extreme in (False, True, False):
+        with torch.cuda.stream(side):
+            A.copy_(first)
+            if extreme:
+                A[5, 1], A[7, 2] = float("inf"), 2.0 ** -120
+            D.zero_()
+            graph.replay()
+        torch.cuda.synchronize()
+        want = A.to(wide) @ B.to(wide)
+        ok = finite(want)
+        assert bool((finite(D) == ok).all()) and bool(ok.all()) != extreme
+        assert float((D.to(wide) - want)[ok].norm() / want[ok].norm()) <= 1e-6
+    del graph
+    ex.close()
